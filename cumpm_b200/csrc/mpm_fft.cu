@@ -1,6 +1,6 @@
 // Batched in-place 1-D DFT along a strided axis (see mpm_fft.h).
 #include "mpm_fft.h"
-#include "mpm_fft_consts.cuh"
+#include "mpm_butterfly.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -65,193 +65,6 @@ __device__ __forceinline__ void pass_reg(const cplx<R>* __restrict__ in, cplx<R>
             }
             out[(kb.y + h * Ns) * CW + c] = mk<R>(s1 - s2, s3 + s4);
             if (h > 0 && 2 * h != r) out[(kb.y + (r - h) * Ns) * CW + c] = mk<R>(s1 + s2, s4 - s3);
-        }
-    }
-}
-
-// -i v (forward rotation) or +i v (inverse)
-template <typename R, bool INV>
-__device__ __forceinline__ cplx<R> rot(cplx<R> v) {
-    return INV ? mk<R>(-v.y, v.x) : mk<R>(v.y, -v.x);
-}
-
-template <typename R, bool INV, int RAD>
-__device__ __forceinline__ void dft_small(cplx<R> (&x)[RAD]);
-
-// W_N^j = exp(-2 pi i j / N) (conjugated for INV) from the constant tables
-template <typename R, bool INV, int N>
-__device__ __forceinline__ cplx<R> wconst(int j) {
-    cplx<R> w;
-    static_assert(N == 7 || (N >= 9 && N <= 16), "no constant table for this radix");
-    if constexpr (sizeof(R) == 8) {
-        if constexpr (N == 7) w = kW7d[j];
-        else if constexpr (N == 9) w = kW9d[j];
-        else if constexpr (N == 10) w = kW10d[j];
-        else if constexpr (N == 11) w = kW11d[j];
-        else if constexpr (N == 12) w = kW12d[j];
-        else if constexpr (N == 13) w = kW13d[j];
-        else if constexpr (N == 14) w = kW14d[j];
-        else if constexpr (N == 15) w = kW15d[j];
-        else w = kW16d[j];
-    } else {
-        if constexpr (N == 7) w = kW7f[j];
-        else if constexpr (N == 9) w = kW9f[j];
-        else if constexpr (N == 10) w = kW10f[j];
-        else if constexpr (N == 11) w = kW11f[j];
-        else if constexpr (N == 12) w = kW12f[j];
-        else if constexpr (N == 13) w = kW13f[j];
-        else if constexpr (N == 14) w = kW14f[j];
-        else if constexpr (N == 15) w = kW15f[j];
-        else w = kW16f[j];
-    }
-    if (INV) w.y = -w.y;
-    return w;
-}
-
-// Composite DFT of A*B points in registers (Cooley-Tukey, decimation in
-// time): input m = B m1 + m2, output k = k1 + A k2,
-//   y_k = sum_m2 W_B^(m2 k2) [ W_N^(m2 k1) sum_m1 x_(B m1 + m2) W_A^(m1 k1) ].
-template <typename R, bool INV, int A, int B>
-__device__ __forceinline__ void dft_ct(cplx<R> (&x)[A * B]) {
-    constexpr int N = A * B;
-    cplx<R> z[B][A];
-#pragma unroll
-    for (int m2 = 0; m2 < B; ++m2) {
-        cplx<R> t[A];
-#pragma unroll
-        for (int m1 = 0; m1 < A; ++m1) t[m1] = x[B * m1 + m2];
-        dft_small<R, INV, A>(t);
-#pragma unroll
-        for (int k1 = 0; k1 < A; ++k1) z[m2][k1] = m2 * k1 == 0 ? t[k1] : t[k1] * wconst<R, INV, N>(m2 * k1);
-    }
-#pragma unroll
-    for (int k1 = 0; k1 < A; ++k1) {
-        cplx<R> t[B];
-#pragma unroll
-        for (int m2 = 0; m2 < B; ++m2) t[m2] = z[m2][k1];
-        dft_small<R, INV, B>(t);
-#pragma unroll
-        for (int k2 = 0; k2 < B; ++k2) x[k1 + A * k2] = t[k2];
-    }
-}
-
-// Odd prime P in registers: with a_q = x_q + x_(P-q), b_q = x_q - x_(P-q),
-// y_p = x_0 + sum_q a_q cos(2 pi p q / P) -+ i sum_q b_q sin(2 pi p q / P)
-// and y_(P-p) the same with the sine term negated.
-template <typename R, bool INV, int P>
-__device__ __forceinline__ void dft_odd(cplx<R> (&x)[P]) {
-    constexpr int H = (P - 1) / 2;
-    cplx<R> a[H], b[H];
-#pragma unroll
-    for (int q = 1; q <= H; ++q) {
-        a[q - 1] = x[q] + x[P - q];
-        b[q - 1] = x[q] - x[P - q];
-    }
-    cplx<R> y0 = x[0];
-#pragma unroll
-    for (int q = 0; q < H; ++q) y0 += a[q];
-#pragma unroll
-    for (int p = 1; p <= H; ++p) {
-        cplx<R> t = x[0], u = mk<R>(R(0), R(0));
-#pragma unroll
-        for (int q = 1; q <= H; ++q) {
-            const cplx<R> w = wconst<R, false, P>((p * q) % P);   // (cos, -sin)
-            t = t + a[q - 1] * w.x;
-            u = u + b[q - 1] * (-w.y);
-        }
-        // -i u (forward) or +i u (inverse)
-        const cplx<R> ru = rot<R, INV>(u);
-        x[p] = t + ru;
-        x[P - p] = t - ru;
-    }
-    x[0] = y0;
-}
-
-// In-register DFT of RAD points, y_p = sum_q x_q W^(p q), W = exp(-+2 pi i/RAD),
-// written out for 2, 3, 4, 5, 6, 8, tabulated primes 7, 11, 13 and composed
-// 9, 10, 12, 14, 15, 16.
-template <typename R, bool INV, int RAD>
-__device__ __forceinline__ void dft_small(cplx<R> (&x)[RAD]) {
-    if constexpr (RAD == 1) {
-    } else if constexpr (RAD == 7) {
-        dft_odd<R, INV, 7>(x);
-    } else if constexpr (RAD == 9) {
-        dft_ct<R, INV, 3, 3>(x);
-    } else if constexpr (RAD == 10) {
-        dft_ct<R, INV, 2, 5>(x);
-    } else if constexpr (RAD == 11) {
-        dft_odd<R, INV, 11>(x);
-    } else if constexpr (RAD == 12) {
-        dft_ct<R, INV, 4, 3>(x);
-    } else if constexpr (RAD == 13) {
-        dft_odd<R, INV, 13>(x);
-    } else if constexpr (RAD == 14) {
-        dft_ct<R, INV, 2, 7>(x);
-    } else if constexpr (RAD == 15) {
-        dft_ct<R, INV, 3, 5>(x);
-    } else if constexpr (RAD == 16) {
-        dft_ct<R, INV, 4, 4>(x);
-    } else if constexpr (RAD == 2) {
-        const cplx<R> a = x[0], b = x[1];
-        x[0] = a + b;
-        x[1] = a - b;
-    } else if constexpr (RAD == 3) {
-        const R h = R(0.86602540378443864676);   // sin(2 pi / 3)
-        const cplx<R> s = x[1] + x[2];
-        const cplx<R> t = x[0] - s * R(0.5);
-        const cplx<R> d = (x[1] - x[2]) * h;
-        x[0] = x[0] + s;
-        x[1] = t + rot<R, INV>(d);
-        x[2] = t - rot<R, INV>(d);
-    } else if constexpr (RAD == 4) {
-        const cplx<R> a = x[0] + x[2], b = x[0] - x[2], c = x[1] + x[3], d = rot<R, INV>(x[1] - x[3]);
-        x[0] = a + c;
-        x[2] = a - c;
-        x[1] = b + d;
-        x[3] = b - d;
-    } else if constexpr (RAD == 5) {
-        const R c1 = R(0.30901699437494742410), c2 = R(-0.80901699437494742410);
-        const R s1 = R(0.95105651629515357212), s2 = R(0.58778525229247312917);
-        const cplx<R> a1 = x[1] + x[4], b1 = x[1] - x[4], a2 = x[2] + x[3], b2 = x[2] - x[3];
-        const cplx<R> t1 = x[0] + a1 * c1 + a2 * c2, t2 = x[0] + a1 * c2 + a2 * c1;
-        const cplx<R> u1 = rot<R, INV>(b1 * s1 + b2 * s2), u2 = rot<R, INV>(b1 * s2 - b2 * s1);
-        x[0] = x[0] + a1 + a2;
-        x[1] = t1 + u1;
-        x[4] = t1 - u1;
-        x[2] = t2 + u2;
-        x[3] = t2 - u2;
-    } else if constexpr (RAD == 6) {
-        // even / odd halves as two 3-point DFTs, then W6^p between them
-        cplx<R> e[3] = {x[0], x[2], x[4]}, o[3] = {x[1], x[3], x[5]};
-        dft_small<R, INV, 3>(e);
-        dft_small<R, INV, 3>(o);
-        const R h = R(0.86602540378443864676);
-        const cplx<R> w1 = mk<R>(R(0.5), INV ? h : -h), w2 = mk<R>(R(-0.5), INV ? h : -h);
-        const cplx<R> o1 = o[1] * w1, o2 = o[2] * w2;
-        x[0] = e[0] + o[0];
-        x[3] = e[0] - o[0];
-        x[1] = e[1] + o1;
-        x[4] = e[1] - o1;
-        x[2] = e[2] + o2;
-        x[5] = e[2] - o2;
-    } else if constexpr (RAD == 8) {
-        const R q = R(0.70710678118654752440);
-        cplx<R> u[4], v[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            u[k] = x[k] + x[k + 4];
-            v[k] = x[k] - x[k + 4];
-        }
-        // v_k *= W8^k
-        v[1] = (v[1] + rot<R, INV>(v[1])) * q;
-        v[2] = rot<R, INV>(v[2]);
-        v[3] = (rot<R, INV>(v[3]) - v[3]) * q;
-        dft_small<R, INV, 4>(u);
-        dft_small<R, INV, 4>(v);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            x[2 * k] = u[k];
-            x[2 * k + 1] = v[k];
         }
     }
 }
@@ -379,21 +192,6 @@ __device__ __forceinline__ void pass_stream(cplx<R>* __restrict__ in, cplx<R>* _
     }
 }
 
-// global -> shared copy of one element without a register round trip, so a
-// thread's whole share of the line is in flight at once (src_bytes = 0 fills
-// the element with zeros and reads nothing)
-template <typename R>
-__device__ __forceinline__ void copy_async(cplx<R>* dst, const cplx<R>* src, bool live) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    const int bytes = live ? int(sizeof(cplx<R>)) : 0;
-    if constexpr (sizeof(cplx<R>) == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
 // All radix passes of one line held in shared memory (ping-pong between
 // `in` and `out`); returns the buffer that holds the result.  T holds the
 // line's twiddles, conjugated for INV.
@@ -514,41 +312,6 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_axis(cplx<R>* __restrict__ 
 
 constexpr int kFft2MaxThreads = 384;
 
-template <int CLS, typename Fn>
-__device__ __forceinline__ void radix_dispatch(int r, Fn&& fn) {
-    switch (r) {
-        case 1: fn(std::integral_constant<int, 1>{}); break;
-        case 2: fn(std::integral_constant<int, 2>{}); break;
-        case 3: fn(std::integral_constant<int, 3>{}); break;
-        case 4: fn(std::integral_constant<int, 4>{}); break;
-        case 5: fn(std::integral_constant<int, 5>{}); break;
-        case 6: fn(std::integral_constant<int, 6>{}); break;
-        case 7: fn(std::integral_constant<int, 7>{}); break;
-        case 8: fn(std::integral_constant<int, 8>{}); break;
-        default:
-            // register classes: radices up to CLS only (8, 12 or 16)
-            if constexpr (CLS > 8) {
-                switch (r) {
-                    case 9: fn(std::integral_constant<int, 9>{}); break;
-                    case 10: fn(std::integral_constant<int, 10>{}); break;
-                    case 11: fn(std::integral_constant<int, 11>{}); break;
-                    case 12: fn(std::integral_constant<int, 12>{}); break;
-                    default: break;
-                }
-            }
-            if constexpr (CLS > 12) {
-                switch (r) {
-                    case 13: fn(std::integral_constant<int, 13>{}); break;
-                    case 14: fn(std::integral_constant<int, 14>{}); break;
-                    case 15: fn(std::integral_constant<int, 15>{}); break;
-                    case 16: fn(std::integral_constant<int, 16>{}); break;
-                    default: break;
-                }
-            }
-            break;
-    }
-}
-
 template <typename R, int CW, int MODE, int CLS>
 __global__ void __launch_bounds__(kFft2MaxThreads) k_fft2(cplx<R>* __restrict__ data, const cplx<R>* __restrict__ tw,
                                                           int r1, int r2, size_t es, int ncols, size_t os,
@@ -661,6 +424,10 @@ std::pair<int, int> fft2_split(int n) {
     }
     return best;
 }
+
+// longest composite m of a dense pass (m FMAs per element against the general
+// kernel's extra shared round trips)
+constexpr int kDenseMaxComposite = 131;
 
 size_t fft2_smem(int n, int cw, size_t elem) { return (size_t(n) * cw + n) * elem; }
 
@@ -847,119 +614,6 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(cplx<R>* __restrict__ dat
     }
 }
 
-// ---------------------------------------------------------------------------
-// Two-pass line transform for n = r1 * p, r1 an in-register radix and p an
-// odd prime above 16 (the monolayer x axis: 366 = 6 * 61).  Pass 1 (radix
-// r1, butterfly j1 < p) reads x[j1 + q p] straight from global memory and
-// stores S[j1 r1 + p1] already multiplied by pass 2's twiddle W_n^(j1 p1)
-// (pass 2 butterfly j reads S[j + q r1], i.e. j1 = q, p1 = j).  Pass 2 (radix
-// p, butterfly j < r1) streams its inputs from shared memory as the general
-// kernel's prime pass does (a_q = x_q + x_(p-q), b_q = x_q - x_(p-q), PC
-// output pairs per work item, W_p^(p' q) from the table PT in shared memory)
-// and writes y[p' r1 + j] straight to global memory.  One CTA = CW columns
-// of one line; L = blockDim.x / CW lanes loop over pass 1's p butterflies and
-// pass 2's r1 * ceil(((p-1)/2) / PC) work items.
-
-// fp64 work items carry half the output pairs, so that their accumulators
-// leave room for three CTAs per SM
-template <typename R>
-__host__ __device__ constexpr int fft2p_pc() { return sizeof(R) == 8 ? 4 : 8; }
-
-template <typename R, int CW, bool INV, int CLS>
-__global__ void __launch_bounds__(kFft2MaxThreads) k_fft2p(cplx<R>* __restrict__ data, const cplx<R>* __restrict__ tw,
-                                                           const cplx<R>* __restrict__ ptw, int pt_total, int pt_ld,
-                                                           int r1, int p, size_t es, int ncols, size_t os,
-                                                           int ngroups) {
-    constexpr int PC = fft2p_pc<R>();   // output pairs per work item
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int n = r1 * p;
-    const int L = blockDim.x / CW;
-    cplx<R>* S = reinterpret_cast<cplx<R>*>(smem_raw);   // [n][CW]
-    cplx<R>* PT = S + size_t(n) * CW;                      // [pt_total], 16-byte aligned (CW >= 2)
-    cplx<R>* T = PT + pt_total;                            // [n]
-    const int o = blockIdx.x / ngroups;
-    const int g = blockIdx.x - o * ngroups;
-    const int c = threadIdx.x & (CW - 1);
-    const int lane = threadIdx.x / CW;
-    const int c0 = g * CW;
-    const bool live = c0 + c < ncols;
-    cplx<R>* line = data + size_t(o) * os + c0 + c;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        cplx<R> w = tw[t];
-        if (INV) w.y = -w.y;
-        T[t] = w;
-    }
-    for (int t = threadIdx.x; t < pt_total; t += blockDim.x) PT[t] = ptw[t];
-    __syncthreads();
-    // pass 1: radix r1, global -> shared with pass 2's twiddles applied
-    radix_dispatch<CLS>(r1, [&](auto rc) {
-        constexpr int RAD = decltype(rc)::value;
-#pragma unroll 2
-        for (int j1 = lane; j1 < p; j1 += L) {
-            cplx<R> x[RAD];
-#pragma unroll
-            for (int q = 0; q < RAD; ++q) x[q] = live ? line[size_t(j1 + q * p) * es] : mk<R>(R(0), R(0));
-            dft_small<R, INV, RAD>(x);
-            S[(j1 * RAD) * CW + c] = x[0];
-#pragma unroll
-            for (int p1 = 1; p1 < RAD; ++p1) S[(j1 * RAD + p1) * CW + c] = x[p1] * T[j1 * p1];
-        }
-    });
-    __syncthreads();
-    // pass 2: radix p streamed from shared memory, outputs to global memory
-    const int half = (p - 1) / 2;
-    const int nchunk = (half + PC - 1) / PC;
-    for (int u = lane; u < r1 * nchunk; u += L) {
-        const int ch = u / r1;
-        const int j = u - ch * r1;
-        const int p0 = 1 + ch * PC;
-        const cplx<R> x0 = S[j * CW + c];
-        R px[PC], py[PC], qx[PC], qy[PC];
-#pragma unroll
-        for (int k = 0; k < PC; ++k) px[k] = py[k] = qx[k] = qy[k] = R(0);
-        R sx = R(0), sy = R(0);
-        const cplx<R>* prow = PT + (p0 - 1);
-        for (int q = 1; q <= half; ++q, prow += pt_ld) {
-            const cplx<R> xa = S[(j + q * r1) * CW + c];
-            const cplx<R> xb = S[(j + (p - q) * r1) * CW + c];
-            const R ax = xa.x + xb.x, ay = xa.y + xb.y, bx = xa.x - xb.x, by = xa.y - xb.y;
-            sx += ax;
-            sy += ay;
-            cplx<R> wk[PC];
-            if constexpr (sizeof(R) == 4) {
-                const float4* p4 = reinterpret_cast<const float4*>(prow);
-#pragma unroll
-                for (int k = 0; k < PC / 2; ++k) {
-                    const float4 v = p4[k];
-                    wk[2 * k] = mk<R>(v.x, v.y);
-                    wk[2 * k + 1] = mk<R>(v.z, v.w);
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < PC; ++k) wk[k] = prow[k];
-            }
-#pragma unroll
-            for (int k = 0; k < PC; ++k) {
-                const R wy = INV ? -wk[k].y : wk[k].y;
-                px[k] = fma(ax, wk[k].x, px[k]);
-                py[k] = fma(ay, wk[k].x, py[k]);
-                qx[k] = fma(bx, wy, qx[k]);
-                qy[k] = fma(by, wy, qy[k]);
-            }
-        }
-        if (!live) continue;
-        if (ch == 0) line[size_t(j) * es] = mk<R>(x0.x + sx, x0.y + sy);
-#pragma unroll
-        for (int k = 0; k < PC; ++k) {
-            const int pp = p0 + k;
-            if (pp <= half) {
-                line[size_t(pp * r1 + j) * es] = mk<R>(x0.x + px[k] - qy[k], x0.y + py[k] + qx[k]);
-                line[size_t((p - pp) * r1 + j) * es] = mk<R>(x0.x + px[k] + qy[k], x0.y + py[k] - qx[k]);
-            }
-        }
-    }
-}
-
 // W_r^(p q) table of a streamed prime pass: rows q = 1..(r-1)/2, columns
 // p = 1..(r-1)/2 padded to a multiple of 8 with zeros, plus 8 spare entries
 // so that a padded row can always be read whole.  Appended to `out`; returns
@@ -1000,192 +654,6 @@ std::pair<int, int> fft2p_split(int n) {
     if (m > 1) p = std::max(p, m);
     if (p <= 16 || !is_prime(p) || !fft2_radix(n / p)) return {0, 0};
     return {n / p, p};
-}
-
-size_t fft2p_smem(int n, int cw, size_t elem, int pt_total) { return (size_t(n) * cw + pt_total + n) * elem; }
-
-template <typename R, bool INV, int CW>
-void launch2p_cw(int cls, int nblocks, int nthreads, size_t shm, cudaStream_t s, cplx<R>* data, const cplx<R>* tw,
-                 const cplx<R>* ptw, int pt_total, int pt_ld, int r1, int p, size_t es, int ncols, size_t os,
-                 int ngroups) {
-    auto go = [&](auto kern) {
-        set_smem_limit(kern, shm);
-        kern<<<nblocks, nthreads, shm, s>>>(data, tw, ptw, pt_total, pt_ld, r1, p, es, ncols, os, ngroups);
-    };
-    if (cls == 8) go(k_fft2p<R, CW, INV, 8>);
-    else go(k_fft2p<R, CW, INV, 16>);
-}
-
-// ---------------------------------------------------------------------------
-// Two-pass line transform n = r1 * p with the prime pass done by Rader's
-// algorithm: with g a primitive root mod p, a_q = x[g^-q], b_s = W_p^(g^s),
-//   y[0] = x[0] + sum_q a_q,   y[g^m] = x[0] + (a (*) b)_m   (cyclic, length N = p-1)
-// and the cyclic convolution is IDFT_N(DFT_N(a) . Bh) with Bh = DFT_N(b) / N
-// precomputed.  N = A * B with both in-register radices, so DFT_N is one
-// Cooley-Tukey step through shared memory: R1 (thread per (j, q2)) an A-point
-// DFT over q1 of a[B q1 + q2] and the twiddles W_N^(q2 k1); R2 (thread per
-// (j, k1)) the B-point DFT over q2, the product with Bh, the B-point inverse
-// DFT and the twiddles W_N^(-m1 k1) in registers; R4 (thread per (j, m1)) the
-// A-point inverse DFT giving c[m1 + B m2], written to global memory at row
-// g^(m1 + B m2).  About a quarter of the direct prime pass's arithmetic.
-// Pass 1 is k_fft2p's (radix r1 from global memory, pass-2 twiddles fused).
-template <typename R, int CW, bool INV, int CLS>
-__global__ void __launch_bounds__(kFft2MaxThreads) k_fft2r(cplx<R>* __restrict__ data, const cplx<R>* __restrict__ tw,
-                                                           const cplx<R>* __restrict__ rtab,
-                                                           const int* __restrict__ rperm, int r1, int p, int A,
-                                                           int B, size_t es, int ncols, size_t os, int ngroups) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int n = r1 * p;
-    const int N = p - 1;
-    const int L = blockDim.x / CW;
-    cplx<R>* S = reinterpret_cast<cplx<R>*>(smem_raw);   // [n][CW] pass-1 output
-    cplx<R>* Tt = S + size_t(n) * CW;                      // [r1 * N][CW] Rader work rows
-    cplx<R>* T = Tt + size_t(r1) * N * CW;                 // [n] line twiddles
-    cplx<R>* WN = T + n;                                   // [N] W_N^t
-    cplx<R>* Bh = WN + N;                                  // [N] this direction's Bh
-    int* pin = reinterpret_cast<int*>(Bh + N);             // [N] g^-q
-    int* pout = pin + N;                                   // [N] g^m
-    const int o = blockIdx.x / ngroups;
-    const int g = blockIdx.x - o * ngroups;
-    const int c = threadIdx.x & (CW - 1);
-    const int lane = threadIdx.x / CW;
-    const int c0 = g * CW;
-    const bool live = c0 + c < ncols;
-    cplx<R>* line = data + size_t(o) * os + c0 + c;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        cplx<R> w = tw[t];
-        if (INV) w.y = -w.y;
-        T[t] = w;
-    }
-    for (int t = threadIdx.x; t < N; t += blockDim.x) {
-        WN[t] = rtab[t];
-        Bh[t] = rtab[(INV ? 2 : 1) * N + t];
-        pin[t] = rperm[t];
-        pout[t] = rperm[N + t];
-    }
-    __syncthreads();
-    // pass 1: radix r1, global -> shared with pass 2's twiddles applied
-    radix_dispatch<CLS>(r1, [&](auto rc) {
-        constexpr int RAD = decltype(rc)::value;
-#pragma unroll 2
-        for (int j1 = lane; j1 < p; j1 += L) {
-            cplx<R> x[RAD];
-#pragma unroll
-            for (int q = 0; q < RAD; ++q) x[q] = live ? line[size_t(j1 + q * p) * es] : mk<R>(R(0), R(0));
-            dft_small<R, INV, RAD>(x);
-            S[(j1 * RAD) * CW + c] = x[0];
-#pragma unroll
-            for (int p1 = 1; p1 < RAD; ++p1) S[(j1 * RAD + p1) * CW + c] = x[p1] * T[j1 * p1];
-        }
-    });
-    __syncthreads();
-    // R1: A-point DFTs over q1 of a[B q1 + q2], twiddled by W_N^(q2 k1)
-    radix_dispatch<CLS>(A, [&](auto rc) {
-        constexpr int RA = decltype(rc)::value;
-        for (int u = lane; u < r1 * B; u += L) {
-            const int q2 = u / r1;
-            const int j = u - q2 * r1;
-            cplx<R> z[RA];
-#pragma unroll
-            for (int q1 = 0; q1 < RA; ++q1) z[q1] = S[(j + pin[B * q1 + q2] * r1) * CW + c];
-            dft_small<R, false, RA>(z);
-            cplx<R>* trow = Tt + (size_t(j) * N + q2 * RA) * CW + c;
-            trow[0] = z[0];
-#pragma unroll
-            for (int k1 = 1; k1 < RA; ++k1) trow[k1 * CW] = q2 ? z[k1] * WN[q2 * k1] : z[k1];
-        }
-    });
-    __syncthreads();
-    // R2: B-point DFT over q2 (-> DFT_N(a) at k1 + A k2), times Bh, B-point
-    // inverse DFT over k2, twiddles W_N^(-m1 k1); the thread rewrites the
-    // same Tt slots it read
-    radix_dispatch<CLS>(B, [&](auto rc) {
-        constexpr int RB = decltype(rc)::value;
-        for (int u = lane; u < r1 * A; u += L) {
-            const int k1 = u / r1;
-            const int j = u - k1 * r1;
-            cplx<R>* tcol = Tt + (size_t(j) * N + k1) * CW + c;
-            cplx<R> v[RB];
-#pragma unroll
-            for (int q2 = 0; q2 < RB; ++q2) v[q2] = tcol[q2 * A * CW];
-            dft_small<R, false, RB>(v);
-            if (k1 == 0 && live) {
-                const cplx<R> x0 = S[j * CW + c];
-                line[size_t(j) * es] = x0 + v[0];   // y[0] = x[0] + sum a
-            }
-#pragma unroll
-            for (int k2 = 0; k2 < RB; ++k2) v[k2] = v[k2] * Bh[k1 + A * k2];
-            dft_small<R, true, RB>(v);
-            tcol[0] = v[0];
-#pragma unroll
-            for (int m1 = 1; m1 < RB; ++m1) {
-                cplx<R> w = WN[m1 * k1];
-                w.y = -w.y;
-                tcol[m1 * A * CW] = k1 ? v[m1] * w : v[m1];
-            }
-        }
-    });
-    __syncthreads();
-    // R4: A-point inverse DFT over k1 -> c[m1 + B m2]; y[g^m] = x[0] + c[m]
-    radix_dispatch<CLS>(A, [&](auto rc) {
-        constexpr int RA = decltype(rc)::value;
-        for (int u = lane; u < r1 * B; u += L) {
-            const int m1 = u / r1;
-            const int j = u - m1 * r1;
-            const cplx<R>* trow = Tt + (size_t(j) * N + m1 * RA) * CW + c;
-            cplx<R> d[RA];
-#pragma unroll
-            for (int k1 = 0; k1 < RA; ++k1) d[k1] = trow[k1 * CW];
-            dft_small<R, true, RA>(d);
-            if (!live) continue;
-            const cplx<R> x0 = S[j * CW + c];
-#pragma unroll
-            for (int m2 = 0; m2 < RA; ++m2) line[size_t(pout[m1 + B * m2] * r1 + j) * es] = x0 + d[m2];
-        }
-    });
-}
-
-size_t fft2r_smem(int n, int r1, int N, int cw, size_t elem) {
-    return (size_t(n) * cw + size_t(r1) * N * cw + n + 2 * size_t(N)) * elem + 2 * sizeof(int) * N;
-}
-
-template <typename R, bool INV, int CW>
-void launch2r_cw(int cls, int nblocks, int nthreads, size_t shm, cudaStream_t s, cplx<R>* data, const cplx<R>* tw,
-                 const cplx<R>* rtab, const int* rperm, int r1, int p, int A, int B, size_t es, int ncols, size_t os,
-                 int ngroups) {
-    auto go = [&](auto kern) {
-        set_smem_limit(kern, shm);
-        kern<<<nblocks, nthreads, shm, s>>>(data, tw, rtab, rperm, r1, p, A, B, es, ncols, os, ngroups);
-    };
-    if (cls == 8) go(k_fft2r<R, CW, INV, 8>);
-    else if (cls == 12) go(k_fft2r<R, CW, INV, 12>);
-    else go(k_fft2r<R, CW, INV, 16>);
-}
-
-// smallest primitive root of the prime p
-int primitive_root(int p) {
-    std::vector<int> f;
-    int m = p - 1;
-    for (int d = 2; d * d <= m; ++d)
-        if (m % d == 0) {
-            f.push_back(d);
-            while (m % d == 0) m /= d;
-        }
-    if (m > 1) f.push_back(m);
-    for (int g = 2; g < p; ++g) {
-        bool ok = true;
-        for (int q : f) {
-            long long e = (p - 1) / q, r = 1, b = g;
-            while (e) {
-                if (e & 1) r = r * b % p;
-                b = b * b % p;
-                e >>= 1;
-            }
-            if (r == 1) { ok = false; break; }
-        }
-        if (ok) return g;
-    }
-    return 0;
 }
 
 size_t fft_smem(int n, int cw, size_t elem, int pt_total) {
@@ -1284,67 +752,16 @@ void AxisFFT::init(int n) {
     }
     f_.pt_total = int(p64.size());
     upload_table(p64, pt64_, pt32_);
-    // Rader tables when p - 1 splits into two in-register radices and the
-    // kernel's shared memory fits at its narrowest tile (4 fp64 columns)
-    ra_ = rb_ = 0;
-    if (kind_ == 2) {
-        const int pr = r2_, N = pr - 1;
-        const std::pair<int, int> ab = fft2_split(N);
-        const int g = primitive_root(pr);
-        if (ab.first && g && fft2r_smem(n, r1_, N, 4, sizeof(double2)) <= kFftSmemBudget) {
-            kind_ = 3;
-            ra_ = ab.first;
-            rb_ = ab.second;
-            std::vector<int> perm(2 * N);
-            std::vector<long long> gp(N);   // g^s mod p
-            long long v = 1;
-            for (int t = 0; t < N; ++t) {
-                gp[t] = v;
-                v = v * g % pr;
-            }
-            for (int q = 0; q < N; ++q) perm[q] = int(gp[(N - q) % N]);   // a_q = x[g^-q]
-            for (int m = 0; m < N; ++m) perm[N + m] = int(gp[m]);         // y[g^m]
-            std::vector<double2> t64(3 * size_t(N));
-            for (int t = 0; t < N; ++t) {
-                const double a = -2.0 * kPi * double(t) / double(N);
-                t64[t] = make_double2(std::cos(a), std::sin(a));
-            }
-            // Bh = DFT_N(b) / N, b_s = W_p^(g^s) (forward) or its conjugate (inverse)
-            for (int k = 0; k < N; ++k) {
-                double fr = 0, fi = 0, ir = 0, ii = 0;
-                for (int t = 0; t < N; ++t) {
-                    const double ab_ = -2.0 * kPi * double(gp[t]) / double(pr);
-                    const double br = std::cos(ab_), bi = std::sin(ab_);
-                    const double e = -2.0 * kPi * double((long long)t * k % N) / double(N);
-                    const double er = std::cos(e), ei = std::sin(e);
-                    fr += br * er - bi * ei;
-                    fi += br * ei + bi * er;
-                    ir += br * er + bi * ei;
-                    ii += br * ei - bi * er;
-                }
-                t64[N + k] = make_double2(fr / N, fi / N);
-                t64[2 * N + k] = make_double2(ir / N, ii / N);
-            }
-            upload_table(t64, rt64_, rt32_);
-            rperm_.ensure(sizeof(int) * perm.size());
-            MPM_CUDA(cudaMemcpy(rperm_.p, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice));
-        }
+    // dense split: the prime split above, the in-register split's own radices,
+    // else the largest radix up to 16 while the rest stays short enough
+    int dr = r1_;
+    if (!kind_) {
+        dr = 1;
+        for (int r = 2; r <= 16; ++r)
+            if (n % r == 0) dr = r;
+        if (n / dr > kDenseMaxComposite) dr = 0;
     }
-    // the streamed prime pass's table; lengths whose table and tile do not
-    // fit in shared memory go to the general multi-pass kernel
-    pp_total_ = pp_ld_ = 0;
-    if (kind_ == 2) {
-        std::vector<double2> q64;
-        const int ld = append_prime_table(r2_, q64);
-        if (fft2p_smem(n, 4, sizeof(double2), int(q64.size())) <= kFftSmemBudget) {
-            pp_ld_ = ld;
-            pp_total_ = int(q64.size());
-            upload_table(q64, pp64_, pp32_);
-        } else {
-            kind_ = 0;
-            r1_ = r2_ = 0;
-        }
-    }
+    dense_.init(n, dr);
 }
 
 void AxisFFT::upload_table(std::vector<double2> t64, DevBuf& d64, DevBuf& d32) {
@@ -1369,72 +786,9 @@ void AxisFFT::launch_line(cplx<R>* data, size_t es, int ncols, size_t os, int no
     ks.sb = sb;
     const cplx<R>* tw = sizeof(R) == 4 ? reinterpret_cast<const cplx<R>*>(tw32_.p)
                                        : reinterpret_cast<const cplx<R>*>(tw64_.p);
-    const int kind = path(ncols, mode);
-    if (kind == 3) {
-        // two-pass with a Rader prime pass
-        const int N = r2_ - 1;
-        const int L = 24;
-        // wide butterfly classes hold more registers: smaller CTAs
-        int cw = register_class(std::max(r1_, ra_)) > 8 ? 8 : 16;
-        while (cw > 4 && (cw * L > (sizeof(R) == 8 ? 192 : kFft2MaxThreads) ||
-                          fft2r_smem(n, r1_, N, cw, sizeof(cplx<R>)) > kFftSmemBudget))
-            cw /= 2;
-        const size_t shm = fft2r_smem(n, r1_, N, cw, sizeof(cplx<R>));
-        if (shm > kFftSmemMax) throw std::runtime_error("FFT line does not fit in shared memory");
-        const int ngroups = (ncols + cw - 1) / cw;
-        const int nblocks = nouter * ngroups;
-        const int cls = register_class(std::max(r1_, ra_));
-        const cplx<R>* rt = sizeof(R) == 4 ? reinterpret_cast<const cplx<R>*>(rt32_.p)
-                                           : reinterpret_cast<const cplx<R>*>(rt64_.p);
-        const int* rp = rperm_.as<int>();
-        auto go = [&](auto invc) {
-            constexpr bool INV = decltype(invc)::value;
-            if (cw == 16)
-                launch2r_cw<R, INV, 16>(cls, nblocks, cw * L, shm, s, data, tw, rt, rp, r1_, r2_, ra_, rb_, es, ncols,
-                                        os, ngroups);
-            else if (cw == 8)
-                launch2r_cw<R, INV, 8>(cls, nblocks, cw * L, shm, s, data, tw, rt, rp, r1_, r2_, ra_, rb_, es, ncols,
-                                       os, ngroups);
-            else
-                launch2r_cw<R, INV, 4>(cls, nblocks, cw * L, shm, s, data, tw, rt, rp, r1_, r2_, ra_, rb_, es, ncols,
-                                       os, ngroups);
-        };
-        if (mode == 1) go(std::true_type{});
-        else go(std::false_type{});
-        MPM_LAUNCH();
-        return;
-    }
+    const int kind = path(ncols, sizeof(R) == 8);
     if (kind == 2) {
-        // two-pass with a streamed prime pass
-        const int half = (r2_ - 1) / 2;
-        const int pc = fft2p_pc<R>();
-        const int nitems = r1_ * ((half + pc - 1) / pc);
-        const int L = std::min(sizeof(R) == 8 ? 24 : 32, std::max(16, nitems));
-        int cw = 16;
-        while (cw > 4 && (cw * L > kFft2MaxThreads ||
-                          fft2p_smem(n, cw, sizeof(cplx<R>), pp_total_) > kFftSmemBudget))
-            cw /= 2;
-        const size_t shm = fft2p_smem(n, cw, sizeof(cplx<R>), pp_total_);
-        const int ngroups = (ncols + cw - 1) / cw;
-        const int nblocks = nouter * ngroups;
-        const int cls = r1_ <= 8 ? 8 : 16;
-        const cplx<R>* ptw = sizeof(R) == 4 ? reinterpret_cast<const cplx<R>*>(pp32_.p)
-                                            : reinterpret_cast<const cplx<R>*>(pp64_.p);
-        auto go = [&](auto invc) {
-            constexpr bool INV = decltype(invc)::value;
-            if (cw == 16)
-                launch2p_cw<R, INV, 16>(cls, nblocks, cw * L, shm, s, data, tw, ptw, pp_total_, pp_ld_, r1_, r2_, es,
-                                        ncols, os, ngroups);
-            else if (cw == 8)
-                launch2p_cw<R, INV, 8>(cls, nblocks, cw * L, shm, s, data, tw, ptw, pp_total_, pp_ld_, r1_, r2_, es,
-                                       ncols, os, ngroups);
-            else
-                launch2p_cw<R, INV, 4>(cls, nblocks, cw * L, shm, s, data, tw, ptw, pp_total_, pp_ld_, r1_, r2_, es,
-                                       ncols, os, ngroups);
-        };
-        if (mode == 1) go(std::true_type{});
-        else go(std::false_type{});
-        MPM_LAUNCH();
+        dense_.run<R>(data, tw, es, ncols, os, nouter, mode, scale, sz, sb, s);
         return;
     }
     if (kind == 1) {
@@ -1466,19 +820,6 @@ void AxisFFT::launch_line(cplx<R>* data, size_t es, int ncols, size_t os, int no
     // indexes the line's own twiddles)
     FftFactors f = f_;
     int cw = pick_cw(n, sizeof(cplx<R>), ncols, 0);
-    {
-        // few lines in all (a batch of a few grid columns): fewer columns per
-        // CTA, so that at least two CTAs per SM share the lines (a heuristic
-        // on the first device's SM count)
-        static const int sms = [] {
-            int d = 0, v = 148;
-            if (cudaGetDevice(&d) != cudaSuccess ||
-                cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d) != cudaSuccess)
-                v = 148;
-            return v;
-        }();
-        while (cw > 4 && (long long)nouter * ((ncols + cw - 1) / cw) < 2LL * sms) cw /= 2;
-    }
     // (only when that costs no columns per CTA)
     if (fft_smem(n, cw, sizeof(cplx<R>), f.pt_total) > kFftSmemBudget) f.pt_total = 0;
     const int pt_total = f.pt_total;

@@ -30,6 +30,26 @@ struct FftFactors {
     int pt_total = 0;     // entries of all tables together
 };
 
+// Line transform of n = r1 * m points by an in-register radix-r1 pass and
+// m-point DFTs as products with their tables (mpm_dense.cu).  r1 = 0: off.
+class DenseDFT {
+public:
+    void init(int n, int r1);
+    // whether a tile of four columns fits in shared memory
+    bool fits(bool fp64) const;
+    // as AxisFFT::run / run_scaled (mode 2: two launches); tw: W_n^t, t < n
+    template <typename R>
+    void run(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, size_t os, int nouter, int mode, const R* scale,
+             int sz, int sb, cudaStream_t s) const;
+
+private:
+    template <typename R>
+    void launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, size_t os, int nouter, bool inverse,
+                const R* scale, int sz, int sb, cudaStream_t s) const;
+    int n_ = 0, r1_ = 0, m_ = 0, H_ = 0, ld_ = 0;
+    DevBuf t64_, t32_;   // [H][2][ld]: cos, sin of 2 pi p q / m
+};
+
 class AxisFFT {
 public:
     void init(int n);
@@ -46,23 +66,26 @@ public:
                     cudaStream_t s) const;
     // whether one line of this length fits in shared memory
     static bool fits(int n, bool fp64);
-    // the two-pass split n = r1 * r2: both in-register radices (r1 >= r2), or
-    // r1 in-register and r2 a prime above 16 (streamed); (0, 0) if neither
+    // the split n = r1 * r2: both in-register radices (r1 >= r2), or r1
+    // in-register and r2 a prime above 16; (0, 0) if neither
     int split_r1() const { return r1_; }
     int split_r2() const { return r2_; }
     // run every length through the general multi-pass kernel (tests)
     void set_force_general(bool v) { force_general_ = v; }
-    // kernel a transform of ncols columns takes: 0 general multi-pass,
-    // 1 two-pass in registers, 2 two-pass with a streamed prime pass, 3
-    // two-pass with a Rader prime pass (modes 0 forward, 1 inverse, 2
-    // forward-scale-inverse; 2 has no prime variant)
-    int path(int ncols, int mode) const {
-        if (!r1_ || ncols < 16 || force_general_) return 0;
-        if (kind_ >= 2 && mode == 2) return 0;
-        return kind_;
+    // kernel a transform of ncols columns takes: 1 two-pass in registers (both
+    // factors in-register radices, at least half a tile of columns per line),
+    // 2 in-register radix times table product (mpm_dense.cu: lengths with one
+    // prime above 16, few columns per line, other lengths with a short rest),
+    // 0 general multi-pass
+    int path(int ncols, bool fp64) const {
+        if (force_general_) return 0;
+        if (kind_ == 1 && ncols >= 16) return 1;
+        return dense_.fits(fp64) ? 2 : 0;
     }
-    // the Rader split p - 1 = A * B (0 when the prime pass is streamed)
-    int rader_a() const { return ra_; }
+    // the split as mpm_line_fft reports it
+    bool reports_split(int ncols, int mode) const {
+        return r1_ && !force_general_ && ncols >= 16 && !(kind_ == 2 && mode == 2);
+    }
 
     // The k-space step of the pruned (z-slab) monodisperse grid fused with
     // this axis's transforms, for the y axis: data is the grid
@@ -91,14 +114,10 @@ private:
     static void upload_table(std::vector<double2> t64, DevBuf& d64, DevBuf& d32);
     FftFactors f_;
     int kind_ = 0, r1_ = 0, r2_ = 0;
-    int ra_ = 0, rb_ = 0;   // Rader split of r2_ - 1
-    DevBuf rt64_, rt32_;     // Rader tables: W_N^t, forward Bh, inverse Bh
-    DevBuf rperm_;           // Rader index maps: g^-q, g^m
     bool force_general_ = false;
     DevBuf tw64_, tw32_;
     DevBuf pt64_, pt32_;   // prime-pass twiddle tables (see FftFactors)
-    DevBuf pp64_, pp32_;   // the prime-streamed two-pass kernel's W_p^(p' q) table
-    int pp_total_ = 0, pp_ld_ = 0;
+    DenseDFT dense_;
 };
 
 }  // namespace mpm
