@@ -1415,14 +1415,134 @@ __global__ void __launch_bounds__(128) k_real(const double2* __restrict__ X, dou
 
 // -------------------------------------------------------------- direct ---
 
-// Open-boundary all-pairs field (direct_field_kernel,
-// direct_electric_field.cu:42-324).  Thread per target, blockIdx.y = rhs,
-// source tiles staged in shared memory.
-template <typename R>
+// Open-boundary all-pairs field of dipoles (direct_field_kernel,
+// direct_electric_field.cu:42-324), SOLVER_AX or at field points.
+//
+// A CTA of 128 threads takes TG targets and CB columns; each target has
+// 128 / TG threads, which take every (128 / TG)-th source, and their sums
+// meet in shared memory in a fixed order.  A pair's tensor
+// T = (3 u u - 1) k / r^3 (one division, one square root) is formed once for
+// its CB columns, 18 FMAs each, against moments that the CTA stages in shared
+// memory (one broadcast read per value).  Bound by the fp64 (fp32) FMA rate
+// where the columns are many, by the chain of a thread's sources where the
+// system is small: hence few targets per CTA there.  One thread per target
+// and column, each with its own geometry, took 1150 us for N = 2000 with 30
+// columns in fp64 (416 here) and 27 us for N = 100 with 3 in fp32
+// (8 us).
+constexpr int kDirectTile = 64;    // sources staged at a time
+
+template <typename R, int CB, int TG>
 __global__ void __launch_bounds__(128) k_direct(const double2* __restrict__ X, double2* __restrict__ Y, int M, int N,
                                                 int Nt, const double* __restrict__ src,
                                                 const double* __restrict__ tgt, const double* __restrict__ rad,
-                                                const int* __restrict__ quad_map, int quads,
+                                                const double2* __restrict__ sc, int solver_ax, int jacobi) {
+    constexpr int SL = 128 / TG;   // source slices
+    constexpr int kStage = kDirectTile * (3 * CB * int(sizeof(cplx<R>)) + 4 * int(sizeof(R)));
+    constexpr int kRed = 128 * 3 * CB * int(sizeof(cplx<R>));
+    __shared__ __align__(16) unsigned char smem[kStage > kRed ? kStage : kRed];
+    cplx<R>* sp = reinterpret_cast<cplx<R>*>(smem);               // [kDirectTile][3][CB]
+    R* sx = reinterpret_cast<R*>(sp + kDirectTile * 3 * CB);       // [4][kDirectTile]: x, y, z, radius^2
+    const int tl = threadIdx.x % TG, slice = threadIdx.x / TG;
+    const int j = blockIdx.x * TG + tl;
+    const int m0 = blockIdx.y * CB;
+    const int mc = min(CB, M - m0);
+    const bool live = j < Nt;
+    const R k4 = R(1.0 / (4.0 * kPi)) * (solver_ax ? R(-1) : R(1));
+    const R jx = live ? R(tgt[j]) : R(0), jy = live ? R(tgt[Nt + j]) : R(0), jz = live ? R(tgt[2 * Nt + j]) : R(0);
+    const R eps_orig = sizeof(R) == 4 ? R(1e-6) : R(1e-9);
+    const R eps_sing = sizeof(R) == 4 ? R(1e-12) : R(1e-18);
+    cplx<R> E[3][CB];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int b = 0; b < CB; ++b) E[c][b] = mk<R>(R(0), R(0));
+    for (int t0 = 0; t0 < N; t0 += kDirectTile) {
+        const int te = min(kDirectTile, N - t0);
+        __syncthreads();
+        for (int t = threadIdx.x; t < te * 3 * CB; t += 128) {
+            const int b = t % CB, row = t / CB;                    // row = 3 source + component
+            sp[t] = b < mc ? to_r<R>(X[(size_t(3) * t0 + row) * M + m0 + b]) : mk<R>(R(0), R(0));
+        }
+        for (int t = threadIdx.x; t < 4 * te; t += 128) {
+            const int c = t / te, i = t - c * te;
+            if (c < 3) sx[c * kDirectTile + i] = R(src[size_t(c) * N + t0 + i]);
+            else {
+                const R a = rad ? R(rad[t0 + i]) : R(0);
+                sx[c * kDirectTile + i] = a * a;
+            }
+        }
+        __syncthreads();
+        if (!live) continue;
+        for (int k = slice; k < te; k += SL) {
+            if (solver_ax && t0 + k == j) continue;
+            R rx = sx[k] - jx, ry = sx[kDirectTile + k] - jy, rz = sx[2 * kDirectTile + k] - jz;
+            R r2 = rx * rx + ry * ry + rz * rz;
+            const R md2 = sx[3 * kDirectTile + k];
+            if (r2 < md2) {          // inside the source sphere: moved to its surface
+                if (sqrt(r2) > eps_orig) {
+                    const R scl = sqrt(md2 / r2);
+                    rx *= scl; ry *= scl; rz *= scl;
+                }
+                r2 = md2;
+            }
+            if (r2 < eps_sing) continue;
+            const R ir2 = R(1) / r2, ir = sqrt(ir2);
+            const R df = k4 * ir2 * ir, t3 = R(3) * df;
+            rx *= ir; ry *= ir; rz *= ir;
+            const R tx = t3 * rx, ty = t3 * ry;
+            const R xx = tx * rx - df, yy = ty * ry - df, zz = t3 * rz * rz - df;
+            const R xy = tx * ry, xz = tx * rz, yz = ty * rz;
+            const cplx<R>* p = sp + k * 3 * CB;
+#pragma unroll
+            for (int b = 0; b < CB; ++b) {
+                const cplx<R> px = p[b], py = p[CB + b], pz = p[2 * CB + b];
+                fma_rc(E[0][b], xx, px); fma_rc(E[0][b], xy, py); fma_rc(E[0][b], xz, pz);
+                fma_rc(E[1][b], xy, px); fma_rc(E[1][b], yy, py); fma_rc(E[1][b], yz, pz);
+                fma_rc(E[2][b], xz, px); fma_rc(E[2][b], yz, py); fma_rc(E[2][b], zz, pz);
+            }
+        }
+    }
+    __syncthreads();
+    // the slices' sums: [3 CB][128] values, then one thread per (component, column, target)
+    cplx<R>* red = reinterpret_cast<cplx<R>*>(smem);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int b = 0; b < CB; ++b) red[(c * CB + b) * 128 + threadIdx.x] = E[c][b];
+    __syncthreads();
+    for (int u = threadIdx.x; u < 3 * CB * TG; u += 128) {
+        // b fastest: neighbouring threads write neighbouring columns
+        const int b = u % CB, w = u / CB, c = w % 3, tt = w / 3;
+        const int jj = blockIdx.x * TG + tt;
+        if (b >= mc || jj >= Nt) continue;
+        cplx<R> e = mk<R>(R(0), R(0));
+        for (int q = 0; q < SL; ++q) e += red[(c * CB + b) * 128 + q * TG + tt];
+        const int m = m0 + b;
+        const size_t o = size_t(3 * jj + c) * M + m;
+        double2 v = to_d(e);
+        double2 s = make_double2(0.0, 0.0);
+        if (sc && (solver_ax || jacobi)) s = sc[size_t(jj) * M + m];
+        if (solver_ax) {
+            const double rj = rad ? rad[jj] : 1.0;
+            const double corr = (1.0 / (4.0 * kPi)) / (rj * rj * rj);
+            v += make_double2(s.x + corr, s.y) * X[o];
+        }
+        if (jacobi && sc) {
+            if (!solver_ax) s = make_double2(0.0, 0.0);
+            const double den = s.x * s.x + s.y * s.y;
+            if (den > 1e-30) v = v * make_double2(s.x / den, -s.y / den);
+        }
+        Y[o] = v;
+    }
+}
+
+// The same with quadrupoles.  Thread per target, blockIdx.y = rhs, source
+// tiles staged in shared memory.
+template <typename R>
+__global__ void __launch_bounds__(128) k_direct_quads(const double2* __restrict__ X, double2* __restrict__ Y, int M,
+                                                      int N, int Nt, const double* __restrict__ src,
+                                                const double* __restrict__ tgt, const double* __restrict__ rad,
+                                                const int* __restrict__ quad_map,
                                                 const double2* __restrict__ sc, int solver_ax, int jacobi) {
     constexpr int TILE = 128;
     __shared__ R sx[TILE], sy[TILE], sz[TILE], sr[TILE];
@@ -1434,7 +1554,7 @@ __global__ void __launch_bounds__(128) k_direct(const double2* __restrict__ X, d
     const R k4 = inv4pi * (solver_ax ? R(-1) : R(1));
     const R jx = j < Nt ? R(tgt[j]) : R(0), jy = j < Nt ? R(tgt[Nt + j]) : R(0),
             jz = j < Nt ? R(tgt[2 * Nt + j]) : R(0);
-    const int qt = (quads && j < N && j < Nt) ? quad_map[j] : -1;
+    const int qt = (j < N && j < Nt) ? quad_map[j] : -1;
     cplx<R> E[3] = {mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0)};
     cplx<R> G[5] = {mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0), mk<R>(0, 0)};
     const R eps_orig = sizeof(R) == 4 ? R(1e-6) : R(1e-9);
@@ -1445,7 +1565,7 @@ __global__ void __launch_bounds__(128) k_direct(const double2* __restrict__ X, d
             sx[threadIdx.x] = R(src[s]); sy[threadIdx.x] = R(src[N + s]); sz[threadIdx.x] = R(src[2 * N + s]);
             sr[threadIdx.x] = rad ? R(rad[s]) : R(0);
             for (int c = 0; c < 3; ++c) sp[threadIdx.x][c] = to_r<R>(X[size_t(3 * s + c) * M + m]);
-            const int qs = quads ? quad_map[s] : -1;
+            const int qs = quad_map[s];
             for (int c = 0; c < 5; ++c)
                 sq[threadIdx.x][c] = qs >= 0 ? to_r<R>(X[size_t(3 * N + 5 * qs + c) * M + m]) : mk<R>(0, 0);
         }
@@ -1477,7 +1597,7 @@ __global__ void __launch_bounds__(128) k_direct(const double2* __restrict__ X, d
                 E[0] += (pr * (R(3) * ux) - px) * df;
                 E[1] += (pr * (R(3) * uy) - py) * df;
                 E[2] += (pr * (R(3) * uz) - pz) * df;
-                if (quads) {
+                {
                     const cplx<R> q0 = sq[k][0] * R(-1), q1 = sq[k][1] * R(-2), q2 = sq[k][2] * R(-2),
                                   q3 = sq[k][3] * R(-1), q4 = sq[k][4] * R(-2);
                     const cplx<R> qzz = (q0 + q3) * R(-1);
@@ -2308,14 +2428,38 @@ void Field::real_part(const double2* X, double2* Y, int M, const double2* sc, bo
 void Field::direct(const double2* X, double2* Y, int M, const double2* sc, bool jacobi, bool fp32, cudaStream_t s) {
     const int nt = num_targets();
     const double* tg = spec_.solver_ax ? sources_.xyz.as<double>() : targets_.xyz.as<double>();
-    dim3 grd(nblk(nt, 128), M);
     StageScope scope(ST_DIRECT, s);
-    if (fp32)
-        k_direct<float><<<grd, 128, 0, s>>>(X, Y, M, N_, nt, sources_.xyz.as<double>(), tg, radius_.as<double>(),
-                                            quad_map_.as<int>(), Nq_ > 0, sc, spec_.solver_ax, jacobi);
-    else
-        k_direct<double><<<grd, 128, 0, s>>>(X, Y, M, N_, nt, sources_.xyz.as<double>(), tg, radius_.as<double>(),
-                                             quad_map_.as<int>(), Nq_ > 0, sc, spec_.solver_ax, jacobi);
+    const double* src = sources_.xyz.as<double>();
+    const double* rad = radius_.as<double>();
+    if (Nq_ > 0) {
+        dim3 grd(nblk(nt, 128), M);
+        if (fp32)
+            k_direct_quads<float><<<grd, 128, 0, s>>>(X, Y, M, N_, nt, src, tg, rad, quad_map_.as<int>(), sc,
+                                                      spec_.solver_ax, jacobi);
+        else
+            k_direct_quads<double><<<grd, 128, 0, s>>>(X, Y, M, N_, nt, src, tg, rad, quad_map_.as<int>(), sc,
+                                                       spec_.solver_ax, jacobi);
+        MPM_LAUNCH();
+        return;
+    }
+    auto go = [&](auto kern, int cb, int tgs) {
+        kern<<<dim3(nblk(nt, tgs), nblk(M, cb)), 128, 0, s>>>(X, Y, M, N_, nt, src, tg, rad, sc, spec_.solver_ax,
+                                                              jacobi);
+    };
+    // columns per CTA: one or three (a frequency's polarisations) in one CTA,
+    // else six, the most whose sums stay in registers.  Targets per CTA: 32,
+    // or 8 (each target's sources over 16 threads) while 32 would leave the
+    // GPU short of four CTAs per SM.
+    auto pick = [&](auto rc) {
+        using R = decltype(rc);
+        const int cb = M == 1 ? 1 : M <= 3 ? 3 : 6;
+        const bool wide = (long long)nblk(nt, 32) * nblk(M, cb) >= 4 * 148;
+        if (cb == 1) wide ? go(k_direct<R, 1, 32>, 1, 32) : go(k_direct<R, 1, 8>, 1, 8);
+        else if (cb == 3) wide ? go(k_direct<R, 3, 32>, 3, 32) : go(k_direct<R, 3, 8>, 3, 8);
+        else wide ? go(k_direct<R, 6, 32>, 6, 32) : go(k_direct<R, 6, 8>, 6, 8);
+    };
+    if (fp32) pick(float{});
+    else pick(double{});
     MPM_LAUNCH();
 }
 
