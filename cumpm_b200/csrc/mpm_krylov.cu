@@ -48,18 +48,76 @@ __global__ void __launch_bounds__(256) k_dots1(const double2* __restrict__ V, si
     }
 }
 
-// k_dots1 + k_dots2 for few columns (M < 16): threads run over the flat
-// [row][M] elements, (256 / M) * M of them per CTA, so that each thread
-// keeps one column m for the whole grid-stride loop (the stride is a
-// multiple of M); the CTA's per-column sums are taken over the threads of
-// that column in a fixed order and written as k_dots1's partials.  The last
-// CTA of each vector group to finish (a counter per group, no waiting) then
-// reduces the partials exactly as k_dots2 does (lanes over CTAs, fixed
-// shuffle tree) into out, and resets its counter.
+// Few columns (M < 16): threads run over the flat [row][M] elements, L =
+// (256 / M) * M of them per CTA, so that each thread keeps one column for the
+// whole grid-stride loop.
+
+// The CTA's per-column sums of acc[0 .. nv) into out[k * M + m]: 2 to 8 lanes
+// per sum (as many as the 256 threads give), a fixed shuffle tree.  One
+// thread per sum walked up to 85 values in shared memory one after another.
+__device__ __forceinline__ void cta_column_sums(const double2 (&acc)[8], int nv, int M, int L, double2 (*red)[256],
+                                                double2* __restrict__ out) {
+    const int j = threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) red[k][j] = acc[k];
+    __syncthreads();
+    const int n = nv * M;
+    const int gs = n <= 32 ? 8 : n <= 64 ? 4 : 2;      // n <= 8 * 15
+    const int o = j / gs, sl = j % gs;
+    const bool live = o < n;
+    const int k = live ? o / M : 0, m = live ? o - k * M : 0;
+    double2 sum = make_double2(0, 0);
+    if (live)
+        for (int q = m + sl * M; q < L; q += gs * M) sum += red[k][q];
+    for (int off = gs / 2; off > 0; off >>= 1) {
+        sum.x += __shfl_xor_sync(0xffffffffu, sum.x, off);
+        sum.y += __shfl_xor_sync(0xffffffffu, sum.y, off);
+    }
+    if (live && sl == 0) out[o] = sum;
+    __syncthreads();
+}
+
+// true in every thread of the last CTA of `total` to get here (one counter,
+// no waiting); everything the others wrote before is then visible
+__device__ __forceinline__ bool last_cta(unsigned int* done, unsigned int total) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(done, 1u) == total - 1;
+        if (last) *done = 0u;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0;
+}
+
+// sums over the gx CTAs of partial[b][n] into out (shared or global): eight
+// lanes per sum, a fixed shuffle tree
+__device__ __forceinline__ void reduce_partials(const double2* __restrict__ partial, int gx, int n,
+                                                double2* __restrict__ out) {
+    const int g = threadIdx.x >> 3, sl = threadIdx.x & 7;
+    for (int o0 = 0; o0 < n; o0 += 32) {
+        const int o = o0 + g;
+        double2 sum = make_double2(0, 0);
+        if (o < n) {
+#pragma unroll 4
+            for (int b = sl; b < gx; b += 8) sum += __ldcg(&partial[size_t(b) * n + o]);
+        }
+        for (int off = 4; off > 0; off >>= 1) {
+            sum.x += __shfl_xor_sync(0xffffffffu, sum.x, off);
+            sum.y += __shfl_xor_sync(0xffffffffu, sum.y, off);
+        }
+        if (o < n && sl == 0) out[o] = sum;
+    }
+}
+
+// k_dots1 + k_dots2 for few columns in one launch: the last CTA reduces the
+// partials; nrm (may be null) takes the square roots of the sums' real parts
 __global__ void __launch_bounds__(256) k_dots1s(const double2* __restrict__ V, size_t vstride, int nvec,
                                                 const double2* __restrict__ w, int rows, int M, int conj,
-                                                double2* __restrict__ partial, int shift,
-                                                double2* __restrict__ out, unsigned int* __restrict__ done) {
+                                                double2* __restrict__ partial, double2* __restrict__ out,
+                                                double* __restrict__ nrm, unsigned int* __restrict__ done) {
     __shared__ double2 red[8][256];
     const int L = (256 / M) * M;
     const int j = threadIdx.x;
@@ -70,45 +128,24 @@ __global__ void __launch_bounds__(256) k_dots1s(const double2* __restrict__ V, s
     for (int k = 0; k < 8; ++k) acc[k] = make_double2(0, 0);
     if (j < L) {
         for (size_t t = size_t(blockIdx.x) * L + j; t < n; t += size_t(gridDim.x) * L) {
-            double2 wv = w[t];
-            if (shift >= 0) wv -= V[size_t(shift) * vstride + t];
+            const double2 wv = w[t];
             // a fixed trip count, so that the group's loads issue together
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 if (k >= nv) break;
-                const double2 v = (shift >= 0 && i0 + k == nvec - 1) ? wv : V[size_t(i0 + k) * vstride + t];
+                const double2 v = V[size_t(i0 + k) * vstride + t];
                 if (conj) acc[k] += conjmul(v, wv);
                 else acc[k] += v * wv;
             }
         }
     }
-    for (int k = 0; k < 8; ++k) red[k][j] = acc[k];
-    __syncthreads();
-    if (j < nv * M) {
-        const int k = j / M, m = j % M;
-        double2 sum = make_double2(0, 0);
-        for (int q = m; q < L; q += M) sum += red[k][q];
-        partial[(size_t(blockIdx.x) * nvec + i0 + k) * M + m] = sum;
+    cta_column_sums(acc, nv, M, L, red, partial + (size_t(blockIdx.x) * nvec + i0) * M);
+    if (!last_cta(done, gridDim.x * gridDim.z)) return;
+    reduce_partials(partial, gridDim.x, nvec * M, out);
+    if (nrm) {
+        __syncthreads();
+        if (j < M) nrm[j] = sqrt(fmax(out[j].x, 0.0));
     }
-    __threadfence();
-    __syncthreads();
-    __shared__ int last;
-    if (j == 0) last = atomicAdd(&done[blockIdx.z], 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const int lane = j & 31, warp = j >> 5;
-    for (int o = warp; o < nv * M; o += 8) {
-        const int t = (i0 + o / M) * M + o % M;
-        double2 sum = make_double2(0, 0);
-        for (int b = lane; b < int(gridDim.x); b += 32) sum += __ldcg(&partial[size_t(b) * nvec * M + t]);
-        for (int off = 16; off > 0; off >>= 1) {
-            sum.x += __shfl_xor_sync(0xffffffffu, sum.x, off);
-            sum.y += __shfl_xor_sync(0xffffffffu, sum.y, off);
-        }
-        if (lane == 0) out[t] = sum;
-    }
-    if (j == 0) done[blockIdx.z] = 0u;
 }
 
 // one warp per output: lanes stride over the per-CTA partials, then a fixed
@@ -226,31 +263,44 @@ __global__ void k_normalize(const double2* __restrict__ src, double2* __restrict
 // The operator writes A V_k straight into V_{k+1}, so one pass of k_dots1 over
 // the k+2 vectors V_0..V_{k+1} gives h_i = V_i^H u (i <= k) and |u|^2 (i =
 // k+1) for u = w - V_k (then h_k(w) = h_k(u) + 1; u has the same projection
-// remainder w' as w).  Classical Gram-Schmidt with selective
-// re-orthogonalisation: after the projection |w'|^2 = |u|^2 - |h(u)|^2
-// (Pythagoras, V orthonormal); a column whose norm dropped below 0.7 |u|
-// (|w'|^2 <= 0.49 |u|^2, where that difference loses digits and
-// orthogonality may suffer) takes a second projection (Kahan and Parlett's
-// "twice is enough" test); the others are finished after one.  The Givens rotation of a column uses the final h and
-// |w'|; k_arn_update projects and normalises V_{k+1} in place.
+// remainder w' as w).  Every column takes two projections (CGS2); the norm of
+// the second remainder follows by Pythagoras.  The Givens rotation of a column
+// uses the final h and |w'|; the last launch projects and normalises V_{k+1}
+// in place.
 
-// Givens update of Hessenberg column k of one right-hand side (the previous
-// rotations, a new rotation, the residual estimate; gmres_solver.cu:120-184)
+// Givens update of Hessenberg column k of one right-hand side (h[i * M + m],
+// i <= k, plus `shift` on the diagonal; the previous rotations, a new rotation, the residual estimate; gmres_solver.cu:120-184)
 __device__ void gm_givens(GState& s, const double2* __restrict__ h, double wn, double2* __restrict__ Hm,
                           double2* __restrict__ gm, double* __restrict__ csm, double2* __restrict__ snm, int k,
-                          int ld, int M, int m, int restart, double tolm, double bnm, int maxiter) {
+                          int ld, int M, int m, int restart, double tolm, double bnm, int maxiter,
+                          double2 shift = make_double2(0.0, 0.0)) {
     double2* col = Hm + size_t(k) * ld;
     // the previous rotations applied down the column, the running entry in
     // a register (the column's inputs and the rotations are independent loads)
     double2 carry = h[m];
-#pragma unroll 4
-    for (int i = 0; i < k; ++i) {
-        const double2 h2 = h[size_t(i + 1) * M + m];
-        const double c = csm[i];
-        const double2 sv = snm[i];
-        const double2 cs_ = make_double2(sv.x, -sv.y);
-        col[i] = carry * c + cs_ * h2;
-        carry = (sv * carry) * -1.0 + h2 * c;
+    if (k == 0) carry += shift;
+    for (int i0 = 0; i0 < k; i0 += 8) {
+        // eight rotations loaded before any is used
+        double c8[8];
+        double2 s8[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (i0 + u < k) {
+                c8[u] = csm[i0 + u];
+                s8[u] = snm[i0 + u];
+            }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (i0 + u < k) {
+                const int i = i0 + u;
+                double2 h2 = h[size_t(i + 1) * M + m];
+                if (i + 1 == k) h2 += shift;
+                const double c = c8[u];
+                const double2 sv = s8[u];
+                const double2 cs_ = make_double2(sv.x, -sv.y);
+                col[i] = carry * c + cs_ * h2;
+                carry = (sv * carry) * -1.0 + h2 * c;
+            }
     }
     const double2 h1 = carry, h2 = make_double2(wn, 0.0);
     double c = 1.0;
@@ -287,81 +337,64 @@ __device__ void gm_givens(GState& s, const double2* __restrict__ h, double wn, d
     }
 }
 
-// givens = 0 (the seeds of a shifted solve): |w'| and the normalisation
-// only; the Givens updates are the members' (shift_givens_body).  always2:
-// every column takes the second projection (CGS2); else only those that
-// fail the 0.7 test.
-// pass 1: hh = [V_0..V_k, w]^H w.  Columns whose projection keeps |w'| >
-// 0.7 |w| get |w'| by Pythagoras and their Givens update now; the others are
-// marked for a second pass.  pass 2 (marked columns, hh2 = [V_0..V_k, w']^H w'
-// after the first projection): h += h2, |w''| likewise, Givens.  Thread per
-// column; one CTA: flag[0] = columns still cycling, flag[1 + m] = column m
-// cycling, flag[1 + M] = columns marked for the second pass.
+// The one-CTA kernel after a projection's sums.  pass 1, h = [V_0..V_k, u]^H u
+// with u = w - V_k: h_k += 1 (the coefficients of w) and the cycling columns
+// marked for their second projection.  pass 2, h2 = [V_0..V_k, w']^H w' after
+// the first: h += h2, |w''| by Pythagoras, the Givens update (givens = 0, the
+// seeds of a shifted solve: none, they are the members', shift_givens_body).
+// flag[0] = columns still cycling, flag[1 + m] = column m cycling.
 __device__ __forceinline__ void arn_finish_body(GState* __restrict__ st, double2* __restrict__ h,
-                                                const double2* __restrict__ h2, int pass, int givens, int always2,
+                                                const double2* __restrict__ h2, int pass, int givens,
                                                 double* __restrict__ nu_out, double* __restrict__ inv_nu,
                                                 double2* __restrict__ H, double2* __restrict__ g,
                                                 double* __restrict__ cs, double2* __restrict__ sn, int k, int restart,
                                                 int M, const double* __restrict__ bn, double tol,
                                                 const double* __restrict__ tolv, int maxiter,
                                                 int* __restrict__ flag) {
-    __shared__ int ncyc, nreo;
-    if (threadIdx.x == 0) ncyc = nreo = 0;
+    if (pass == 1) {
+        for (int m = threadIdx.x; m < M; m += blockDim.x) {
+            const int cyc = st[m].cyc;
+            st[m].reorth = cyc ? 1 : 0;
+            if (cyc) h[size_t(k) * M + m].x += 1.0;
+        }
+        return;
+    }
+    __shared__ int ncyc;
+    if (threadIdx.x == 0) ncyc = 0;
+    // (columns not cycling have w' = 0, so h2 = 0)
+    for (int t = threadIdx.x; t < (k + 1) * M; t += blockDim.x) h[t] += h2[t];
     __syncthreads();
     const int ld = restart + 1;
-    int c_cyc = 0, c_reo = 0;
+    int c_cyc = 0;
     for (int m = threadIdx.x; m < M; m += blockDim.x) {
         GState s = st[m];
-        if (pass == 1) s.reorth = 0;
-        bool go = s.cyc && (pass == 1 || s.reorth == 1);
-        if (go) {
-            double wn2, hs = 0.0;
-            if (pass == 1) {
-                // h holds V^H u and |u|^2 for u = w - V_k: h_k(w) = h_k(u) + 1
-                wn2 = h[size_t(k + 1) * M + m].x;
-                for (int i = 0; i <= k; ++i) {
-                    const double2 v = h[size_t(i) * M + m];
-                    hs += v.x * v.x + v.y * v.y;
-                }
-                h[size_t(k) * M + m].x += 1.0;
-            } else {
-                wn2 = h2[size_t(k + 1) * M + m].x;
-                for (int i = 0; i <= k; ++i) {
-                    const double2 v = h2[size_t(i) * M + m];
-                    hs += v.x * v.x + v.y * v.y;
-                    h[size_t(i) * M + m] += v;
-                }
+        if (s.cyc && s.reorth == 1) {
+            const double wn2 = h2[size_t(k + 1) * M + m].x;
+            double hs = 0.0;
+#pragma unroll 8
+            for (int i = 0; i <= k; ++i) {
+                const double2 v = h2[size_t(i) * M + m];
+                hs += v.x * v.x + v.y * v.y;
             }
-            const double nu2 = wn2 - hs;
-            if (pass == 1 && (always2 || !(nu2 > 0.49 * wn2))) {
-                s.reorth = 1;   // second projection before the Givens update
-            } else {
-                const double nu = sqrt(fmax(nu2, 0.0));
-                inv_nu[m] = nu > 0.0 ? 1.0 / nu : 0.0;
-                if (nu_out) nu_out[m] = nu;
-                if (givens)
-                    gm_givens(s, h, nu, H + size_t(m) * ld * restart, g + size_t(m) * ld, cs + size_t(m) * restart,
-                              sn + size_t(m) * restart, k, ld, M, m, restart, col_tol(tol, tolv, m), bn[m],
-                              maxiter);
-                if (pass == 2) s.reorth = 2;
-            }
+            const double nu = sqrt(fmax(wn2 - hs, 0.0));
+            inv_nu[m] = nu > 0.0 ? 1.0 / nu : 0.0;
+            if (nu_out) nu_out[m] = nu;
+            if (givens)
+                gm_givens(s, h, nu, H + size_t(m) * ld * restart, g + size_t(m) * ld, cs + size_t(m) * restart,
+                          sn + size_t(m) * restart, k, ld, M, m, restart, col_tol(tol, tolv, m), bn[m], maxiter);
+            s.reorth = 2;
             st[m] = s;
         }
         c_cyc += s.cyc;
-        c_reo += s.reorth == 1;
         flag[1 + m] = s.cyc;
     }
     if (c_cyc) atomicAdd(&ncyc, c_cyc);
-    if (c_reo) atomicAdd(&nreo, c_reo);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        flag[0] = ncyc;
-        flag[1 + M] = nreo;
-    }
+    if (threadIdx.x == 0) flag[0] = ncyc;
 }
 
-__global__ void __launch_bounds__(1024) k_arn_finish(GState* __restrict__ st, double2* __restrict__ h,
-                                                     const double2* __restrict__ h2, int pass, int givens, int always2,
+__global__ void __launch_bounds__(256) k_arn_finish(GState* __restrict__ st, double2* __restrict__ h,
+                                                     const double2* __restrict__ h2, int pass, int givens,
                                                      double* __restrict__ nu_out,
                                                      double* __restrict__ inv_nu, double2* __restrict__ H,
                                                      double2* __restrict__ g, double* __restrict__ cs,
@@ -369,8 +402,8 @@ __global__ void __launch_bounds__(1024) k_arn_finish(GState* __restrict__ st, do
                                                      const double* __restrict__ bn, double tol,
                                                      const double* __restrict__ tolv, int maxiter,
                                                      int* __restrict__ flag) {
-    arn_finish_body(st, h, h2, pass, givens, always2, nu_out, inv_nu, H, g, cs, sn, k, restart, M, bn, tol, tolv,
-                    maxiter, flag);
+    arn_finish_body(st, h, h2, pass, givens, nu_out, inv_nu, H, g, cs, sn, k, restart, M, bn, tol, tolv, maxiter,
+                    flag);
 }
 
 // V_{k+1} -= sum_{i <= k} V_i h_i for the columns of this pass (pass 1: the
@@ -456,16 +489,14 @@ __global__ void k_col_equal(const double2* __restrict__ b, int rows, int M, int*
 }
 
 // member m of seed grp[m]: Hessenberg column k of the seed plus sigma_m on
-// the diagonal, then its Givens update (gm_givens).  pass 1 takes the members
-// of seeds finished after one projection, pass 2 those of seeds whose second
-// projection just finished (reorth 2); members of a seed still waiting for
-// its second projection keep it cycling.  A seed cycles while any member
-// does (written back to its state).  One CTA: flag[0] = seeds cycling,
+// the diagonal, then its Givens update (gm_givens), once the seed's second
+// projection is done (reorth 2).  A seed cycles while any member does
+// (written back to its state).  One CTA: flag[0] = seeds cycling,
 // flag[1 + g] = seed g cycling.
 __device__ __forceinline__ void shift_givens_body(GState* __restrict__ mst, GState* __restrict__ sst,
                                                   const double2* __restrict__ hs, const double* __restrict__ nu,
                                                   const double2* __restrict__ sigma, const int* __restrict__ grp,
-                                                  int G, int pass, double2* __restrict__ hm, double2* __restrict__ H,
+                                                  int G, double2* __restrict__ H,
                                                   double2* __restrict__ g, double* __restrict__ cs,
                                                   double2* __restrict__ sn, int k, int restart, int M,
                                                   const double* __restrict__ bs, const double* __restrict__ tolv,
@@ -479,16 +510,9 @@ __device__ __forceinline__ void shift_givens_body(GState* __restrict__ mst, GSta
         GState s = mst[m];
         if (!s.cyc) continue;
         const int gi = grp[m];
-        const int sr = sst[gi].reorth;
-        if (sr == 1) {              // second projection pending
-            atomicOr(&seed_cyc[gi], 1);
-            continue;
-        }
-        if (sr == (pass == 1 ? 0 : 2)) {
-            for (int i = 0; i <= k; ++i) hm[size_t(i) * M + m] = hs[size_t(i) * G + gi];
-            hm[size_t(k) * M + m] += sigma[m];
-            gm_givens(s, hm, nu[gi], H + size_t(m) * ld * restart, g + size_t(m) * ld, cs + size_t(m) * restart,
-                      sn + size_t(m) * restart, k, ld, M, m, restart, tolv[m], bs[gi], maxiter);
+        if (sst[gi].reorth == 2) {
+            gm_givens(s, hs, nu[gi], H + size_t(m) * ld * restart, g + size_t(m) * ld, cs + size_t(m) * restart,
+                      sn + size_t(m) * restart, k, ld, G, gi, restart, tolv[m], bs[gi], maxiter, sigma[m]);
             mst[m] = s;
         }
         if (s.cyc) atomicOr(&seed_cyc[gi], 1);
@@ -504,25 +528,150 @@ __device__ __forceinline__ void shift_givens_body(GState* __restrict__ mst, GSta
 }
 
 // The seeds' second projection (k_arn_finish pass 2, no Givens) and the
-// members' Givens updates (shift_givens_body, pass 2) in one CTA: the members
+// members' Givens updates (shift_givens_body) in one CTA: the members
 // read only the seeds' Hessenberg column and norm, which the first part
 // writes, so the seeds' normalisation of V_{k+1} can follow.
-__global__ void __launch_bounds__(1024) k_seed_finish_givens(GState* __restrict__ sst, double2* __restrict__ h,
-                                                             const double2* __restrict__ h2,
-                                                             double* __restrict__ nu, double* __restrict__ inv_nu,
-                                                             int k, int restart, int G, const double* __restrict__ bs,
-                                                             double tol, int maxiter, GState* __restrict__ mst,
-                                                             const double2* __restrict__ sigma,
-                                                             const int* __restrict__ grp, double2* __restrict__ hm,
-                                                             double2* __restrict__ H, double2* __restrict__ g,
-                                                             double* __restrict__ cs, double2* __restrict__ sn, int M,
-                                                             const double* __restrict__ tolv,
-                                                             int* __restrict__ seed_cyc, int* __restrict__ flag) {
-    arn_finish_body(sst, h, h2, 2, 0, 1, nu, inv_nu, nullptr, nullptr, nullptr, nullptr, k, restart, G, bs, tol,
-                    nullptr, maxiter, flag);
+struct MemberArgs {
+    GState* st;             // null: no members (plain GMRES)
+    const double2* sigma;
+    const int* grp;
+    int M;
+    const double* tolv;
+    int* seed_cyc;
+};
+
+// The Hessenberg / Givens state a finish works on (plain GMRES: of the columns
+// themselves; shifted solve: of the members)
+struct HessArgs {
+    double2* H;
+    double2* g;
+    double* cs;
+    double2* sn;
+    const double* bn;       // |b| per column (shifted: per seed)
+    double tol;
+    const double* tolv;
+    int maxiter, restart;
+    double* nu;             // |w'| per seed (shifted), or null
+    double* inv_nu;
+    int* flag;
+};
+
+__device__ __forceinline__ void finish2_body(GState* st, double2* h, const double2* h2, const HessArgs& a,
+                                             const MemberArgs& mb, int k, int M) {
+    const bool seeds = mb.st != nullptr;
+    arn_finish_body(st, h, h2, 2, seeds ? 0 : 1, a.nu, a.inv_nu, a.H, a.g, a.cs, a.sn, k, a.restart, M, a.bn, a.tol,
+                    seeds ? nullptr : a.tolv, a.maxiter, a.flag);
+    if (!seeds) return;
     __syncthreads();
-    shift_givens_body(mst, sst, h, nu, sigma, grp, G, 2, hm, H, g, cs, sn, k, restart, M, bs, tolv, maxiter,
-                      seed_cyc, flag);
+    shift_givens_body(mb.st, st, h, a.nu, mb.sigma, mb.grp, M, a.H, a.g, a.cs, a.sn, k, a.restart, mb.M, a.bn,
+                      mb.tolv, a.maxiter, mb.seed_cyc, a.flag);
+}
+
+__global__ void __launch_bounds__(256) k_seed_finish_givens(GState* __restrict__ sst, double2* __restrict__ h,
+                                                             const double2* __restrict__ h2, HessArgs a,
+                                                             MemberArgs mb, int k, int G) {
+    finish2_body(sst, h, h2, a, mb, k, G);
+}
+
+// ---- the Arnoldi step of few columns (M < 16) in three launches
+//
+// Each projection's sums, their reduction and the one-CTA kernel that follows
+// are one launch: the last CTA to finish reduces the partials and does the
+// finish.  The second launch also applies the first projection.  With the
+// launches separate (dots, finish, update, twice) a step took 44 to 66 us of
+// 5 to 15 us launches, all latency; 31 now (N = 4000, 3 columns, 5 steps).
+
+// pass 1: [V_0 .. V_k, u]^H u for u = w - V_k, then arn_finish_body pass 1
+__global__ void __launch_bounds__(256) k_arn_dots(const double2* __restrict__ V, size_t vstride, int k, int rows,
+                                                  int M, double2* __restrict__ partial, GState* __restrict__ st,
+                                                  double2* __restrict__ h, HessArgs a, unsigned int* __restrict__ done) {
+    __shared__ double2 red[8][256];
+    const int nvec = k + 2;
+    const int L = (256 / M) * M;
+    const int j = threadIdx.x;
+    const int i0 = blockIdx.z * 8;
+    const int nv = min(8, nvec - i0);
+    const size_t n = size_t(rows) * M;
+    const double2* w = V + size_t(k + 1) * vstride;
+    const double2* vk = V + size_t(k) * vstride;
+    double2 acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = make_double2(0, 0);
+    if (j < L) {
+        for (size_t t = size_t(blockIdx.x) * L + j; t < n; t += size_t(gridDim.x) * L) {
+            const double2 u = w[t] - vk[t];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (i >= nv) break;
+                const double2 v = i0 + i == nvec - 1 ? u : V[size_t(i0 + i) * vstride + t];
+                acc[i] += conjmul(v, u);
+            }
+        }
+    }
+    cta_column_sums(acc, nv, M, L, red, partial + (size_t(blockIdx.x) * nvec + i0) * M);
+    if (!last_cta(done, gridDim.x * gridDim.z)) return;
+    reduce_partials(partial, gridDim.x, nvec * M, h);
+    __syncthreads();
+    arn_finish_body(st, h, nullptr, 1, 0, nullptr, a.inv_nu, nullptr, nullptr, nullptr, nullptr, k, a.restart, M, a.bn,
+                    a.tol, nullptr, a.maxiter, a.flag);
+}
+
+// w' = w - sum_{i <= k} V_i h_i (columns not cycling: 0), then pass 2:
+// [V_0 .. V_k, w']^H w' into h2, h += h2, the norm and the Givens updates
+__global__ void __launch_bounds__(256) k_arn_project(double2* __restrict__ V, size_t vstride, int k, int rows, int M,
+                                                     double2* __restrict__ partial, GState* __restrict__ st,
+                                                     double2* __restrict__ h, double2* __restrict__ h2, HessArgs a,
+                                                     MemberArgs mb, unsigned int* __restrict__ done) {
+    __shared__ double2 red[8][256];
+    const int nvec = k + 2;
+    const int L = (256 / M) * M;
+    const int j = threadIdx.x;
+    const size_t n = size_t(rows) * M;
+    double2* w = V + size_t(k + 1) * vstride;
+    const size_t step = size_t(gridDim.x) * L;
+    const size_t t0 = size_t(blockIdx.x) * L + j;
+    const int m = j % M;
+    if (j < L) {
+        const bool mine = st[m].cyc != 0;
+        for (size_t t = t0; t < n; t += step) {
+            if (!mine) {
+                w[t] = make_double2(0, 0);
+                continue;
+            }
+            double2 a0 = make_double2(0, 0), a1 = a0, a2 = a0, a3 = a0;
+            int i = 0;
+            for (; i + 3 <= k; i += 4) {
+                a0 += V[size_t(i) * vstride + t] * h[size_t(i) * M + m];
+                a1 += V[size_t(i + 1) * vstride + t] * h[size_t(i + 1) * M + m];
+                a2 += V[size_t(i + 2) * vstride + t] * h[size_t(i + 2) * M + m];
+                a3 += V[size_t(i + 3) * vstride + t] * h[size_t(i + 3) * M + m];
+            }
+            for (; i <= k; ++i) a0 += V[size_t(i) * vstride + t] * h[size_t(i) * M + m];
+            w[t] = w[t] - ((a0 + a1) + (a2 + a3));
+        }
+    }
+    // (a thread reads back only what it wrote)
+    for (int i0 = 0; i0 < nvec; i0 += 8) {
+        const int nv = min(8, nvec - i0);
+        double2 acc[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = make_double2(0, 0);
+        if (j < L) {
+            for (size_t t = t0; t < n; t += step) {
+                const double2 u = w[t];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (i >= nv) break;
+                    acc[i] += conjmul(V[size_t(i0 + i) * vstride + t], u);
+                }
+            }
+        }
+        cta_column_sums(acc, nv, M, L, red, partial + (size_t(blockIdx.x) * nvec + i0) * M);
+    }
+    if (!last_cta(done, gridDim.x)) return;
+    reduce_partials(partial, gridDim.x, nvec * M, h2);
+    __syncthreads();
+    finish2_body(st, h, h2, a, mb, k, M);
 }
 
 // member states: active and cycling from the start, x0 = 0; g_m = (beta, 0..);
@@ -557,23 +706,45 @@ __global__ void k_shift_x(double2* __restrict__ x, const double2* __restrict__ V
     x[t] = acc;
 }
 
-// back substitution H y = g, y stored [i][m]
-__global__ void k_gm_backsub(const GState* __restrict__ st, const double2* __restrict__ H,
-                             const double2* __restrict__ g, double2* __restrict__ y, int restart, int M,
-                             int* __restrict__ kper) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
+// back substitution H y = g, y stored [i][m].  Warp per column, lanes over the
+// rows still to solve (the running right-hand side in shared memory): a step
+// divides one entry and subtracts its column of H, read contiguously and
+// ahead of its use.  One thread per column took 112 us for 30 columns of 14
+// steps.
+constexpr int kBacksubWarps = 4;
+
+__global__ void __launch_bounds__(kBacksubWarps * 32) k_gm_backsub(const GState* __restrict__ st,
+                                                                   const double2* __restrict__ H,
+                                                                   const double2* __restrict__ g,
+                                                                   double2* y, int restart, int M,
+                                                                   int* __restrict__ kper, int in_smem) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m = blockIdx.x * kBacksubWarps + warp;
+    if (m >= M) return;   // whole warps leave together
+    // the running right-hand side (in y itself when the restart is too long)
+    double2* v = in_smem ? reinterpret_cast<double2*>(smem_raw) + size_t(warp) * restart : y + m;
+    const size_t vs = in_smem ? 1 : size_t(M);
     const int k = st[m].kcount;
-    kper[m] = k;
+    if (lane == 0) kper[m] = k;
     const int ld = restart + 1;
     const double2* Hm = H + size_t(m) * ld * restart;
-    const double2* gm = g + size_t(m) * ld;
+    for (int i = lane; i < k; i += 32) v[i * vs] = g[size_t(m) * ld + i];
+    __syncwarp();
+    double2 d = k > 0 ? Hm[size_t(k - 1) * ld + k - 1] : make_double2(1.0, 0.0);
     for (int i = k - 1; i >= 0; --i) {
-        double2 v = gm[i];
-        for (int j = i + 1; j < k; ++j) v -= Hm[size_t(j) * ld + i] * y[size_t(j) * M + m];
-        const double2 d = Hm[size_t(i) * ld + i];
+        const double2* col = Hm + size_t(i) * ld;
+        const double2 dn = i > 0 ? Hm[size_t(i - 1) * ld + i - 1] : d;
+        const double2 c0 = lane < i ? col[lane] : make_double2(0, 0);
+        const double2 vi = v[i * vs];
         const double den = d.x * d.x + d.y * d.y;
-        y[size_t(i) * M + m] = make_double2((v.x * d.x + v.y * d.y) / den, (v.y * d.x - v.x * d.y) / den);
+        const double2 yi = make_double2((vi.x * d.x + vi.y * d.y) / den, (vi.y * d.x - vi.x * d.y) / den);
+        __syncwarp();      // every lane has read v[i]
+        if (lane == 0) y[size_t(i) * M + m] = yi;
+        if (lane < i) v[lane * vs] -= c0 * yi;
+        for (int l = lane + 32; l < i; l += 32) v[l * vs] -= col[l] * yi;
+        __syncwarp();
+        d = dn;
     }
 }
 
@@ -889,24 +1060,33 @@ int BatchSolver::apply_cols(Field& F, const double2* X, double2* Y, int M, const
     return Ma;
 }
 
+// CTAs of the few-column kernels over n elements: at most two per SM, so that
+// the last one's reduction stays short
+int BatchSolver::small_ctas(size_t n, int M) const {
+    const size_t L = size_t(256 / M) * M;
+    return int(std::max<size_t>(1, std::min<size_t>(296, (n + L - 1) / L)));
+}
+
+unsigned int* BatchSolver::done_counter(cudaStream_t s) {
+    if (!dots_done_.p) {
+        dots_done_.ensure(sizeof(unsigned int));
+        MPM_CUDA(cudaMemsetAsync(dots_done_.p, 0, sizeof(unsigned int), s));
+    }
+    return dots_done_.as<unsigned int>();
+}
+
 void BatchSolver::dots(const double2* V, size_t vstride, int nvec, const double2* w, int rows, int M, int conj,
-                       double2* out, cudaStream_t s, int shift) {
+                       double2* out, cudaStream_t s, int shift, double* nrm) {
     StageScope scope(ST_KRYLOV, s);
-    // four CTAs per SM: the sums are latency-bound, not bandwidth-bound
-    if (M < 16) {
-        const long long L = (256 / M) * M;
-        const int gx = int(std::max(1LL, std::min(592LL, (1LL * rows * M + L - 1) / L)));
-        const int nz = (nvec + 7) / 8;
+    if (M < 16 && shift < 0) {
+        const int gx = small_ctas(size_t(rows) * M, M);
         partial_.ensure(sizeof(double2) * size_t(gx) * nvec * M);
-        if (!dots_done_.p || dots_done_.bytes < sizeof(unsigned int) * size_t(nz)) {
-            dots_done_.ensure(sizeof(unsigned int) * std::max<size_t>(size_t(nz), 64));
-            MPM_CUDA(cudaMemsetAsync(dots_done_.p, 0, dots_done_.bytes, s));
-        }
-        k_dots1s<<<dim3(gx, 1, nz), 256, 0, s>>>(V, vstride, nvec, w, rows, M, conj, partial_.as<double2>(), shift,
-                                                 out, dots_done_.as<unsigned int>());
+        k_dots1s<<<dim3(gx, 1, (nvec + 7) / 8), 256, 0, s>>>(V, vstride, nvec, w, rows, M, conj,
+                                                             partial_.as<double2>(), out, nrm, done_counter(s));
         MPM_LAUNCH();
         return;
     }
+    // four CTAs per SM: the sums are latency-bound, not bandwidth-bound
     const int gx = std::max(1, std::min(592, (rows + 7) / 8));
     partial_.ensure(sizeof(double2) * size_t(gx) * nvec * M);
     dim3 grd(gx, (M + 31) / 32, (nvec + 7) / 8);
@@ -914,12 +1094,71 @@ void BatchSolver::dots(const double2* V, size_t vstride, int nvec, const double2
     MPM_LAUNCH();
     k_dots2<<<nblk((long long)nvec * M * 32, 256), 256, 0, s>>>(partial_.as<double2>(), gx, nvec, M, out);
     MPM_LAUNCH();
+    if (nrm) {
+        k_sqrt_re<<<nblk(M, 128), 128, 0, s>>>(out, M, nrm);
+        MPM_LAUNCH();
+    }
 }
 
 void BatchSolver::norms(const double2* w, int rows, int M, double* out, cudaStream_t s) {
     h2_.ensure(sizeof(double2) * M);
-    dots(w, 0, 1, w, rows, M, 1, h2_.as<double2>(), s);
-    k_sqrt_re<<<nblk(M, 128), 128, 0, s>>>(h2_.as<double2>(), M, out);
+    dots(w, 0, 1, w, rows, M, 1, h2_.as<double2>(), s, -1, out);
+}
+
+namespace {
+void backsub(const GState* st, const double2* H, const double2* g, double2* y, int restart, int M, int* kper,
+             cudaStream_t s) {
+    size_t shm = sizeof(double2) * kBacksubWarps * size_t(restart);
+    const int in_smem = shm <= 48 * 1024;
+    if (!in_smem) shm = 0;
+    k_gm_backsub<<<nblk(M, kBacksubWarps), kBacksubWarps * 32, shm, s>>>(st, H, g, y, restart, M, kper, in_smem);
+    MPM_LAUNCH();
+}
+}  // namespace
+
+// Orthogonalisation of V_{k+1} = A V_k against V_0 .. V_k, the Hessenberg
+// column and the Givens updates: CGS2, [V_0..V_k, u]^H u with u = w - V_k (the
+// preconditioned operator is close to the identity, so w is mostly V_k: the
+// first projection then works on the part that is not), w -= V h; then
+// [V_0..V_k, w']^H w', w' -= V h2, normalised.
+template <typename Hess, typename Member>
+void BatchSolver::arnoldi(double2* V, int k, int rows, int M, void* state, const Hess& a, const Member& mb,
+                          cudaStream_t s) {
+    GState* st = static_cast<GState*>(state);
+    const size_t n = size_t(rows) * M;
+    double2* h = h_.as<double2>();
+    double2* h2 = h2_.as<double2>();
+    const int vb = nblk((long long)n, 256);
+    StageScope scope(ST_KRYLOV, s);
+    if (M < 16) {
+        const int gx = small_ctas(n, M);
+        partial_.ensure(sizeof(double2) * size_t(gx) * (a.restart + 2) * M);
+        double2* part = partial_.as<double2>();
+        unsigned int* done = done_counter(s);
+        k_arn_dots<<<dim3(gx, 1, (k + 2 + 7) / 8), 256, 0, s>>>(V, n, k, rows, M, part, st, h, a, done);
+        MPM_LAUNCH();
+        k_arn_project<<<gx, 256, 0, s>>>(V, n, k, rows, M, part, st, h, h2, a, mb, done);
+        MPM_LAUNCH();
+    } else {
+        double2* w = V + size_t(k + 1) * n;
+        const bool seeds = mb.st != nullptr;
+        const int fthr = std::min(256, ((std::max(M, seeds ? mb.M : M) + 31) / 32) * 32);
+        dots(V, n, k + 2, w, rows, M, 1, h, s, k);
+        k_arn_finish<<<1, fthr, 0, s>>>(st, h, h2, 1, 0, nullptr, a.inv_nu, nullptr, nullptr, nullptr, nullptr, k,
+                                        a.restart, M, a.bn, a.tol, nullptr, a.maxiter, a.flag);
+        MPM_LAUNCH();
+        k_arn_update<<<vb, 256, 0, s>>>(V, n, k, h, st, a.inv_nu, rows, M, 1);
+        MPM_LAUNCH();
+        dots(V, n, k + 2, w, rows, M, 1, h2, s);
+        if (seeds) {
+            k_seed_finish_givens<<<1, fthr, 0, s>>>(st, h, h2, a, mb, k, M);
+        } else {
+            k_arn_finish<<<1, fthr, 0, s>>>(st, h, h2, 2, 1, nullptr, a.inv_nu, a.H, a.g, a.cs, a.sn, k, a.restart, M,
+                                            a.bn, a.tol, a.tolv, a.maxiter, a.flag);
+        }
+        MPM_LAUNCH();
+    }
+    k_arn_update<<<vb, 256, 0, s>>>(V, n, k, h2, st, a.inv_nu, rows, M, 2);
     MPM_LAUNCH();
 }
 
@@ -1010,45 +1249,19 @@ void BatchSolver::gmres(Field& F, const double2* b, double2* x, int M, const dou
         std::vector<int> cyc = begin_cols;
         for (int k = 0; k < restart; ++k) {
             double2* Vk = V + size_t(k) * n;
-            double2* w = V + size_t(k + 1) * n;   // A V_k lands in V_{k+1}, projected and normalised in place
+            double2* w = V + size_t(k + 1) * n;   // A V_k lands in V_{k+1}
             st.column_matvecs += apply_cols(F, Vk, w, M, sc, opt.jacobi, r32, re32, cyc.data(), opt.compact, s);
             st.matvecs++;
-            const int fthr = std::min(1024, ((M + 31) / 32) * 32);
-            auto finish = [&](int pass) {
-                k_arn_finish<<<1, fthr, 0, s>>>(gs, h_.as<double2>(), h2_.as<double2>(), pass, 1, 1, nullptr,
-                                                rnorm_.as<double>(), H_.as<double2>(), g_.as<double2>(), cs_.as<double>(),
-                                                sn_.as<double2>(), k, restart, M, bnorm_.as<double>(), opt.tol, tolv,
-                                                opt.maxiter, dflag);
-                MPM_LAUNCH();
-            };
-            auto update = [&](const double2* hv, int pass) {
-                k_arn_update<<<vb, 256, 0, s>>>(V, n, k, hv, gs, rnorm_.as<double>(), rows, M, pass);
-                MPM_LAUNCH();
-            };
-            // CGS2: [V_0..V_k, u]^H u with u = w - V_k (the preconditioned
-            // operator is close to the identity, so w is mostly V_k: the
-            // first projection then works on the part that is not), w -= V h;
-            // then [V_0..V_k, w']^H w', w' -= V h2, normalised; one flag read
-            dots(V, n, k + 2, w, rows, M, 1, h_.as<double2>(), s, k);
-            {
-                StageScope sc1(ST_KRYLOV, s);
-                finish(1);
-                update(h_.as<double2>(), 1);
-            }
-            dots(V, n, k + 2, w, rows, M, 1, h2_.as<double2>(), s);
-            {
-                StageScope sc2(ST_KRYLOV, s);
-                finish(2);
-                update(h2_.as<double2>(), 2);
-            }
+            HessArgs ha{H_.as<double2>(), g_.as<double2>(), cs_.as<double>(), sn_.as<double2>(), bnorm_.as<double>(),
+                        opt.tol, tolv, opt.maxiter, restart, nullptr, rnorm_.as<double>(), dflag};
+            arnoldi(V, k, rows, M, gs, ha, MemberArgs{}, s);
             st.reorth_steps++;
             // the count and the M column flags
             const int left = read_flags(dflag, M, s);
             if (left == 0) break;
             cyc.assign(flag_ + 1, flag_ + 1 + M);
         }
-        k_gm_backsub<<<mb, 128, 0, s>>>(gs, H_.as<double2>(), g_.as<double2>(), y_.as<double2>(), restart, M, kper);
-        MPM_LAUNCH();
+        backsub(gs, H_.as<double2>(), g_.as<double2>(), y_.as<double2>(), restart, M, kper, s);
         k_vupdate<<<vb, 256, 0, s>>>(x, V, n, restart, y_.as<double2>(), rows, M, 1.0, kper);
         MPM_LAUNCH();
     }
@@ -1138,7 +1351,6 @@ void BatchSolver::gmres_shifted(Field& F, const double2* b, double2* x, int M, c
     y_.ensure(sizeof(double2) * size_t(M) * restart);
     h_.ensure(sizeof(double2) * size_t(G) * (restart + 1));
     h2_.ensure(sizeof(double2) * size_t(G) * (restart + 1));
-    hm_.ensure(sizeof(double2) * size_t(M) * (restart + 1));
     state_.ensure(sizeof(GState) * M + sizeof(int) * M);
     // seed states, seed cycling flags, then |b~| and |w'| per seed (8-byte aligned)
     const size_t bs_off = (sizeof(GState) * G + sizeof(int) * G + 7) & ~size_t(7);
@@ -1168,45 +1380,21 @@ void BatchSolver::gmres_shifted(Field& F, const double2* b, double2* x, int M, c
     std::vector<int> used(G, live ? 0 : 1);
     for (int m = 0; m < M && live; ++m) used[grp[m]] |= live[m] != 0;
     for (int gi = 0; gi < G; ++gi) cyc[gi] = hbs[gi] > 0.0 && used[gi];
-    const int vb = nblk((long long)ns, 256);
-    const int fthr = std::min(1024, ((std::max(M, G) + 31) / 32) * 32);
     for (int k = 0; k < restart; ++k) {
         if (std::count(cyc.begin(), cyc.end(), 1) == 0) break;
         double2* Vk = V + size_t(k) * ns;
         double2* w = V + size_t(k + 1) * ns;
         st.column_matvecs += apply_cols(F, Vk, w, G, scs, true, r32, re32, cyc.data(), opt.compact, s);
         st.matvecs++;
-        auto seed_pass = [&](int pass, const double2* hv) {
-            // (every seed takes both projections: the members' Givens updates
-            // follow the second, in the same one-CTA kernel)
-            StageScope sc1(ST_KRYLOV, s);
-            if (pass == 1) {
-                k_arn_finish<<<1, fthr, 0, s>>>(sst, h_.as<double2>(), h2_.as<double2>(), pass, 0, 1, nu,
-                                                rnorm_.as<double>(), nullptr, nullptr, nullptr, nullptr, k, restart,
-                                                G, bs, opt.tol, nullptr, opt.maxiter, dflag);
-            } else {
-                k_seed_finish_givens<<<1, fthr, 0, s>>>(sst, h_.as<double2>(), h2_.as<double2>(), nu,
-                                                        rnorm_.as<double>(), k, restart, G, bs, opt.tol,
-                                                        opt.maxiter, mst, dsig, dgrp, hm_.as<double2>(),
-                                                        H_.as<double2>(), g_.as<double2>(), cs_.as<double>(),
-                                                        sn_.as<double2>(), M, tolv, scyc, dflag);
-            }
-            MPM_LAUNCH();
-            k_arn_update<<<vb, 256, 0, s>>>(V, ns, k, hv, sst, rnorm_.as<double>(), rows, G, pass);
-            MPM_LAUNCH();
-        };
-        dots(V, ns, k + 2, w, rows, G, 1, h_.as<double2>(), s, k);
-        seed_pass(1, h_.as<double2>());
-        dots(V, ns, k + 2, w, rows, G, 1, h2_.as<double2>(), s);
-        seed_pass(2, h2_.as<double2>());
+        HessArgs ha{H_.as<double2>(), g_.as<double2>(), cs_.as<double>(), sn_.as<double2>(), bs, opt.tol, nullptr,
+                    opt.maxiter, restart, nu, rnorm_.as<double>(), dflag};
+        arnoldi(V, k, rows, G, sst, ha, MemberArgs{mst, dsig, dgrp, M, tolv, scyc}, s);
         st.reorth_steps++;
         const int left = read_flags(dflag, G, s);
         if (left == 0) break;
         cyc.assign(flag_ + 1, flag_ + 1 + G);
     }
-    k_gm_backsub<<<nblk(M, 128), 128, 0, s>>>(mst, H_.as<double2>(), g_.as<double2>(), y_.as<double2>(), restart, M,
-                                              kper);
-    MPM_LAUNCH();
+    backsub(mst, H_.as<double2>(), g_.as<double2>(), y_.as<double2>(), restart, M, kper, s);
     k_shift_x<<<nblk((long long)rows * M, 256), 256, 0, s>>>(x, V, ns, G, y_.as<double2>(), dgrp, kper, skip, rows,
                                                              M);
     MPM_LAUNCH();

@@ -107,7 +107,11 @@ private:
                        const std::vector<int>& grp, const std::vector<double2>& f, const int* skip,
                        const int* live);
     void dots(const double2* V, size_t vstride, int nvec, const double2* w, int rows, int M, int conj,
-              double2* out, cudaStream_t s, int shift = -1);
+              double2* out, cudaStream_t s, int shift = -1, double* nrm = nullptr);
+    int small_ctas(size_t n, int M) const;
+    unsigned int* done_counter(cudaStream_t s);   // finished-CTA counter of the few-column kernels
+    template <typename Hess, typename Member>
+    void arnoldi(double2* V, int k, int rows, int M, void* state, const Hess& a, const Member& mb, cudaStream_t s);
     void norms(const double2* w, int rows, int M, double* out, cudaStream_t s);
 
     // reads the count and the nflags words that follow it into flag_
@@ -118,8 +122,8 @@ private:
     DevBuf cidx_, xc_, yc_, scc_;        // compact-batch gather buffers
     DevBuf bn2_, rn2_, convd_;           // refinement: |b|, true |r|, converged flags
     DevBuf sel_, rn64_;                  // refinement: columns re-checked in fp64, their |r|
-    DevBuf dots_done_;                   // finished-CTA counters of the fused small dot kernel
-    DevBuf shf_, shflag_, shmeta_, shsc_, shb_, shst_, hm_;   // shifted solve: detection, seeds, members
+    DevBuf dots_done_;                   // see done_counter
+    DevBuf shf_, shflag_, shmeta_, shsc_, shb_, shst_;   // shifted solve: detection, seeds, members
     int* flag_ = nullptr;                // pinned host words: count + per-column flags
     int flag_cap_ = 0;
     int* hidx_ = nullptr;                // pinned host column list for the gather
