@@ -187,10 +187,10 @@ __device__ void lookup_pair(double d, double a, double b, double xi, int tn, dou
 __global__ void k_poly_pair_dT(const double* __restrict__ pgeo, const int* __restrict__ off,
                                const int* __restrict__ src, int nt, const int* __restrict__ cls,
                                const double* __restrict__ crad, double xi, int table_n, double* __restrict__ dT) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;   // warp per target
     if (j >= nt) return;
     const double aj = crad[cls[j]];
-    for (int p = off[j]; p < off[j + 1]; ++p) {
+    for (int p = off[j] + (threadIdx.x & 31); p < off[j + 1]; p += 32) {
         const double ai = crad[cls[src[p]]];
         const double d = pgeo[4 * size_t(p) + 3];
         const double de = d < 1e-6 ? 1e-6 : d;
@@ -416,7 +416,7 @@ void Field::grad_bilinear(const double2* lam, const double2* p, int M, double2* 
         const size_t np = size_t(std::max<long long>(1, num_pairs_));
         pair_dT_.ensure(sizeof(double) * 4 * np);
         if (num_pairs_ > 0) {
-            k_poly_pair_dT<<<nblk(N_, 128), 128, 0, s>>>(pair_geo_.as<double>(), pair_off_.as<int>(),
+            k_poly_pair_dT<<<nblk((long long)N_ * 32, 128), 128, 0, s>>>(pair_geo_.as<double>(), pair_off_.as<int>(),
                                                          pair_src_.as<int>(), N_, pcls_.as<int>(), prad_.as<double>(),
                                                          spec_.xi, pgeom_.table_n, pair_dT_.as<double>());
             MPM_LAUNCH();

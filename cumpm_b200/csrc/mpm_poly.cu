@@ -17,8 +17,9 @@
 //    voxel's M columns are one coalesced vector.
 //  * Spreading is a gather over 8^3 voxel tiles from spatial bins of the
 //    stencil origins (no atomics, deterministic, every voxel written once).
-//  * Contraction is one CTA per target, its warps splitting the P^3 nodes,
-//    lanes over right-hand sides, a fixed-order reduction at the end.
+//  * Contraction is one CTA per target, its warps (and lane groups, for few
+//    right-hand sides) splitting the P^3 nodes, lanes over right-hand sides, a
+//    fixed-order reduction at the end.
 //  * The reference tabulates the pair functions on r = 0, 1, 1.001, ... for
 //    every pair of radius classes and interpolates linearly.  Here each
 //    pair's value is that same interpolation, but the two table nodes it
@@ -157,6 +158,15 @@ __device__ int poly_tile_bins(const PolyTile& t, int bx, int by, int bz, int (&b
     return nbv[0] * nbv[1] * nbv[2];
 }
 
+// index within a support of P nodes from `org` (cyclic in N) that voxel v falls
+// on, -1 outside (or past the grid)
+__device__ __forceinline__ int poly_support(int v, int org, int N, int P) {
+    if (v >= N) return -1;
+    int k = v - org;
+    if (k < 0) k += N;      // both are in [0, N)
+    return k < P ? k : -1;
+}
+
 // Candidate lists of the spread tiles, built once per frame: pass 0 counts
 // (and keeps the largest count), pass 1 writes each tile's list in bin
 // order at its CSR offset.
@@ -187,134 +197,196 @@ __global__ void k_poly_cands(PolyTile t, const int* __restrict__ bin_start, cons
     }
 }
 
-// Covered runs of every tile candidate, built once per frame (thread per
-// tile, candidates in list order).  The support index along an axis is
-// k = (t0 + u - origin) mod N and a tile offset u is covered when k < P;
-// within a covered run k grows by one per voxel (P < N, so a wrap would pass
-// N-1 >= P, which is not covered): at most two runs per axis.  Run word:
-// u | len << 4 | k << 8; word 6 holds the run counts (2 bits per axis).
-// Candidates that miss the tile along an axis are dropped, the others keep
-// their order (so each voxel's sum keeps its order): cnt[tile] of them at the
-// tile's CSR offset in clist / 8 words each in cruns.
-__global__ void k_poly_runs(PolyTile t, const int4* __restrict__ base, const int* __restrict__ off,
-                            const int* __restrict__ list, int* __restrict__ cnt, int* __restrict__ clist,
-                            int* __restrict__ cruns) {
-    const int tile = blockIdx.x * blockDim.x + threadIdx.x;
+// The tile candidates whose support covers the tile along every axis, built
+// once per frame: cnt[tile] of them at the tile's CSR offset in clist, in list
+// order (so each voxel's sum keeps its order).  Warp per tile, 32 candidates
+// per ballot (a thread per tile walked its list alone: 421 us for 125 tiles
+// of 80 candidates).
+__global__ void k_poly_filter(PolyTile t, const int4* __restrict__ base, const int* __restrict__ off,
+                              const int* __restrict__ list, int* __restrict__ cnt, int* __restrict__ clist) {
+    const int tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     const int ntile = t.nb[0] * t.nb[1] * t.nb[2];
-    if (tile >= ntile) return;
+    if (tile >= ntile) return;   // whole warps leave together
     const int bx = tile % t.nb[0], by = (tile / t.nb[0]) % t.nb[1], bz = tile / (t.nb[0] * t.nb[1]);
     const int t0[3] = {bx * 8, by * 8, bz * 8};
     const int c0 = off[tile], c1 = off[tile + 1];
     int kept = 0;
-    for (int c = c0; c < c1; ++c) {
-        const int i = list[c];
-        const int4 o = base[i];
-        const int org[3] = {o.x, o.y, o.z};
-        int w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        bool all = true;
-        for (int d = 0; d < 3; ++d) {
-            int nr = 0, open = 0, r0 = 0, r1 = 0;
-            int k = pmod(t0[d] - org[d], t.N[d]);
-            for (int u = 0; u < 8; ++u) {
-                const int cov = (t0[d] + u < t.N[d]) && k < t.P;
-                if (cov && open) {
-                    if (nr == 1) r0 += 1 << 4; else r1 += 1 << 4;
-                } else if (cov && nr < 2) {
-                    const int word = u | (1 << 4) | (k << 8);
-                    if (nr == 0) r0 = word; else r1 = word;
-                    ++nr;
-                    open = 1;
-                } else {
-                    open = 0;
-                }
-                k = k + 1 == t.N[d] ? 0 : k + 1;
+    for (int cb = c0; cb < c1; cb += 32) {
+        const int c = cb + lane;
+        const int i = c < c1 ? list[c] : -1;
+        bool all = i >= 0;
+        if (all) {
+            const int4 o = base[i];
+            const int org[3] = {o.x, o.y, o.z};
+            for (int d = 0; d < 3; ++d) {
+                bool any = false;
+                for (int u = 0; u < 8; ++u) any |= poly_support(t0[d] + u, org[d], t.N[d], t.P) >= 0;
+                all = all && any;
             }
-            w[2 * d] = r0;
-            w[2 * d + 1] = r1;
-            w[6] |= nr << (2 * d);
-            all = all && nr > 0;
         }
-        if (!all) continue;
-        clist[c0 + kept] = i;
-        for (int q = 0; q < 8; ++q) cruns[size_t(c0 + kept) * 8 + q] = w[q];
-        ++kept;
+        const unsigned hit = __ballot_sync(0xffffffffu, all);
+        if (all) clist[c0 + kept + __popc(hit & ((1u << lane) - 1u))] = i;
+        kept += __popc(hit);
     }
-    cnt[tile] = kept;
+    if (lane == 0) cnt[tile] = kept;
 }
 
-// Spread onto one 8^3 voxel tile x CM consecutive columns per CTA.  The
-// tile's accumulators live in shared memory; the tile's candidate particles
-// are added one after another in candidate order, all threads sharing the
-// (covered voxel, column) pairs of the current particle, with a barrier
-// between particles.  So every voxel's sum has a fixed order, there are no
-// atomics, and every voxel of the grid is written exactly once.
-// grid[((x*Ny+y)*Nz+z)*M + m].
+// Spread onto one 8^3 voxel tile x CM consecutive columns per CTA, every
+// voxel written once, each voxel's sum in candidate order (no atomics).  A
+// thread keeps CM / 4 rows of eight z voxels of its column in registers, the
+// eight z weights of a row come from shared memory as 16-byte words that its
+// CM columns share, and the candidates' weights are copied in (cp.async,
+// zeros where the support does not cover the tile) two candidates at a time,
+// three stages deep.  Accumulators in shared memory, updated candidate by
+// candidate between barriers, cost three shared accesses per six FMAs: 320
+// us for 1000 particles, 109^3 voxels and 48 columns (278 here),
+// and 195 us in fp64 for 512 particles, 35^3 and 8 columns (105).
+constexpr int kPolyStages = 3;
+constexpr int kPolyPer = 2;       // candidates per stage
+
+__device__ __forceinline__ void copy_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+template <typename R>
+__device__ __forceinline__ void copy_async_value(R* dst, const R* src, bool live) {
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    if constexpr (sizeof(R) == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(live ? 8 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(live ? 4 : 0) : "memory");
+}
+
+// values of the candidates' part of the shared memory, per candidate: moments
+// [3][CM], support tables [3][8] (short), particle
+template <typename R> __host__ __device__ constexpr size_t poly_spread_smem(int cap, int CM) {
+    return size_t(kPolyStages) * kPolyPer * 64 * 24 * sizeof(R) + size_t(cap) * (3 * CM * sizeof(cplx<R>) + 24 * 2 + 4);
+}
+
 template <typename R, int CM>
 __global__ void __launch_bounds__(256) k_poly_spread(const double2* __restrict__ X, int M, const R* __restrict__ w,
-                                                     const int* __restrict__ toff, const int* __restrict__ tcnt,
-                                                     const int* __restrict__ clist, const int* __restrict__ cruns,
+                                                     const int4* __restrict__ base, const int* __restrict__ toff,
+                                                     const int* __restrict__ tcnt, const int* __restrict__ clist,
                                                      PolyTile t, cplx<R>* __restrict__ grid) {
     extern __shared__ __align__(16) unsigned char shraw[];
-    cplx<R>* acc = reinterpret_cast<cplx<R>*>(shraw);              // [512][CM] tile accumulators
-    cplx<R>* pm = acc + 512 * CM;                                 // [cap][3][CM] candidate moments
-    int* runs = reinterpret_cast<int*>(pm + size_t(t.cap) * 3 * CM);  // [cap][8] covered runs
-    int* cand = runs + 8 * t.cap;                                 // [cap] particle index
-    // the column blocks of one tile are adjacent in launch order, so the
-    // candidates' weights are read from DRAM once and then hit in L2
+    R* wb = reinterpret_cast<R*>(shraw);                                    // [stages][kPolyPer][64 rows][8 z][3]
+    cplx<R>* pm = reinterpret_cast<cplx<R>*>(wb + kPolyStages * kPolyPer * 64 * 24);   // [cap][3][CM]
+    int* cand = reinterpret_cast<int*>(pm + size_t(t.cap) * 3 * CM);         // [cap]
+    short* sup = reinterpret_cast<short*>(cand + t.cap);                     // [cap][3][8] support index or -1
     const int ncb = (M + CM - 1) / CM;
-    const int tile = blockIdx.x / ncb;
+    const int tile = blockIdx.x / ncb;        // the column blocks of a tile are adjacent in launch order
     const int m0 = (blockIdx.x - tile * ncb) * CM;
     const int bx = tile % t.nb[0], by = (tile / t.nb[0]) % t.nb[1], bz = tile / (t.nb[0] * t.nb[1]);
     const int t0[3] = {bx * 8, by * 8, bz * 8};
     const int c0 = toff[tile];
     const int nc = min(tcnt[tile], t.cap);
-    const int P = t.P, P3 = P * P * P;
-    // the tile's covering candidates and their runs (k_poly_runs)
-    for (int c = threadIdx.x; c < nc; c += blockDim.x) cand[c] = clist[c0 + c];
-    for (int q = threadIdx.x; q < nc * 8; q += blockDim.x) runs[q] = cruns[size_t(c0) * 8 + q];
-    for (int k = threadIdx.x; k < nc * 3 * CM; k += blockDim.x) {
+    const int P = t.P;
+    const size_t P3 = size_t(P) * P * P;
+    for (int q = threadIdx.x; q < nc * 24; q += 256) {
+        const int c = q / 24, r = q - c * 24, d = r >> 3, u = r & 7;
+        const int i = clist[c0 + c];
+        const int4 o = base[i];
+        const int org = d == 0 ? o.x : d == 1 ? o.y : o.z;
+        const int tt = d == 0 ? t0[0] : d == 1 ? t0[1] : t0[2];
+        const int N = d == 0 ? t.N[0] : d == 1 ? t.N[1] : t.N[2];
+        sup[q] = short(poly_support(tt + u, org, N, P));
+        if (r == 0) cand[c] = i;
+    }
+    for (int k = threadIdx.x; k < nc * 3 * CM; k += 256) {
         const int cm = k % CM, comp = (k / CM) % 3, c = k / (3 * CM);
         const int m = m0 + cm;
         pm[k] = m < M ? to_r<R>(X[size_t(3 * clist[c0 + c] + comp) * M + m]) : mk<R>(0, 0);
     }
-    for (int k = threadIdx.x; k < 512 * CM; k += blockDim.x) acc[k] = mk<R>(0, 0);
     __syncthreads();
-    const int cm = threadIdx.x % CM;            // this thread's column
-    const int slot = threadIdx.x / CM;          // and voxel slot
-    constexpr int NSLOT = 256 / CM;
-    for (int c = 0; c < nc; ++c) {
-        const int* rr = runs + c * 8;
-        const int nrs = rr[6];
-        // a candidate that misses the tile along some axis adds nothing (the
-        // branch is uniform across the CTA, so its barrier goes too)
-        if (!(nrs & 3) || !(nrs & 12) || !(nrs & 48)) continue;
-        const cplx<R> p0 = pm[(c * 3 + 0) * CM + cm], p1 = pm[(c * 3 + 1) * CM + cm], p2 = pm[(c * 3 + 2) * CM + cm];
-        const R* wi = w + size_t(cand[c]) * P3 * 3;
-        for (int ax = 0; ax < (nrs & 3); ++ax)
-            for (int ay = 0; ay < ((nrs >> 2) & 3); ++ay)
-                for (int az = 0; az < ((nrs >> 4) & 3); ++az) {
-                    const int qx = rr[ax], qy = rr[2 + ay], qz = rr[4 + az];
-                    const int lx = (qx >> 4) & 15, ly = (qy >> 4) & 15, lz = (qz >> 4) & 15;
-                    // slot = one (x, y) row of the covered box; its z run is
-                    // contiguous in both the accumulators and the weights
-                    for (int r = slot; r < lx * ly; r += NSLOT) {
-                        const int ix = r / ly, iy = r - ix * ly;
-                        const int ux = (qx & 15) + ix, uy = (qy & 15) + iy;
-                        const int kx = (qx >> 8) + ix, ky = (qy >> 8) + iy;
-                        const R* wp = wi + ((kx * P + ky) * P + (qz >> 8)) * 3;
-                        cplx<R>* ap = acc + ((ux * 8 + uy) * 8 + (qz & 15)) * CM + cm;
-                        for (int iz = 0; iz < lz; ++iz, wp += 3, ap += CM)
-                            *ap += p0 * wp[0] + p1 * wp[1] + p2 * wp[2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // a warp copies eight of the 64 (x, y) rows of a candidate, lane = 3 z + component
+    const int lz = lane / 3;
+    auto copy_stage = [&](int st) {
+        R* dst0 = wb + size_t(st % kPolyStages) * kPolyPer * 64 * 24;
+#pragma unroll
+        for (int e = 0; e < kPolyPer; ++e) {
+            const int c = st * kPolyPer + e;
+            if (c < nc && lane < 24) {
+                const short* sc = sup + c * 24;
+                const int kz = sc[16 + lz];
+                const R* wi = w + size_t(cand[c]) * P3 * 3;
+                const int kx = sc[warp];      // row = 8 x + y, x = warp
+                R* dst = dst0 + (e * 64 + warp * 8) * 24 + lane;
+                if (kx >= 0) {
+#pragma unroll
+                    for (int y = 0; y < 8; ++y) {
+                        const int ky = sc[8 + y];
+                        const bool live = ky >= 0 && kz >= 0;
+                        const R* src = live ? wi + (size_t(kx * P + ky) * P + kz) * 3 + (lane - 3 * lz) : w;
+                        copy_async_value<R>(dst + y * 24, src, live);
                     }
                 }
-        __syncthreads();
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    constexpr int NSLOT = 256 / CM, RPT = 64 / NSLOT;
+    const int cm = threadIdx.x % CM, slot = threadIdx.x / CM;
+    cplx<R> acc[RPT][8];
+#pragma unroll
+    for (int r = 0; r < RPT; ++r)
+#pragma unroll
+        for (int z = 0; z < 8; ++z) acc[r][z] = mk<R>(R(0), R(0));
+    const int nst = (nc + kPolyPer - 1) / kPolyPer;
+#pragma unroll
+    for (int st = 0; st < kPolyStages - 1; ++st) copy_stage(st);
+    for (int st = 0; st < nst; ++st) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kPolyStages - 2) : "memory");
+        __syncthreads();          // this stage is in; the one before it has been used
+        copy_stage(st + kPolyStages - 1);
+        const R* src0 = wb + size_t(st % kPolyStages) * kPolyPer * 64 * 24;
+#pragma unroll
+        for (int e = 0; e < kPolyPer; ++e) {
+            const int c = st * kPolyPer + e;
+            if (c >= nc) break;
+            const short* sc = sup + c * 24;
+            const cplx<R> p0 = pm[(c * 3 + 0) * CM + cm], p1 = pm[(c * 3 + 1) * CM + cm], p2 = pm[(c * 3 + 2) * CM + cm];
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) {
+                const int row = slot + r * NSLOT;
+                if (sc[row >> 3] < 0 || sc[8 + (row & 7)] < 0) continue;
+                const float4* wp = reinterpret_cast<const float4*>(src0 + (e * 64 + row) * 24);
+                // four z at a time: 12 weights, 16-byte reads
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    R v[12];
+                    constexpr int NV = 12 * sizeof(R) / 16;
+#pragma unroll
+                    for (int q = 0; q < NV; ++q) {
+                        const float4 f = wp[h * NV + q];
+                        if constexpr (sizeof(R) == 4) {
+                            v[4 * q] = f.x; v[4 * q + 1] = f.y; v[4 * q + 2] = f.z; v[4 * q + 3] = f.w;
+                        } else {
+                            const double2 d = *reinterpret_cast<const double2*>(&f);
+                            v[2 * q] = d.x; v[2 * q + 1] = d.y;
+                        }
+                    }
+#pragma unroll
+                    for (int z = 0; z < 4; ++z) {
+                        fma_rc(acc[r][4 * h + z], v[3 * z], p0);
+                        fma_rc(acc[r][4 * h + z], v[3 * z + 1], p1);
+                        fma_rc(acc[r][4 * h + z], v[3 * z + 2], p2);
+                    }
+                }
+            }
+        }
     }
-    for (int k = threadIdx.x; k < 512 * CM; k += blockDim.x) {
-        const int kc = k % CM, v = k / CM;
-        const int x = t0[0] + (v >> 6), y = t0[1] + ((v >> 3) & 7), z = t0[2] + (v & 7);
-        const int m = m0 + kc;
-        if (m < M && x < t.N[0] && y < t.N[1] && z < t.N[2])
-            grid[((size_t(x) * t.N[1] + y) * t.N[2] + z) * M + m] = acc[k];
+    copy_async_wait_all();
+    const int m = m0 + cm;
+    if (m >= M) return;
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        const int row = slot + r * NSLOT;
+        const int x = t0[0] + (row >> 3), y = t0[1] + (row & 7);
+        if (x >= t.N[0] || y >= t.N[1]) continue;
+        cplx<R>* g = grid + ((size_t(x) * t.N[1] + y) * t.N[2] + t0[2]) * M + m;
+#pragma unroll
+        for (int z = 0; z < 8; ++z)
+            if (t0[2] + z < t.N[2]) g[size_t(z) * M] = acc[r][z];
     }
 }
 
@@ -343,66 +415,72 @@ __global__ void k_poly_scale(cplx<R>* __restrict__ grid, const R* __restrict__ s
     grid[t] = grid[t] * sc[t / M];
 }
 
-// Contraction.  CTA = one target x one block of up to 32*MC columns; its
-// CW warps take every CW-th support node (unrolled so several grid loads are
-// in flight), lanes over columns, then a fixed-order sum over the warps.
+// Contraction.  CTA = one target x one block of GS * MC columns; its eight
+// warps take every eighth (x, y) row of the support, a warp's 32 / GS lane
+// groups every (32 / GS)-th node of the row, a group's lanes MC columns each
+// (unrolled so several grid loads are in flight); then a fixed-order sum over
+// groups and warps.  GS = 32 for every batch left 24 of 32 lanes idle at 8
+// columns (fp64, 512 targets: 127 us, 24 here).
 // Y rows 3j+c, already scaled by h^3.
-template <typename R, int MC>
+template <typename R, int GS, int MC>
 __global__ void __launch_bounds__(256) k_poly_contract(const cplx<R>* __restrict__ grid, int M,
                                                        const int4* __restrict__ base, const R* __restrict__ w, int P,
                                                        int Nx, int Ny, int Nz, double factor,
                                                        double2* __restrict__ Y) {
-    constexpr int CW = 8;
-    __shared__ cplx<R> red[CW][3][32];
+    constexpr int CW = 8, NG = 32 / GS;
+    __shared__ cplx<R> red[CW][3][GS];
     const int j = blockIdx.x;
-    const int m0 = blockIdx.y * 32 * MC;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & (GS - 1), grp = (threadIdx.x & 31) / GS;
+    const int m0 = blockIdx.y * GS * MC + lane;
     const int P3 = P * P * P;
     const int4 o = base[j];
     cplx<R> acc[3][MC];
 #pragma unroll
     for (int q = 0; q < MC; ++q) acc[0][q] = acc[1][q] = acc[2][q] = mk<R>(0, 0);
-    // warp = (x, y) rows of the support (P < N, so a coordinate wraps at
-    // most once); each row's z run is contiguous in the weights and, up to
-    // one wrap, in the grid
+    // the support's (x, y) rows (P < N, so a coordinate wraps at most once);
+    // each row's z run is contiguous in the weights and, up to one wrap, in
+    // the grid
     for (int r = warp; r < P * P; r += CW) {
         const int kx = r / P, ky = r - kx * P;
         int x = o.x + kx, y = o.y + ky;
         if (x >= Nx) x -= Nx;
         if (y >= Ny) y -= Ny;
-        const size_t rowbase = (size_t(x) * Ny + y) * Nz;
+        const cplx<R>* gr = grid + (size_t(x) * Ny + y) * Nz * M + m0;
         const R* wp = w + (size_t(j) * P3 + size_t(r) * P) * 3;
-        int z = o.z;
 #pragma unroll 4
-        for (int kz = 0; kz < P; ++kz) {
-            const size_t vo = (rowbase + z) * M;
+        for (int kz = grp; kz < P; kz += NG) {
+            const int z = o.z + kz < Nz ? o.z + kz : o.z + kz - Nz;
             const R w0 = wp[3 * kz], w1 = wp[3 * kz + 1], w2 = wp[3 * kz + 2];
 #pragma unroll
             for (int q = 0; q < MC; ++q) {
-                const int m = m0 + q * 32 + lane;
-                if (m < M) {
-                    const cplx<R> g = grid[vo + m];
-                    acc[0][q] += g * w0;
-                    acc[1][q] += g * w1;
-                    acc[2][q] += g * w2;
+                if (m0 + q * GS < M) {
+                    const cplx<R> g = gr[size_t(z) * M + q * GS];
+                    fma_rc(acc[0][q], w0, g);
+                    fma_rc(acc[1][q], w1, g);
+                    fma_rc(acc[2][q], w2, g);
                 }
             }
-            z = z + 1 == Nz ? 0 : z + 1;
         }
     }
 #pragma unroll
     for (int q = 0; q < MC; ++q) {
-        for (int c = 0; c < 3; ++c) red[warp][c][lane] = acc[c][q];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            for (int off = GS; off < 32; off <<= 1) {
+                acc[c][q].x += __shfl_xor_sync(0xffffffffu, acc[c][q].x, off);
+                acc[c][q].y += __shfl_xor_sync(0xffffffffu, acc[c][q].y, off);
+            }
+            if (grp == 0) red[warp][c][lane] = acc[c][q];
+        }
         __syncthreads();
-        if (warp == 0) {
-            const int m = m0 + q * 32 + lane;
+        if (threadIdx.x < 3 * GS) {
+            const int c = threadIdx.x / GS, l = threadIdx.x & (GS - 1);
+            const int m = blockIdx.y * GS * MC + q * GS + l;
             if (m < M) {
-                for (int c = 0; c < 3; ++c) {
-                    cplx<R> s = red[0][c][lane];
-                    for (int q2 = 1; q2 < CW; ++q2) s += red[q2][c][lane];
-                    const double2 d = to_d(s);
-                    Y[size_t(3 * j + c) * M + m] = make_double2(d.x * factor, d.y * factor);
-                }
+                cplx<R> s = red[0][c][l];
+                for (int q2 = 1; q2 < CW; ++q2) s += red[q2][c][l];
+                const double2 d = to_d(s);
+                Y[size_t(3 * j + c) * M + m] = make_double2(d.x * factor, d.y * factor);
             }
         }
         __syncthreads();
@@ -411,16 +489,16 @@ __global__ void __launch_bounds__(256) k_poly_contract(const cplx<R>* __restrict
 
 // Per pair: delta = r / max(d, 1e-6) and the pair-table values of the two
 // radius classes at max(d, 1e-6) (real_space_precalcs_kernel_polydisperse,
-// :352-441).  Thread per target; a target index past the particles takes
+// :352-441).  Warp per target; a target index past the particles takes
 // class 0 (:407).  Same layout as the monodisperse pair coefficients.
 __global__ void k_poly_pair_coefs(const double* __restrict__ pgeo, const int* __restrict__ off,
                                   const int* __restrict__ src, int nt, int N, const int* __restrict__ cls,
                                   const double* __restrict__ rad, double xi, int table_n, double* __restrict__ T64,
                                   float* __restrict__ T32) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (j >= nt) return;
     const int cj = j < N ? cls[j] : 0;
-    for (int p = off[j]; p < off[j + 1]; ++p) {
+    for (int p = off[j] + (threadIdx.x & 31); p < off[j + 1]; p += 32) {
         const int ci = cls[src[p]];
         const double a = rad[min(ci, cj)], b = rad[max(ci, cj)];
         const double d = pgeo[4 * size_t(p) + 3];
@@ -765,9 +843,9 @@ void Field::poly_weights(PointSet& ps, const double* radius_dev, cudaStream_t s,
     MPM_LAUNCH();
     ptcnt_.ensure(sizeof(int) * std::max(1, nbins));
     ptclist_.ensure(sizeof(int) * std::max(1, hv[1]));
-    ptruns_.ensure(sizeof(int) * 8 * size_t(std::max(1, hv[1])));
-    k_poly_runs<<<nblk(nbins, 128), 128, 0, s>>>(t, ps.base.as<int4>(), ptoff_.as<int>(), ptlist_.as<int>(),
-                                                 ptcnt_.as<int>(), ptclist_.as<int>(), ptruns_.as<int>());
+    k_poly_filter<<<nblk((long long)nbins * 32, 128), 128, 0, s>>>(t, ps.base.as<int4>(), ptoff_.as<int>(),
+                                                                   ptlist_.as<int>(), ptcnt_.as<int>(),
+                                                                   ptclist_.as<int>());
     MPM_LAUNCH();
     pcand_cap_ = std::max(1, h);
     const size_t shm = 65536 + (3 * 128 + 9 * sizeof(int)) * size_t(pcand_cap_);
@@ -779,7 +857,7 @@ void Field::poly_weights(PointSet& ps, const double* radius_dev, cudaStream_t s,
 void Field::poly_pair_coefs(cudaStream_t s) {
     const int nt = spec_.solver_ax ? N_ : targets_.n;
     if (num_pairs_ <= 0) return;
-    k_poly_pair_coefs<<<nblk(nt, 128), 128, 0, s>>>(pair_geo_.as<double>(), pair_off_.as<int>(), pair_src_.as<int>(),
+    k_poly_pair_coefs<<<nblk((long long)nt * 32, 128), 128, 0, s>>>(pair_geo_.as<double>(), pair_off_.as<int>(), pair_src_.as<int>(),
                                                     nt, N_, pcls_.as<int>(), prad_.as<double>(), spec_.xi,
                                                     pgeom_.table_n, pair_T64_.as<double>(), pair_T32_.as<float>());
     MPM_LAUNCH();
@@ -825,23 +903,34 @@ void Field::poly_precalc(cudaStream_t s) {
 
 template <typename R>
 void Field::poly_recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStream_t s) {
-    constexpr int MC = sizeof(R) == 4 ? 4 : 2;   // contraction column chunks of 32 per CTA
-    const int nmb = (M + 32 * MC - 1) / (32 * MC);
-    constexpr int CM = sizeof(R) == 4 ? 16 : 8;   // spread columns per CTA (64 KB of accumulators)
     const PointSet& ps = sources_;
     PolyTile t;
     for (int d = 0; d < 3; ++d) { t.N[d] = pgeom_.ng[d]; t.nb[d] = ps.nb[d]; }
     t.P = pgeom_.P;
     t.T = 8;
     t.cap = pcand_cap_;
-    const size_t shm = sizeof(cplx<R>) * (512 + 3 * size_t(t.cap)) * CM + sizeof(int) * 9 * t.cap;
-    set_smem_limit(k_poly_spread<R, CM>, shm);
     const R* w1 = sizeof(R) == 4 ? reinterpret_cast<const R*>(ps.w32.p) : reinterpret_cast<const R*>(ps.w64.p);
     const int ntile = ps.nb[0] * ps.nb[1] * ps.nb[2];
     {
         StageScope sc(ST_SPREAD, s);
-        k_poly_spread<R, CM><<<ntile * ((M + CM - 1) / CM), 256, shm, s>>>(
-            X, M, w1, ptoff_.as<int>(), ptcnt_.as<int>(), ptclist_.as<int>(), ptruns_.as<int>(), t, grid);
+        // columns per CTA: as many as the accumulators allow (16 fp32, 8 fp64),
+        // fewer for narrow batches and while the tiles would leave SMs idle
+        auto go = [&](auto cmc) {
+            constexpr int CM = decltype(cmc)::value;
+            const size_t shm = poly_spread_smem<R>(t.cap, CM);
+            set_smem_limit(k_poly_spread<R, CM>, shm);
+            k_poly_spread<R, CM><<<ntile * ((M + CM - 1) / CM), 256, shm, s>>>(
+                X, M, w1, ps.base.as<int4>(), ptoff_.as<int>(), ptcnt_.as<int>(), ptclist_.as<int>(), t, grid);
+        };
+        auto ctas = [&](int cm) { return (long long)ntile * ((M + cm - 1) / cm); };
+        if constexpr (sizeof(R) == 4) {
+            if (M > 8 && ctas(16) >= 2 * 148) go(std::integral_constant<int, 16>{});
+            else if (M > 4 && ctas(8) >= 2 * 148) go(std::integral_constant<int, 8>{});
+            else go(std::integral_constant<int, 4>{});
+        } else {
+            if (M > 4 && ctas(8) >= 2 * 148) go(std::integral_constant<int, 8>{});
+            else go(std::integral_constant<int, 4>{});
+        }
         MPM_LAUNCH();
     }
     const R* scl = sizeof(R) == 4 ? reinterpret_cast<const R*>(scale32_.p) : reinterpret_cast<const R*>(scale64_.p);
@@ -914,8 +1003,18 @@ void Field::poly_recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cu
     const PointSet& tg = spec_.solver_ax ? sources_ : targets_;
     const R* tw = sizeof(R) == 4 ? reinterpret_cast<const R*>(tg.w32.p) : reinterpret_cast<const R*>(tg.w64.p);
     const double factor = pgeom_.h[0] * pgeom_.h[1] * pgeom_.h[2];
-    k_poly_contract<R, MC><<<dim3(tg.n, nmb), 256, 0, s>>>(grid, M, tg.base.as<int4>(), tw, pgeom_.P, gv_.Nx, gv_.Ny,
-                                                          gv_.Nz, factor, Y);
+    auto contract = [&](auto gsc, auto mcc) {
+        constexpr int GS = decltype(gsc)::value, MC = decltype(mcc)::value;
+        k_poly_contract<R, GS, MC><<<dim3(tg.n, (M + GS * MC - 1) / (GS * MC)), 256, 0, s>>>(
+            grid, M, tg.base.as<int4>(), tw, pgeom_.P, gv_.Nx, gv_.Ny, gv_.Nz, factor, Y);
+    };
+    using std::integral_constant;
+    if (M <= 4) contract(integral_constant<int, 4>{}, integral_constant<int, 1>{});
+    else if (M <= 8) contract(integral_constant<int, 8>{}, integral_constant<int, 1>{});
+    else if (M <= 16) contract(integral_constant<int, 16>{}, integral_constant<int, 1>{});
+    else if (M <= 32) contract(integral_constant<int, 16>{}, integral_constant<int, 2>{});
+    else if (M <= 48) contract(integral_constant<int, 16>{}, integral_constant<int, 3>{});
+    else contract(integral_constant<int, 32>{}, integral_constant<int, 3>{});
     MPM_LAUNCH();
     if (Nq_) {
         k_poly_quad_contract<R><<<Nq_, 128, 0, s>>>(gq, M, tg.base.as<int4>(), qw, pgeom_.P, gv_.Nx, gv_.Ny, gv_.Nz,
