@@ -100,6 +100,48 @@ __global__ void k_stencil(const double* __restrict__ xyz, int n, StencilArgs a, 
     base[i] = make_int4(gw[0], gw[1], slot, gw[2]);
 }
 
+// The ranges of the sorted particle list (spatial bins, z outermost) whose
+// stencils can reach the tile [x0, x1) x [y0, y1) x [z0, z1): starts and the
+// running total of their lengths.  All threads; ends with a barrier.
+struct TileBins { int b[3][8], n[3]; };
+
+__device__ __forceinline__ void tile_ranges(const GridView& g, int x0, int x1, int y0, int y1, int z0, int z1, int TX,
+                                            int TY, int TZ, int nbx, int nby, const int* __restrict__ bin_start,
+                                            const int* __restrict__ bin_end, TileBins& t, int (&rstart)[512],
+                                            int (&rpre)[513], int& nranges) {
+    if (threadIdx.x == 0) t.n[0] = reach_bins(x0 - g.off, x1 - 1 + g.off, g.Nx, TX, true, t.b[0]);
+    if (threadIdx.x == 32) t.n[1] = reach_bins(y0 - g.off, y1 - 1 + g.off, g.Ny, TY, true, t.b[1]);
+    if (threadIdx.x == 64) t.n[2] = reach_bins(z0 - g.off, z1 - 1 + g.off, g.Zs, TZ, !g.pruned, t.b[2]);
+    __syncthreads();
+    const int nr = min(512, t.n[0] * t.n[1] * t.n[2]);
+    for (int k = threadIdx.x; k < nr; k += blockDim.x) {
+        const int c = k % t.n[0], q = k / t.n[0];
+        const int key = (t.b[2][q / t.n[1]] * nby + t.b[1][q % t.n[1]]) * nbx + t.b[0][c];
+        const int s0 = bin_start[key];
+        rstart[k] = s0;
+        rpre[k + 1] = s0 < 0 ? 0 : bin_end[key] - s0;     // an empty bin: a range of no length
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int carry = 0;
+        for (int k0 = 0; k0 < nr; k0 += 32) {
+            const int k = k0 + threadIdx.x;
+            int v = k < nr ? rpre[k + 1] : 0;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, v, o);
+                if (int(threadIdx.x) >= o) v += u;
+            }
+            if (k < nr) rpre[k + 1] = carry + v;
+            carry += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (threadIdx.x == 0) {
+            rpre[0] = 0;
+            nranges = nr;
+        }
+    }
+    __syncthreads();
+}
+
 // Gather spread: every voxel of this CTA's tile is written once with the sum
 // of all particle contributions (no atomics).  grid[((x*Ny+y)*Zs+s)*B + b].
 // Candidates come from the spatial bins that can reach the tile; for each
@@ -118,33 +160,14 @@ __global__ void __launch_bounds__(256) k_spread(const double2* __restrict__ X, i
                                                 int TZ, int nbx, int nby, int nzt, int cap, int bc,
                                                 cplx<R>* __restrict__ grid) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int bx[8], by[8], bz[8], nbxs, nbys, nbzs;
-    __shared__ int rstart[512], rlen[512], rpre[513], nranges;
+    __shared__ TileBins bins;
+    __shared__ int rstart[512], rpre[513], nranges;
     // blockIdx.z = z tile + nzt * (column chunk of bc columns)
     const int zt = blockIdx.z % nzt, chunk = blockIdx.z / nzt;
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = zt * TZ;
     const int x1 = min(x0 + TX, g.Nx), y1 = min(y0 + TY, g.Ny), z1 = min(z0 + TZ, g.Zs);
     const int B = C * M;
-    if (threadIdx.x == 0) {
-        nbxs = reach_bins(x0 - g.off, x1 - 1 + g.off, g.Nx, TX, true, bx);
-        nbys = reach_bins(y0 - g.off, y1 - 1 + g.off, g.Ny, TY, true, by);
-        nbzs = reach_bins(z0 - g.off, z1 - 1 + g.off, g.Zs, TZ, !g.pruned, bz);
-        int k = 0;
-        rpre[0] = 0;
-        for (int a = 0; a < nbzs; ++a)
-            for (int b2 = 0; b2 < nbys; ++b2)
-                for (int c = 0; c < nbxs; ++c) {
-                    const int key = (bz[a] * nby + by[b2]) * nbx + bx[c];
-                    const int s0 = bin_start[key];
-                    if (s0 < 0 || k >= 512) continue;
-                    rstart[k] = s0;
-                    rlen[k] = bin_end[key] - s0;
-                    rpre[k + 1] = rpre[k] + rlen[k];
-                    ++k;
-                }
-        nranges = k;
-    }
-    __syncthreads();
+    tile_ranges(g, x0, x1, y0, y1, z0, z1, TX, TY, TZ, nbx, nby, bin_start, bin_end, bins, rstart, rpre, nranges);
     const int total = rpre[nranges];
     const int wlen = TX + TY + TZ;
     const int ncol = TX * TY;
@@ -299,8 +322,8 @@ __global__ void __launch_bounds__(256) k_spread_plan(const int4* __restrict__ ba
                                                      double* __restrict__ w64T, float* __restrict__ w32T,
                                                      double* __restrict__ lw64, float* __restrict__ lw32,
                                                      int* __restrict__ lcT, int* __restrict__ lnT) {
-    __shared__ int bx[8], by[8], bz[8], nbxs, nbys, nbzs;
-    __shared__ int rstart[512], rlen[512], rpre[513], nranges;
+    __shared__ TileBins bins;
+    __shared__ int rstart[512], rpre[513], nranges;
     __shared__ int cand[kPlanCandMax];
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* wloc = reinterpret_cast<double*>(smem_raw);   // [kPlanCandMax][wlen]
@@ -308,26 +331,7 @@ __global__ void __launch_bounds__(256) k_spread_plan(const int4* __restrict__ ba
     const int tx = tile % nbx, ty = (tile / nbx) % nby, zt = tile / (nbx * nby);
     const int x0 = tx * TX, y0 = ty * TY, z0 = zt * TZ;
     const int x1 = min(x0 + TX, g.Nx), y1 = min(y0 + TY, g.Ny), z1 = min(z0 + TZ, g.Zs);
-    if (threadIdx.x == 0) {
-        nbxs = reach_bins(x0 - g.off, x1 - 1 + g.off, g.Nx, TX, true, bx);
-        nbys = reach_bins(y0 - g.off, y1 - 1 + g.off, g.Ny, TY, true, by);
-        nbzs = reach_bins(z0 - g.off, z1 - 1 + g.off, g.Zs, TZ, !g.pruned, bz);
-        int k = 0;
-        rpre[0] = 0;
-        for (int a = 0; a < nbzs; ++a)
-            for (int b2 = 0; b2 < nbys; ++b2)
-                for (int c = 0; c < nbxs; ++c) {
-                    const int key = (bz[a] * nby + by[b2]) * nbx + bx[c];
-                    const int s0 = bin_start[key];
-                    if (s0 < 0 || k >= 512) continue;
-                    rstart[k] = s0;
-                    rlen[k] = bin_end[key] - s0;
-                    rpre[k + 1] = rpre[k] + rlen[k];
-                    ++k;
-                }
-        nranges = k;
-    }
-    __syncthreads();
+    tile_ranges(g, x0, x1, y0, y1, z0, z1, TX, TY, TZ, nbx, nby, bin_start, bin_end, bins, rstart, rpre, nranges);
     const int total = rpre[nranges];
     if (total > kPlanCandMax) {
         if (threadIdx.x == 0) atomicOr(overflow, 1);
@@ -412,9 +416,12 @@ __global__ void __launch_bounds__(256) k_spread_plan(const int4* __restrict__ ba
 }
 
 // Spread with the per-frame plan: CTA = one tile x one chunk of bc grid
-// columns; loads the tile's candidate moments, then thread = one (x, y)
-// column x one grid column with the whole z run in registers.  The same
-// contributors in the same order as k_spread.
+// columns; stages the tile's candidate moments and z weights and every (x, y)
+// column's contributor list in shared memory, then thread = one (x, y) column
+// x one grid column with the whole z run in registers.  The same contributors
+// in the same order as k_spread.  With the lists and weights read from global
+// memory in the loop it waited on one dependent load after another: 119 us
+// for 8000 particles, 84^3 voxels and 9 columns, 90 here.
 template <typename R, int ZMAX>
 __global__ void __launch_bounds__(256) k_spread_planned(const double2* __restrict__ X, int M, int N, int C,
                                                         const int* __restrict__ quad_map, GridView g, int TX,
@@ -424,17 +431,28 @@ __global__ void __launch_bounds__(256) k_spread_planned(const double2* __restric
                                                         const int* __restrict__ lcT, const int* __restrict__ lnT,
                                                         cplx<R>* __restrict__ grid) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    cplx<R>* pv = reinterpret_cast<cplx<R>*>(smem_raw);   // [capT][bc]
+    const int ncol = TX * TY;
+    cplx<R>* pv = reinterpret_cast<cplx<R>*>(smem_raw);                  // [capT][bc]
+    R* wz = reinterpret_cast<R*>(pv + size_t(capT) * bc);                 // [capT][TZ]
+    R* lwS = wz + size_t(capT) * TZ;                                      // [ncol][kSpreadListCap]
+    int* lcS = reinterpret_cast<int*>(lwS + size_t(ncol) * kSpreadListCap);
+    int* lnS = lcS + size_t(ncol) * kSpreadListCap;                        // [ncol]
     const int zt = blockIdx.z % nzt, chunk = blockIdx.z / nzt;
     const int tile = (zt * nby + blockIdx.y) * nbx + blockIdx.x;
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = zt * TZ;
     const int B = C * M;
     const int wlen = TX + TY + TZ;
-    const int ncol = TX * TY;
     const int nc = ncT[tile];
     const size_t trow = size_t(tile) * capT;
     const int b0 = chunk * bc;
     const int nb = min(bc, B - b0);
+    const R* wTt = wT + trow * wlen;
+    for (int t = threadIdx.x; t < ncol; t += blockDim.x) lnS[t] = lnT[size_t(tile) * ncol + t];
+    for (int t = threadIdx.x; t < nc * TZ; t += blockDim.x) {
+        const int c = t / TZ;
+        wz[t] = wTt[size_t(c) * wlen + TX + TY + (t - c * TZ)];
+    }
+#pragma unroll 4
     for (int t = threadIdx.x; t < nc * nb; t += blockDim.x) {
         const int c = t / nb, bb = t % nb;
         const int i = cidT[trow + c];
@@ -450,35 +468,65 @@ __global__ void __launch_bounds__(256) k_spread_planned(const double2* __restric
         pv[c * bc + bb] = to_r<R>(v);
     }
     __syncthreads();
-    const R* wTt = wT + trow * wlen;
+    if (nc > 0) {
+        // a warp's list loads for eight columns in flight together
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+        constexpr int kCPW = 8;
+        for (int col0 = warp; col0 < ncol; col0 += nwarp * kCPW) {
+            for (int k0 = 0; k0 < kSpreadListCap; k0 += 32) {
+                int cc[kCPW];
+                R ww[kCPW];
+#pragma unroll
+                for (int u = 0; u < kCPW; ++u) {
+                    const int col = col0 + u * nwarp, k = k0 + lane;
+                    cc[u] = -1;
+                    if (col < ncol && k < lnS[col]) {
+                        const size_t lrow = (size_t(tile) * ncol + col) * kSpreadListCap;
+                        cc[u] = lcT[lrow + k];
+                        ww[u] = lwT[lrow + k];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kCPW; ++u) {
+                    if (cc[u] < 0) continue;
+                    const int col = col0 + u * nwarp, k = k0 + lane;
+                    lcS[col * kSpreadListCap + k] = cc[u];
+                    lwS[col * kSpreadListCap + k] = ww[u];
+                }
+            }
+        }
+        __syncthreads();
+    }
     for (int t = threadIdx.x; t < ncol * nb; t += blockDim.x) {
         const int bb = t % nb, col = t / nb;
         const int lx = col / TY, ly = col % TY;
         const int x = x0 + lx, y = y0 + ly;
         if (x >= g.Nx || y >= g.Ny) continue;
-        const int nl = lnT[size_t(tile) * ncol + col];
+        const int nl = lnS[col];
         cplx<R> acc[ZMAX];
 #pragma unroll
         for (int lz = 0; lz < ZMAX; ++lz) acc[lz] = mk<R>(0, 0);
         if (nl >= 0) {
-            const size_t lrow = (size_t(tile) * ncol + col) * kSpreadListCap;
+            const int* lc = lcS + col * kSpreadListCap;
+            const R* lw = lwS + col * kSpreadListCap;
             for (int k = 0; k < nl; ++k) {
-                const int c = lcT[lrow + k];
-                const R wxy = lwT[lrow + k];
+                const int c = lc[k];
+                const R wxy = lw[k];
                 const cplx<R> pc = pv[c * bc + bb];
-                const R* wz = wTt + c * wlen + TX + TY;
+                const R* wzc = wz + c * TZ;
 #pragma unroll
                 for (int lz = 0; lz < ZMAX; ++lz)
-                    if (lz < TZ) fma_rc(acc[lz], wxy * wz[lz], pc);
+                    if (lz < TZ) fma_rc(acc[lz], wxy * wzc[lz], pc);
             }
-        } else {
+        } else {   // list overflowed: every candidate, in order
             for (int c = 0; c < nc; ++c) {
-                const R* wc = wTt + c * wlen;
+                const R* wc = wTt + size_t(c) * wlen;
                 const R wxy = wc[lx] * wc[TX + ly];
                 const cplx<R> pc = pv[c * bc + bb];
+                const R* wzc = wz + c * TZ;
 #pragma unroll
                 for (int lz = 0; lz < ZMAX; ++lz)
-                    if (lz < TZ) fma_rc(acc[lz], wxy * wc[TX + TY + lz], pc);
+                    if (lz < TZ) fma_rc(acc[lz], wxy * wzc[lz], pc);
             }
         }
         const size_t o0 = ((size_t(x) * g.Ny + y) * g.Zs + z0) * B + b0 + bb;
@@ -893,7 +941,7 @@ __global__ void k_column(cplx<R>* __restrict__ grid, const cplx<R>* __restrict__
 template <typename R, int SZ, int SXY>
 __global__ void k_contract(const cplx<R>* __restrict__ grid, GridView g, int M, int C, int Nt,
                            const int4* __restrict__ base, const R* __restrict__ w1, double factor,
-                           const int* __restrict__ quad_map, double2* __restrict__ Y, int negate,
+                           const int* __restrict__ quad_map, double2* __restrict__ Y,
                            const int* __restrict__ order, int accumulate, const double2* __restrict__ jsc) {
     __shared__ R w[3 * kMaxStencil];
     __shared__ int idx[3 * kMaxStencil];
@@ -961,7 +1009,6 @@ __global__ void k_contract(const cplx<R>* __restrict__ grid, GridView g, int M, 
         }
         double2 v = to_d(acc);
         v.x *= factor; v.y *= factor;
-        if (negate) { v.x = -v.x; v.y = -v.y; }
         const int m = b - comp * M;
         const size_t row = (comp < 3) ? size_t(3 * j + comp) : size_t(3 * Nt + 5 * q + comp - 3);
         if (accumulate && comp < 3) {
@@ -976,86 +1023,114 @@ __global__ void k_contract(const cplx<R>* __restrict__ grid, GridView g, int M, 
     }
 }
 
-// k_contract for one stored z slot (single layer) and few grid columns
-// (B = 3M <= 16, dipoles only): a CTA holds 128 / gsz targets, gsz = B
-// rounded up to a power of two lanes each, instead of one target per CTA
-// with B of its 32 lanes busy.  Same arithmetic, in the same order, as
-// k_contract<R, 1, SXY>.
-constexpr int kContractSmallMaxT = 32;   // targets per CTA (gsz >= 4)
-
-template <typename R, int SXY>
-__global__ void __launch_bounds__(128) k_contract_small(const cplx<R>* __restrict__ grid, GridView g, int M, int Nt,
-                                                        const int4* __restrict__ base, const R* __restrict__ w1,
-                                                        double factor, double2* __restrict__ Y, int negate,
-                                                        const int* __restrict__ order, int accumulate,
-                                                        const double2* __restrict__ jsc, int gsz) {
-    __shared__ R wxy[kContractSmallMaxT][2 * kMaxStencil];
-    __shared__ long long offxy[kContractSmallMaxT][2 * kMaxStencil];
-    __shared__ R wzs[kContractSmallMaxT];
-    __shared__ int zos[kContractSmallMaxT];
-    const int B = 3 * M;
-    const int per = blockDim.x / gsz;
-    const int slot = threadIdx.x / gsz, sl = threadIdx.x % gsz;
-    const int jj = blockIdx.x * per + slot;
+// k_contract for few grid columns (B = C M <= 16): a warp per target, or four
+// where the targets alone would leave the GPU idle; a warp's 32 / B groups of
+// B lanes share the stencil's (x, y) columns, then a fixed-order sum over
+// groups and warps.  One target per 32-thread CTA, a lane per column, left 23
+// of 32 lanes idle at B = 9 (8000 targets on 84^3: 134 us, 52 here)
+// and all but 500 warps unused at 500 targets (fp64, B = 3: 43 us,
+// 9).  SZ: the stencil's z run on the stored grid is at most SZ.
+template <typename R, int SZ, int WPT>
+__global__ void __launch_bounds__(128) k_contract_few(const cplx<R>* __restrict__ grid, GridView g, int M, int C,
+                                                      int Nt, const int4* __restrict__ base, const R* __restrict__ w1,
+                                                      double factor, const int* __restrict__ quad_map,
+                                                      double2* __restrict__ Y, const int* __restrict__ order,
+                                                      int accumulate, const double2* __restrict__ jsc) {
+    constexpr int TPC = 4 / WPT;
+    __shared__ R w[TPC][3 * kMaxStencil];
+    __shared__ long long off[TPC][2 * kMaxStencil];    // x then y stencil offsets into the grid (elements)
+    __shared__ int zo[TPC][kMaxStencil];                // z offsets
+    __shared__ cplx<R> red[4][16];
+    const int B = C * M;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slot = warp / WPT, wi = warp % WPT;
+    const int jj = blockIdx.x * TPC + slot;
     const bool live = jj < Nt;
+    // targets in spatial-bin order when given: CTAs that run together share
+    // their stencils' voxels in L2
     const int j = live ? (order ? order[jj] : jj) : 0;
+    const int S = g.S;
     if (live) {
         const int4 bs = base[j];
-        const int zc = g.off - g.offz;   // the stored slot's entry of the z stencil
-        for (int t = sl; t < 2 * g.S + 1; t += gsz) {
-            if (t < 2 * g.S) {
-                const int d = t / g.S, o = t % g.S;
-                wxy[slot][t] = w1[(size_t(j) * 3 + d) * g.S + o];
-                const int dd = o - g.off;
-                if (d == 0) offxy[slot][t] = (long long)pmod(bs.x + dd, g.Nx) * g.Ny * g.Zs * B;
-                else offxy[slot][t] = (long long)pmod(bs.y + dd, g.Ny) * g.Zs * B;
-            } else {
-                wzs[slot] = w1[(size_t(j) * 3 + 2) * g.S + zc];
-                const int dz = zc - g.off;
-                zos[slot] = g.pruned ? bs.z + dz : pmod(bs.z + dz, g.Nz);
+        for (int t = wi * 32 + lane; t < 3 * S; t += WPT * 32) {
+            const int d = t / S, o = t - d * S;
+            const int dd = o - g.off;
+            if (d < 2) {
+                w[slot][t] = w1[(size_t(j) * 3 + d) * S + o];
+                off[slot][t] = d == 0 ? (long long)pmod(bs.x + dd, g.Nx) * g.Ny * g.Zs * B
+                                      : (long long)pmod(bs.y + dd, g.Ny) * g.Zs * B;
+            } else if (o >= g.off - g.offz && o <= g.off + g.offz) {
+                // the z window on the stored grid
+                const int k = o - (g.off - g.offz);
+                w[slot][2 * S + k] = w1[(size_t(j) * 3 + 2) * S + o];
+                zo[slot][k] = (g.pruned ? bs.z + dd : pmod(bs.z + dd, g.Nz)) * B;
             }
         }
     }
     __syncthreads();
-    if (!live) return;
-    const int S = SXY > 0 ? SXY : g.S;
-    const R* w = wxy[slot];
-    const long long* off = offxy[slot];
-    const R wz = wzs[slot];
-    for (int b = sl; b < B; b += gsz) {
-        const int comp = b / M;
-        const int zo = zos[slot] * B + b;
-        cplx<R> acc = mk<R>(0, 0);
-        for (int ox = 0; ox < S; ++ox) {
-            const R wx = w[ox];
-            const cplx<R>* gx = grid + off[ox];
-            auto cell = [&](int oy) {
-                cplx<R> a2 = mk<R>(0, 0);
-                fma_rc(a2, wz, gx[off[S + oy] + zo]);
-                fma_rc(acc, wx * w[S + oy], a2);
-            };
-            if constexpr (SXY > 0) {
+    const int ng = 32 / B;
+    const int grp = lane / B, b = lane - grp * B;
+    const int comp = b / M;
+    const int q = (C > 3 && quad_map && live) ? quad_map[j] : -1;
+    const bool use = live && grp < ng && (comp < 3 || q >= 0);
+    cplx<R> acc = mk<R>(0, 0);
+    if (use) {
+        R wz[SZ];
+        int zb[SZ];
 #pragma unroll
-                for (int oy = 0; oy < SXY; ++oy) cell(oy);
-            } else {
-                for (int oy = 0; oy < S; ++oy) cell(oy);
-            }
+        for (int o = 0; o < SZ; ++o) {
+            wz[o] = o < g.Sz ? w[slot][2 * S + o] : R(0);
+            zb[o] = o < g.Sz ? zo[slot][o] + b : b;
         }
-        double2 v = to_d(acc);
-        v.x *= factor; v.y *= factor;
-        if (negate) { v.x = -v.x; v.y = -v.y; }
-        const int m = b - comp * M;
-        const size_t row = size_t(3 * j + comp);
-        if (accumulate) {
-            v += Y[row * M + m];
-            if (jsc) {
-                const double2 sv = jsc[size_t(j) * M + m];
-                const double den = sv.x * sv.x + sv.y * sv.y;
-                if (den > 1e-30) v = v * make_double2(sv.x / den, -sv.y / den);
-            }
+        const R* ws = w[slot];
+        const long long* os = off[slot];
+        const int step = WPT * ng;
+        int t = wi * ng + grp;
+        int ox = t / S, oy = t - ox * S;
+        const int sx = step / S, sy = step - sx * S;
+#pragma unroll (SZ == 1 ? 9 : 1)
+        for (; t < S * S; t += step) {
+            const cplx<R>* gp = grid + os[ox] + os[S + oy];
+            const R wxy = ws[ox] * ws[S + oy];
+            cplx<R> v[SZ];
+#pragma unroll
+            for (int o = 0; o < SZ; ++o)
+                if (o < g.Sz) v[o] = gp[zb[o]];
+            cplx<R> a2 = mk<R>(0, 0);
+#pragma unroll
+            for (int o = 0; o < SZ; ++o)
+                if (o < g.Sz) fma_rc(a2, wz[o], v[o]);
+            fma_rc(acc, wxy, a2);
+            ox += sx;
+            oy += sy;
+            if (oy >= S) { oy -= S; ++ox; }
         }
-        Y[row * M + m] = v;
     }
+    // group 0 collects the groups in order
+    for (int k = 1; k < ng; ++k) {
+        const R x = __shfl_sync(0xffffffffu, acc.x, (k * B + b) & 31), y = __shfl_sync(0xffffffffu, acc.y, (k * B + b) & 31);
+        if (grp == 0) acc += mk<R>(x, y);
+    }
+    if constexpr (WPT > 1) {
+        if (grp == 0) red[warp][b] = acc;
+        __syncthreads();
+        if (wi == 0 && grp == 0)
+            for (int k = 1; k < WPT; ++k) acc += red[warp + k][b];
+    }
+    if (!use || grp != 0 || wi != 0) return;
+    double2 v = to_d(acc);
+    v.x *= factor; v.y *= factor;
+    const int m = b - comp * M;
+    const size_t row = (comp < 3) ? size_t(3 * j + comp) : size_t(3 * Nt + 5 * q + comp - 3);
+    if (accumulate && comp < 3) {
+        v += Y[row * M + m];
+        if (jsc) {
+            const double2 sv = jsc[size_t(j) * M + m];
+            const double den = sv.x * sv.x + sv.y * sv.y;
+            if (den > 1e-30) v = v * make_double2(sv.x / den, -sv.y / den);
+        }
+    }
+    Y[row * M + m] = v;
 }
 
 // ------------------------------------------------------------ neighbours
@@ -1293,11 +1368,10 @@ __global__ void __launch_bounds__(128) k_real(const double2* __restrict__ X, dou
     const double sign = (a.solver_ax || a.pairs_plus) ? 1.0 : -1.0;
     const double selfc = selfv ? selfv[j] : a.selfo;  // polydisperse: self value of the particle's radius class
     const int qt = (QUADS && quad_map && j < a.N) ? quad_map[j] : -1;
-    // fewer than 32 columns (dipoles only): the warp splits into 32 / gsz
-    // groups of gsz lanes (gsz = M rounded up to a power of two); group g
+    // fewer than 32 columns: the warp splits into 32 / gsz groups of gsz lanes (gsz = M rounded up to a power of two); group g
     // takes pairs p0 + g, p0 + g + 32/gsz, ... and the groups' sums meet in a
     // fixed shuffle tree
-    const int gsz = (!QUADS && M < 32) ? (M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16) : 32;
+    const int gsz = M < 32 ? (M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16) : 32;
     const int ng = 32 / gsz, grp = lane / gsz;
     for (int m0 = 0; m0 < M; m0 += gsz) {
         const int m = m0 + lane % gsz;
@@ -1315,8 +1389,7 @@ __global__ void __launch_bounds__(128) k_real(const double2* __restrict__ X, dou
                 e2.y += __shfl_xor_sync(0xffffffffu, e2.y, o);
             }
         }
-        if (m >= M || grp != 0) continue;
-        for (int p = p0; QUADS && p < p1; ++p) {
+        for (int p = p0 + grp; QUADS && m < M && p < p1; p += ng) {
             const int i = src[p];
             const R* t = T + 8 * size_t(p);
             const R dx = t[0], dy = t[1], dz = t[2], perp = t[3], para = t[4];
@@ -1370,6 +1443,21 @@ __global__ void __launch_bounds__(128) k_real(const double2* __restrict__ X, dou
                 }
             }
         }
+        if constexpr (QUADS) {
+            for (int o = gsz; o < 32; o <<= 1) {
+                e0.x += __shfl_xor_sync(0xffffffffu, e0.x, o);
+                e0.y += __shfl_xor_sync(0xffffffffu, e0.y, o);
+                e1.x += __shfl_xor_sync(0xffffffffu, e1.x, o);
+                e1.y += __shfl_xor_sync(0xffffffffu, e1.y, o);
+                e2.x += __shfl_xor_sync(0xffffffffu, e2.x, o);
+                e2.y += __shfl_xor_sync(0xffffffffu, e2.y, o);
+                for (int c = 0; c < 5; ++c) {
+                    G[c].x += __shfl_xor_sync(0xffffffffu, G[c].x, o);
+                    G[c].y += __shfl_xor_sync(0xffffffffu, G[c].y, o);
+                }
+            }
+        }
+        if (m >= M || grp != 0) continue;
         double2 out[3] = {to_d(e0) * sign, to_d(e1) * sign, to_d(e2) * sign};
         double2 inv = make_double2(1.0, 0.0);
         double2 s = make_double2(0.0, 0.0);
@@ -1766,7 +1854,8 @@ void Field::set_positions(const double* x, const double* y, const double* z, int
     precalc(s);
 }
 
-void Field::set_field_points(const double* x, const double* y, const double* z, int n, cudaStream_t s) {
+void Field::set_field_points(const double* x, const double* y, const double* z, int n, cudaStream_t s,
+                             bool rebuild) {
     if (spec_.solver_ax) throw std::runtime_error("Cannot update field coordinates when SOLVER_AX mode is active.");
     targets_.n = n;
     targets_.xyz.ensure(sizeof(double) * 3 * std::max(n, 1));
@@ -1774,7 +1863,7 @@ void Field::set_field_points(const double* x, const double* y, const double* z, 
     MPM_CUDA(cudaMemcpyAsync(targets_.xyz.as<double>() + n, y, sizeof(double) * n, cudaMemcpyHostToDevice, s));
     MPM_CUDA(cudaMemcpyAsync(targets_.xyz.as<double>() + 2 * n, z, sizeof(double) * n, cudaMemcpyHostToDevice, s));
     precalc_dirty_ = true;
-    if (N_ > 0) precalc(s);
+    if (N_ > 0 && rebuild) precalc(s);
 }
 
 void Field::choose_layout(cudaStream_t) {
@@ -2165,7 +2254,12 @@ void Field::precalc(cudaStream_t s) {
             if (!gv_.pruned) fftz_.init(gv_.Nz);
         }
         build_stencil(sources_, s, true);
-        build_spread_plan(s);
+        // a solve applies the operator many times per frame; a field at points
+        // is applied once, and the plan costs several spreads (near field of
+        // 1000 particles on 185 x 41 x 240: 2 x 165 us against 70 us more
+        // per spread without it)
+        if (spec_.solver_ax) build_spread_plan(s);
+        else plan_cap_ = 0;
         if (!spec_.solver_ax) build_stencil(targets_, s, false);  // SOLVER_AX: targets share the source stencil
         build_pairs(s);
         if (use_slab()) {
@@ -2250,7 +2344,7 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
     // spread
     const PointSet& ps = sources_;
     const int TX = ps.tile[0], TY = ps.tile[1], TZ = ps.tile[2];
-    const int bc = sizeof(R) == 4 ? 32 : 16;
+    const int bc = std::min(B, sizeof(R) == 4 ? 32 : 16);
     const int cap = 96;
     const size_t ncol = size_t(TX) * TY;
     const size_t shm = sizeof(R) * cap * (TX + TY + TZ) + sizeof(cplx<R>) * cap * bc +
@@ -2261,7 +2355,9 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
     const R* w1 = sizeof(R) == 4 ? reinterpret_cast<const R*>(ps.w32.p) : reinterpret_cast<const R*>(ps.w64.p);
     Profiler::get().begin(ST_SPREAD, s);
     if (plan_cap_ > 0) {
-        const size_t pshm = sizeof(cplx<R>) * size_t(plan_cap_) * bc;
+        // moments, z weights (multi-slot tiles), contributor lists
+        const size_t pshm = sizeof(cplx<R>) * size_t(plan_cap_) * bc + sizeof(R) * size_t(plan_cap_) * TZ +
+                            (sizeof(R) + sizeof(int)) * ncol * kSpreadListCap + sizeof(int) * ncol;
         const bool f32 = sizeof(R) == 4;
         const R* wT = f32 ? reinterpret_cast<const R*>(plan_w32_.p) : reinterpret_cast<const R*>(plan_w64_.p);
         const R* lw = f32 ? reinterpret_cast<const R*>(plan_lw32_.p) : reinterpret_cast<const R*>(plan_lw64_.p);
@@ -2273,9 +2369,8 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
         };
         // the tile's z run in registers: as many accumulators as it needs
         if (TZ == 1 && gv_.Zs == 1) {
-            const size_t lshm = pshm + (sizeof(R) + sizeof(int)) * ncol * kSpreadListCap + sizeof(int) * ncol;
-            set_smem_limit(k_spread_planned_1z<R>, lshm);
-            k_spread_planned_1z<R><<<grd, 256, lshm, s>>>(X, M, N_, C, quad_map_.as<int>(), gv_, TX, TY, ps.nb[0],
+            set_smem_limit(k_spread_planned_1z<R>, pshm);
+            k_spread_planned_1z<R><<<grd, 256, pshm, s>>>(X, M, N_, C, quad_map_.as<int>(), gv_, TX, TY, ps.nb[0],
                                                           ps.nb[1], plan_cap_, bc, plan_nc_.as<int>(),
                                                           plan_cid_.as<int>(), wT, lw, plan_lc_.as<int>(),
                                                           plan_ln_.as<int>(), grid);
@@ -2357,20 +2452,22 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
     if (ov) MPM_CUDA(cudaStreamWaitEvent(s, ov->join, 0));   // the real-space part is in Y
     auto contract = [&](auto kern) {
         kern<<<nt, thr, 0, s>>>(grid, gv_, M, C, nt, tg.base.as<int4>(), tw, factor,
-                                spec_.solver_ax ? quad_map_.as<int>() : nullptr, Y, 0,
+                                spec_.solver_ax ? quad_map_.as<int>() : nullptr, Y,
                                 spec_.solver_ax ? sources_.idx_sorted.as<int>() : nullptr, ov ? 1 : 0,
                                 ov ? ov->jacobi_sc : nullptr);
     };
-    if (gv_.Sz == 1 && C == 3 && B <= 16) {
-        const int gsz = B <= 4 ? 4 : B <= 8 ? 8 : 16;
-        const int per = 128 / gsz;
-        auto small = [&](auto kern) {
-            kern<<<nblk(nt, per), 128, 0, s>>>(grid, gv_, M, nt, tg.base.as<int4>(), tw, factor, Y, 0,
-                                               spec_.solver_ax ? sources_.idx_sorted.as<int>() : nullptr,
-                                               ov ? 1 : 0, ov ? ov->jacobi_sc : nullptr, gsz);
+    if (B <= 16 && gv_.Sz <= 13) {
+        auto few = [&](auto kern, int tpc) {
+            kern<<<nblk(nt, tpc), 128, 0, s>>>(grid, gv_, M, C, nt, tg.base.as<int4>(), tw, factor,
+                                               spec_.solver_ax ? quad_map_.as<int>() : nullptr, Y,
+                                               spec_.solver_ax ? sources_.idx_sorted.as<int>() : nullptr, ov ? 1 : 0,
+                                               ov ? ov->jacobi_sc : nullptr);
         };
-        if (gv_.S == 9) small(k_contract_small<R, 9>);
-        else small(k_contract_small<R, 0>);
+        // four warps per target below 16 warps per SM in all
+        const bool one = nt >= 16 * 148;
+        if (gv_.Sz == 1) one ? few(k_contract_few<R, 1, 1>, 4) : few(k_contract_few<R, 1, 4>, 1);
+        else if (gv_.Sz <= 9) one ? few(k_contract_few<R, 9, 1>, 4) : few(k_contract_few<R, 9, 4>, 1);
+        else one ? few(k_contract_few<R, 13, 1>, 4) : few(k_contract_few<R, 13, 4>, 1);
     } else if (gv_.Sz == 1) {
         if (gv_.S == 9) contract(k_contract<R, 1, 9>);
         else contract(k_contract<R, 1, 0>);

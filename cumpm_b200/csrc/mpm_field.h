@@ -127,7 +127,9 @@ public:
     // Host coordinate arrays (already non-dimensionalised).  In SOLVER_AX
     // mode the field points are the particles.
     void set_positions(const double* x, const double* y, const double* z, int n, cudaStream_t s);
-    void set_field_points(const double* x, const double* y, const double* z, int n, cudaStream_t s);
+    // rebuild = false: set_positions follows and rebuilds the per-frame tables
+    void set_field_points(const double* x, const double* y, const double* z, int n, cudaStream_t s,
+                          bool rebuild = true);
 
     // Y = A X for M right-hand sides.  self_coef: device [N][M] complex (may
     // be null => zero), jacobi: apply diag(self_coef)^-1 to the result rows.

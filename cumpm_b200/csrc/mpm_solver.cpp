@@ -635,7 +635,7 @@ std::vector<double> NearField::calculate() {
     std::vector<double> x(N_), y(N_), z(N_), a(M), b(M), c(M);
     for (size_t i = 0; i < N_; ++i) { x[i] = px_[i] / length_scale_; y[i] = py_[i] / length_scale_; z[i] = pz_[i] / length_scale_; }
     for (size_t i = 0; i < M; ++i) { a[i] = fx_[i] / length_scale_; b[i] = fy_[i] / length_scale_; c[i] = fz_[i] / length_scale_; }
-    field_->set_field_points(a.data(), b.data(), c.data(), int(M), stream_);
+    field_->set_field_points(a.data(), b.data(), c.data(), int(M), stream_, false);
     field_->set_positions(x.data(), y.data(), z.data(), int(N_), stream_);
     dX_.ensure(sizeof(double2) * N_ * 3);
     dY_.ensure(sizeof(double2) * M * 3);
