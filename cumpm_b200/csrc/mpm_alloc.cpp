@@ -1,0 +1,137 @@
+// Device and page-locked host memory of DevBuf / HostBuf (see mpm_common.cuh).
+//
+// A program that solves one parameter set after another builds and drops a
+// solver with some eighty buffers each time; cudaMalloc, cudaFree and above
+// all page-locking cost more than the solve of a small system (a spectrum of
+// the N = 4000 monolayer spent 27 of its 43 ms outside the kernels; with the
+// tables of mpm_tables.cpp 26 ms are left, and passes no longer wait up to a
+// second for the driver's allocator when other processes use it).
+// Released blocks are therefore kept for the next request of about the same
+// size:
+//  * bounded: at most 256 MB of device and 64 MB of host memory, no block
+//    above a quarter of that, and a block that kMaxAge later releases did not
+//    reuse is freed;
+//  * a block is kept only after the device that may still be using it has
+//    been waited for, as cudaFree does, so the next owner may be any thread
+//    and any stream;
+//  * when the driver is out of memory the kept blocks are freed first.
+#include "mpm_common.cuh"
+
+#include <list>
+#include <mutex>
+#include <unordered_map>
+
+namespace mpm {
+
+namespace {
+
+struct Pool {
+    struct Block {
+        void* p;
+        size_t bytes;
+        int dev;
+        unsigned long long born;
+    };
+    std::mutex mu;
+    std::list<Block> kept;                                   // oldest first
+    std::unordered_map<void*, std::pair<size_t, int>> live;  // size, device
+    size_t total = 0;
+    unsigned long long clock = 0;
+    const bool host;
+    const size_t cap;
+    Pool(bool h, size_t c) : host(h), cap(c) {}
+
+    void drop(const Block& b) {
+        if (host) cudaFreeHost(b.p);
+        else cudaFree(b.p);
+    }
+    // frees kept blocks: all of them, or those past the age limit and beyond the cap
+    void trim(bool all) {
+        while (!kept.empty() && (all || total > cap || clock - kept.front().born > kMaxAge)) {
+            total -= kept.front().bytes;
+            drop(kept.front());
+            kept.pop_front();
+        }
+    }
+    static constexpr unsigned long long kMaxAge = 1024;
+};
+
+// (never destroyed: buffers of static objects may outlive this file's statics)
+Pool& pool(bool host) {
+    static Pool* dev = new Pool(false, size_t(256) << 20);
+    static Pool* hst = new Pool(true, size_t(64) << 20);
+    return host ? *hst : *dev;
+}
+
+size_t rounded(size_t n) {
+    size_t unit = 512;
+    while (unit * 8 < n) unit *= 2;      // steps of an eighth
+    return (n + unit - 1) / unit * unit;
+}
+
+}  // namespace
+
+void* buf_alloc(size_t n, bool host) {
+    Pool& P = pool(host);
+    int dev = 0;
+    MPM_CUDA(cudaGetDevice(&dev));
+    const size_t want = rounded(n);
+    std::lock_guard<std::mutex> lock(P.mu);
+    auto best = P.kept.end();
+    for (auto it = P.kept.begin(); it != P.kept.end(); ++it)
+        if (it->bytes >= want && it->bytes <= want + want / 4 + 4096 && (host || it->dev == dev) &&
+            (best == P.kept.end() || it->bytes < best->bytes))
+            best = it;
+    void* p = nullptr;
+    size_t got = want;
+    if (best != P.kept.end()) {
+        p = best->p;
+        got = best->bytes;
+        P.total -= got;
+        P.kept.erase(best);
+    } else {
+        auto get = [&] { return host ? cudaHostAlloc(&p, want, cudaHostAllocPortable) : cudaMalloc(&p, want); };
+        cudaError_t e = get();
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            P.trim(true);
+            e = get();
+        }
+        MPM_CUDA(e);
+    }
+    P.live[p] = {got, dev};
+    return p;
+}
+
+void buf_free(void* p, bool host) {
+    if (!p) return;
+    Pool& P = pool(host);
+    std::pair<size_t, int> b;
+    {
+        std::lock_guard<std::mutex> lock(P.mu);
+        auto it = P.live.find(p);
+        if (it == P.live.end()) return;
+        b = it->second;
+        P.live.erase(it);
+    }
+    // wait for whatever still uses the block (outside the lock)
+    bool idle = b.first <= P.cap / 4;
+    if (idle) {
+        int cur = 0;
+        idle = cudaGetDevice(&cur) == cudaSuccess;
+        if (idle && cur != b.second) idle = cudaSetDevice(b.second) == cudaSuccess;
+        if (idle) idle = cudaDeviceSynchronize() == cudaSuccess;
+        if (cur != b.second) cudaSetDevice(cur);
+    }
+    if (!idle) {       // too large, or the device is not in a state to keep anything
+        if (host) cudaFreeHost(p);
+        else cudaFree(p);
+        return;
+    }
+    std::lock_guard<std::mutex> lock(P.mu);
+    P.kept.push_back({p, b.first, b.second, ++P.clock});
+    P.total += b.first;
+    P.trim(false);
+}
+
+}  // namespace mpm

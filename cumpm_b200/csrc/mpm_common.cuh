@@ -100,16 +100,22 @@ constexpr double kPi = 3.14159265358979323846;
 
 // --------------------------------------------------------------- buffers --
 
-// Minimal owning device buffer (cudaMalloc/cudaFree, no caching allocator).
-struct DevBuf {
+// device (or page-locked host) memory from / to the bounded cache of
+// mpm_alloc.cpp; buf_free waits for the device, as cudaFree does
+void* buf_alloc(size_t n, bool host);
+void buf_free(void* p, bool host);
+
+// Owning buffer; contents do not survive a growing ensure().
+template <bool HOST>
+struct Buffer {
     void* p = nullptr;
     size_t bytes = 0;
-    DevBuf() = default;
-    DevBuf(const DevBuf&) = delete;
-    DevBuf& operator=(const DevBuf&) = delete;
-    ~DevBuf() { release(); }
+    Buffer() = default;
+    Buffer(const Buffer&) = delete;
+    Buffer& operator=(const Buffer&) = delete;
+    ~Buffer() { release(); }
     void release() {
-        if (p) cudaFree(p);
+        if (p) buf_free(p, HOST);
         p = nullptr;
         bytes = 0;
     }
@@ -117,34 +123,14 @@ struct DevBuf {
         if (n <= bytes && p) return;
         release();
         if (n == 0) return;
-        MPM_CUDA(cudaMalloc(&p, n));
+        p = buf_alloc(n, HOST);
         bytes = n;
     }
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
-
+using DevBuf = Buffer<false>;
 // Page-locked host buffer (reused across calls, so host<->device copies run
 // at full PCIe/C2C speed and never fault fresh pages).
-struct HostBuf {
-    void* p = nullptr;
-    size_t bytes = 0;
-    HostBuf() = default;
-    HostBuf(const HostBuf&) = delete;
-    HostBuf& operator=(const HostBuf&) = delete;
-    ~HostBuf() { release(); }
-    void release() {
-        if (p) cudaFreeHost(p);
-        p = nullptr;
-        bytes = 0;
-    }
-    void ensure(size_t n) {
-        if (n <= bytes && p) return;
-        release();
-        if (n == 0) return;
-        MPM_CUDA(cudaHostAlloc(&p, n, cudaHostAllocDefault));
-        bytes = n;
-    }
-    template <typename T> T* as() const { return static_cast<T*>(p); }
-};
+using HostBuf = Buffer<true>;
 
 }  // namespace mpm

@@ -1772,11 +1772,11 @@ Field::Field(const FieldSpec& spec) : spec_(spec) {
         if (spec_.tile[0] * spec_.tile[1] > 128 || (spec_.tile[0] == 0 ? 8 : spec_.tile[0]) *
                                                            (spec_.tile[1] == 0 ? 8 : spec_.tile[1]) > 128)
             throw std::invalid_argument("a spread tile holds at most 128 columns");
-        tables_ = build_mono_tables(spec_.xi);
+        tables_ = build_mono_tables(spec_.xi, spec_.quads);
         tab_r_.ensure(sizeof(double) * kTableSize);
         tab_f_.ensure(sizeof(double) * kTableSize * T_COUNT);
         MPM_CUDA(cudaMemcpy(tab_r_.p, tables_.r.data(), sizeof(double) * kTableSize, cudaMemcpyHostToDevice));
-        for (int f = 0; f < T_COUNT; ++f)
+        for (int f = 0; f < (spec_.quads ? int(T_COUNT) : int(T_FD2) + 1); ++f)
             MPM_CUDA(cudaMemcpy(tab_f_.as<double>() + size_t(f) * kTableSize, tables_.f[f].data(),
                                 sizeof(double) * kTableSize, cudaMemcpyHostToDevice));
     } else if (spec_.kind == FIELD_POLY) {

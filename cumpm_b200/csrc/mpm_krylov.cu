@@ -981,23 +981,13 @@ __global__ void k_inner_tol(const double* __restrict__ rn, const double* __restr
 
 // ------------------------------------------------------------ host side --
 
-BatchSolver::BatchSolver() {
-    MPM_CUDA(cudaMallocHost(&flag_, sizeof(int)));
-    flag_cap_ = 1;
-}
-BatchSolver::~BatchSolver() {
-    if (flag_) cudaFreeHost(flag_);
-    if (hidx_) cudaFreeHost(hidx_);
-}
+BatchSolver::BatchSolver() = default;
+BatchSolver::~BatchSolver() = default;
 
 int BatchSolver::read_flags(const int* dflag, int M, cudaStream_t s) {
-    if (M + 1 > flag_cap_) {
-        MPM_CUDA(cudaStreamSynchronize(s));
-        if (flag_) MPM_CUDA(cudaFreeHost(flag_));
-        flag_ = nullptr;
-        MPM_CUDA(cudaMallocHost(&flag_, sizeof(int) * (M + 1)));
-        flag_cap_ = M + 1;
-    }
+    // (no copy into the words is in flight: every read ends with a wait)
+    flagbuf_.ensure(sizeof(int) * (size_t(M) + 1));
+    flag_ = flagbuf_.as<int>();
     MPM_CUDA(cudaMemcpyAsync(flag_, dflag, sizeof(int) * (M + 1), cudaMemcpyDeviceToHost, s));
     MPM_CUDA(cudaStreamSynchronize(s));
     return *flag_;
@@ -1022,18 +1012,12 @@ int BatchSolver::apply_cols(Field& F, const double2* X, double2* Y, int M, const
     const int rin = F.rows_in(), rout = F.rows_out(), N = F.num_particles();
     if (cols != cur_cols_) {
         StageScope scope(ST_KRYLOV, s);
-        if (Ma > hidx_cap_) {
-            MPM_CUDA(cudaStreamSynchronize(s));
-            if (hidx_) MPM_CUDA(cudaFreeHost(hidx_));
-            hidx_ = nullptr;
-            MPM_CUDA(cudaMallocHost(&hidx_, sizeof(int) * M));
-            hidx_cap_ = M;
-        }
         // the previous upload from hidx_ has completed: every change of the
         // column set follows a flag read, which synchronises the stream
-        std::copy(cols.begin(), cols.end(), hidx_);
+        hidx_.ensure(sizeof(int) * M);
+        std::copy(cols.begin(), cols.end(), hidx_.as<int>());
         cidx_.ensure(sizeof(int) * M);
-        MPM_CUDA(cudaMemcpyAsync(cidx_.p, hidx_, sizeof(int) * Ma, cudaMemcpyHostToDevice, s));
+        MPM_CUDA(cudaMemcpyAsync(cidx_.p, hidx_.p, sizeof(int) * Ma, cudaMemcpyHostToDevice, s));
         if (sc) {
             scc_.ensure(sizeof(double2) * size_t(N) * M);
             k_gather_cols<<<nblk((long long)N * Ma, 256), 256, 0, s>>>(sc, M, scc_.as<double2>(), Ma,

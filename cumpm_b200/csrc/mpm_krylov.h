@@ -124,10 +124,8 @@ private:
     DevBuf sel_, rn64_;                  // refinement: columns re-checked in fp64, their |r|
     DevBuf dots_done_;                   // see done_counter
     DevBuf shf_, shflag_, shmeta_, shsc_, shb_, shst_;   // shifted solve: detection, seeds, members
-    int* flag_ = nullptr;                // pinned host words: count + per-column flags
-    int flag_cap_ = 0;
-    int* hidx_ = nullptr;                // pinned host column list for the gather
-    int hidx_cap_ = 0;
+    HostBuf flagbuf_, hidx_;             // count + per-column flags; column list for the gather
+    int* flag_ = nullptr;                // the words of flagbuf_
     std::vector<int> cur_cols_;          // column list the device buffers hold
     const double2* cur_sc_ = nullptr;    // self coefficients gathered into scc_
 };

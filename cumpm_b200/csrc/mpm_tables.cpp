@@ -22,12 +22,24 @@ struct Terms {
     double ep, em, e0, fp, fm, f0, reg;
 };
 
-inline double combine(double r, double xi, const Terms& t) {
-    const double x2 = xi * xi;
-    double v = t.ep * std::exp(-(r + 2.0) * (r + 2.0) * x2) + t.fp * std::erfc((r + 2.0) * xi) +
-               t.em * std::exp(-(r - 2.0) * (r - 2.0) * x2) + t.fm * std::erfc((r - 2.0) * xi) +
-               t.e0 * std::exp(-r * r * x2) + t.f0 * std::erfc(r * xi);
-    if (r < 2.0) v += t.reg;
+// the exponentials and error functions at one r, shared by every function
+// there (they are most of a table's cost)
+struct Basis {
+    double r, ep, em, e0, fp, fm, f0;
+    Basis(double r_, double xi) : r(r_) {
+        const double x2 = xi * xi;
+        ep = std::exp(-(r + 2.0) * (r + 2.0) * x2);
+        fp = std::erfc((r + 2.0) * xi);
+        em = std::exp(-(r - 2.0) * (r - 2.0) * x2);
+        fm = std::erfc((r - 2.0) * xi);
+        e0 = std::exp(-r * r * x2);
+        f0 = std::erfc(r * xi);
+    }
+};
+
+inline double combine(const Basis& b, const Terms& t) {
+    double v = t.ep * b.ep + t.fp * b.fp + t.em * b.em + t.fm * b.fm + t.e0 * b.e0 + t.f0 * b.f0;
+    if (b.r < 2.0) v += t.reg;
     return v;
 }
 
@@ -305,18 +317,20 @@ double gradient_self_value(double xi) {
 
 }  // namespace
 
-MonoTables build_mono_tables(double xi) {
+MonoTables build_mono_tables(double xi, bool quads) {
     MonoTables T;
+    const int nf = quads ? int(T_COUNT) : int(T_FD2) + 1;
     const Powers p(xi);
     T.r.resize(kTableSize);
-    for (auto& v : T.f) v.resize(kTableSize);
+    for (int f = 0; f < nf; ++f) T.f[f].resize(kTableSize);
     using Fn = Terms (*)(double, const Powers&);
     const Fn fns[T_COUNT] = {fd1_terms, fd2_terms, fq1_terms, fq2_terms, fq3_terms,
                              gq1_terms, gq2_terms, gq3_terms, gq4_terms};
     for (int k = 0; k < kTableSteps; ++k) {
         const double r = 1.0 + k * kTableDr;
         T.r[k + 1] = r;
-        for (int f = 0; f < T_COUNT; ++f) T.f[f][k + 1] = combine(r, xi, fns[f](r, p));
+        const Basis e(r, xi);
+        for (int f = 0; f < nf; ++f) T.f[f][k + 1] = combine(e, fns[f](r, p));
     }
     const double x2 = p.x2;
     T.selfo = (-1.0 + 6.0 * x2 + (1.0 - 2.0 * x2) * std::exp(-4.0 * x2)) / (16.0 * std::pow(PI, 1.5) * x2 * xi) +
@@ -325,6 +339,7 @@ MonoTables build_mono_tables(double xi) {
     T.r[0] = 0.0;
     T.f[T_FD1][0] = T.selfo;
     T.f[T_FD2][0] = T.selfo;
+    if (!quads) return T;
     T.f[T_FQ1][0] = T.f[T_FQ2][0] = T.f[T_FQ3][0] = 0.0;
     for (int f = T_GQ1; f <= T_GQ4; ++f) T.f[f][0] = T.self_grad;
     return T;
@@ -341,7 +356,8 @@ PolyQuadTables build_poly_quad_tables(double xi, int n_nodes) {
     for (int k = 0; k + 1 < n_nodes; ++k) {
         const double r = 1.0 + k * kTableDr;
         T.r[k + 1] = r;
-        for (int f = 0; f < PQ_COUNT; ++f) T.f[f][k + 1] = combine(r, xi, fns[f](r, p));
+        const Basis e(r, xi);
+        for (int f = 0; f < PQ_COUNT; ++f) T.f[f][k + 1] = combine(e, fns[f](r, p));
     }
     T.self_grad = gradient_self_value(xi);
     T.r[0] = 0.0;

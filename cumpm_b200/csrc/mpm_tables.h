@@ -22,7 +22,8 @@ struct MonoTables {
     double self_grad = 0.0;                // r = 0 entry of the gradient tables
 };
 
-MonoTables build_mono_tables(double xi);
+// quads = false: the two dipole tables only (the others stay empty)
+MonoTables build_mono_tables(double xi, bool quads = true);
 
 // Radius-1 quadrupole tables of the polydisperse field
 // (polydisperse_ewald_electric_field.cu:1690-2035): nodes r = 0 and
