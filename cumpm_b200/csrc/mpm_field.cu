@@ -415,6 +415,11 @@ __global__ void __launch_bounds__(256) k_spread_plan(const int4* __restrict__ ba
     }
 }
 
+// staged contributor lists are padded to whole fours with weight-0 entries of
+// candidate 0, so that four list steps' loads issue together (the capacity is
+// a multiple of four; -1 marks a list that overflowed)
+__device__ __forceinline__ int list_padded(int n) { return n > 0 ? (n + 3) & ~3 : 0; }
+
 // Spread with the per-frame plan: CTA = one tile x one chunk of bc grid
 // columns; stages the tile's candidate moments and z weights and every (x, y)
 // column's contributor list in shared memory, then thread = one (x, y) column
@@ -480,10 +485,14 @@ __global__ void __launch_bounds__(256) k_spread_planned(const double2* __restric
                 for (int u = 0; u < kCPW; ++u) {
                     const int col = col0 + u * nwarp, k = k0 + lane;
                     cc[u] = -1;
-                    if (col < ncol && k < lnS[col]) {
-                        const size_t lrow = (size_t(tile) * ncol + col) * kSpreadListCap;
-                        cc[u] = lcT[lrow + k];
-                        ww[u] = lwT[lrow + k];
+                    ww[u] = R(0);
+                    if (col < ncol && k < list_padded(lnS[col])) {
+                        cc[u] = 0;
+                        if (k < lnS[col]) {
+                            const size_t lrow = (size_t(tile) * ncol + col) * kSpreadListCap;
+                            cc[u] = lcT[lrow + k];
+                            ww[u] = lwT[lrow + k];
+                        }
                     }
                 }
 #pragma unroll
@@ -509,14 +518,22 @@ __global__ void __launch_bounds__(256) k_spread_planned(const double2* __restric
         if (nl >= 0) {
             const int* lc = lcS + col * kSpreadListCap;
             const R* lw = lwS + col * kSpreadListCap;
-            for (int k = 0; k < nl; ++k) {
-                const int c = lc[k];
-                const R wxy = lw[k];
-                const cplx<R> pc = pv[c * bc + bb];
-                const R* wzc = wz + c * TZ;
+            for (int k = 0; k < nl; k += 4) {
+                int c[4];
+                cplx<R> v[4];
 #pragma unroll
-                for (int lz = 0; lz < ZMAX; ++lz)
-                    if (lz < TZ) fma_rc(acc[lz], wxy * wzc[lz], pc);
+                for (int u = 0; u < 4; ++u) {
+                    c[u] = lc[k + u];
+                    v[u] = pv[c[u] * bc + bb];
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const R wxy = lw[k + u];
+                    const R* wzc = wz + c[u] * TZ;
+#pragma unroll
+                    for (int lz = 0; lz < ZMAX; ++lz)
+                        if (lz < TZ) fma_rc(acc[lz], wxy * wzc[lz], v[u]);
+                }
             }
         } else {   // list overflowed: every candidate, in order
             for (int c = 0; c < nc; ++c) {
@@ -572,6 +589,7 @@ __global__ void __launch_bounds__(256) k_spread_planned_1z(const double2* __rest
     const int b0 = chunk * bc;
     const int nb = min(bc, B - b0);
     const R* wTt = wT + trow * wlen;
+#pragma unroll 4
     for (int t = threadIdx.x; t < nc * nb; t += blockDim.x) {
         const int c = t / nb, bb = t % nb;
         const int i = cidT[trow + c];
@@ -598,10 +616,14 @@ __global__ void __launch_bounds__(256) k_spread_planned_1z(const double2* __rest
             for (int u = 0; u < kCPW; ++u) {
                 const int col = col0 + u * nwarp, k = k0 + lane;
                 cc[u] = -1;
-                if (col < ncol && k < lnS[col]) {
-                    const size_t lrow = (size_t(tile) * ncol + col) * kSpreadListCap;
-                    cc[u] = lcT[lrow + k];
-                    ww[u] = lwT[lrow + k];
+                ww[u] = R(0);
+                if (col < ncol && k < list_padded(lnS[col])) {
+                    cc[u] = 0;
+                    if (k < lnS[col]) {
+                        const size_t lrow = (size_t(tile) * ncol + col) * kSpreadListCap;
+                        cc[u] = lcT[lrow + k];
+                        ww[u] = lwT[lrow + k];
+                    }
                 }
             }
 #pragma unroll
@@ -628,7 +650,13 @@ __global__ void __launch_bounds__(256) k_spread_planned_1z(const double2* __rest
         for (int bb = sl; bb < nb; bb += gsz) {
             cplx<R> acc = mk<R>(0, 0);
             if (nl >= 0) {
-                for (int k = 0; k < nl; ++k) fma_rc(acc, lw[k], pv[lc[k] * bc + bb]);
+                for (int k = 0; k < nl; k += 4) {
+                    cplx<R> v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = pv[lc[k + u] * bc + bb];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) fma_rc(acc, lw[k + u], v[u]);
+                }
             } else {   // list overflowed: every candidate, in order
                 for (int c = 0; c < nc; ++c) {
                     const R* wc = wTt + c * wlen;

@@ -3,6 +3,7 @@
 #include "mpm_profile.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 namespace mpm {
@@ -337,28 +338,29 @@ __device__ void gm_givens(GState& s, const double2* __restrict__ h, double wn, d
     }
 }
 
-// The one-CTA kernel after a projection's sums.  pass 1, h = [V_0..V_k, u]^H u
+// What follows a projection's sums, by one CTA.  First, h = [V_0..V_k, u]^H u
 // with u = w - V_k: h_k += 1 (the coefficients of w) and the cycling columns
-// marked for their second projection.  pass 2, h2 = [V_0..V_k, w']^H w' after
-// the first: h += h2, |w''| by Pythagoras, the Givens update (givens = 0, the
-// seeds of a shifted solve: none, they are the members', shift_givens_body).
-// flag[0] = columns still cycling, flag[1 + m] = column m cycling.
-__device__ __forceinline__ void arn_finish_body(GState* __restrict__ st, double2* __restrict__ h,
-                                                const double2* __restrict__ h2, int pass, int givens,
-                                                double* __restrict__ nu_out, double* __restrict__ inv_nu,
-                                                double2* __restrict__ H, double2* __restrict__ g,
-                                                double* __restrict__ cs, double2* __restrict__ sn, int k, int restart,
-                                                int M, const double* __restrict__ bn, double tol,
-                                                const double* __restrict__ tolv, int maxiter,
-                                                int* __restrict__ flag) {
-    if (pass == 1) {
-        for (int m = threadIdx.x; m < M; m += blockDim.x) {
-            const int cyc = st[m].cyc;
-            st[m].reorth = cyc ? 1 : 0;
-            if (cyc) h[size_t(k) * M + m].x += 1.0;
-        }
-        return;
+// marked for their second projection.
+__device__ __forceinline__ void arn_finish1_body(GState* __restrict__ st, double2* __restrict__ h, int k, int M) {
+    for (int m = threadIdx.x; m < M; m += blockDim.x) {
+        const int cyc = st[m].cyc;
+        st[m].reorth = cyc ? 1 : 0;
+        if (cyc) h[size_t(k) * M + m].x += 1.0;
     }
+}
+
+// Second, h2 = [V_0..V_k, w']^H w' after the first: h += h2, |w''| by
+// Pythagoras, the Givens update (givens = 0, the seeds of a shifted solve:
+// none, they are the members', shift_givens_body).  flag[0] = columns still
+// cycling, flag[1 + m] = column m cycling.
+__device__ __forceinline__ void arn_finish2_body(GState* __restrict__ st, double2* __restrict__ h,
+                                                 const double2* __restrict__ h2, int givens,
+                                                 double* __restrict__ nu_out, double* __restrict__ inv_nu,
+                                                 double2* __restrict__ H, double2* __restrict__ g,
+                                                 double* __restrict__ cs, double2* __restrict__ sn, int k, int restart,
+                                                 int M, const double* __restrict__ bn, double tol,
+                                                 const double* __restrict__ tolv, int maxiter,
+                                                 int* __restrict__ flag) {
     __shared__ int ncyc;
     if (threadIdx.x == 0) ncyc = 0;
     // (columns not cycling have w' = 0, so h2 = 0)
@@ -393,17 +395,8 @@ __device__ __forceinline__ void arn_finish_body(GState* __restrict__ st, double2
     if (threadIdx.x == 0) flag[0] = ncyc;
 }
 
-__global__ void __launch_bounds__(256) k_arn_finish(GState* __restrict__ st, double2* __restrict__ h,
-                                                     const double2* __restrict__ h2, int pass, int givens,
-                                                     double* __restrict__ nu_out,
-                                                     double* __restrict__ inv_nu, double2* __restrict__ H,
-                                                     double2* __restrict__ g, double* __restrict__ cs,
-                                                     double2* __restrict__ sn, int k, int restart, int M,
-                                                     const double* __restrict__ bn, double tol,
-                                                     const double* __restrict__ tolv, int maxiter,
-                                                     int* __restrict__ flag) {
-    arn_finish_body(st, h, h2, pass, givens, nu_out, inv_nu, H, g, cs, sn, k, restart, M, bn, tol, tolv, maxiter,
-                    flag);
+__global__ void __launch_bounds__(256) k_arn_finish1(GState* __restrict__ st, double2* __restrict__ h, int k, int M) {
+    arn_finish1_body(st, h, k, M);
 }
 
 // V_{k+1} -= sum_{i <= k} V_i h_i for the columns of this pass (pass 1: the
@@ -554,23 +547,35 @@ struct HessArgs {
     double* nu;             // |w'| per seed (shifted), or null
     double* inv_nu;
     int* flag;
+    int* hflag;             // the same words for the host (page-locked): hflag[0] = seq once hflag[1 + t] = flag[t]
+    int seq;
 };
 
 __device__ __forceinline__ void finish2_body(GState* st, double2* h, const double2* h2, const HessArgs& a,
                                              const MemberArgs& mb, int k, int M) {
     const bool seeds = mb.st != nullptr;
-    arn_finish_body(st, h, h2, 2, seeds ? 0 : 1, a.nu, a.inv_nu, a.H, a.g, a.cs, a.sn, k, a.restart, M, a.bn, a.tol,
+    arn_finish2_body(st, h, h2, seeds ? 0 : 1, a.nu, a.inv_nu, a.H, a.g, a.cs, a.sn, k, a.restart, M, a.bn, a.tol,
                     seeds ? nullptr : a.tolv, a.maxiter, a.flag);
-    if (!seeds) return;
     __syncthreads();
-    shift_givens_body(mb.st, st, h, a.nu, mb.sigma, mb.grp, M, a.H, a.g, a.cs, a.sn, k, a.restart, mb.M, a.bn,
-                      mb.tolv, a.maxiter, mb.seed_cyc, a.flag);
+    if (seeds) {
+        shift_givens_body(mb.st, st, h, a.nu, mb.sigma, mb.grp, M, a.H, a.g, a.cs, a.sn, k, a.restart, mb.M, a.bn,
+                          mb.tolv, a.maxiter, mb.seed_cyc, a.flag);
+        __syncthreads();
+    }
+    // the flags go straight to the host, which waits for them while the last
+    // launch of the step still runs
+    for (int t = threadIdx.x; t <= M; t += blockDim.x) a.hflag[1 + t] = a.flag[t];
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) *static_cast<volatile int*>(a.hflag) = a.seq;
 }
 
-__global__ void __launch_bounds__(256) k_seed_finish_givens(GState* __restrict__ sst, double2* __restrict__ h,
-                                                             const double2* __restrict__ h2, HessArgs a,
-                                                             MemberArgs mb, int k, int G) {
-    finish2_body(sst, h, h2, a, mb, k, G);
+// the second finish of many columns (M >= 16), with the members' updates when
+// there are seeds
+__global__ void __launch_bounds__(256) k_arn_finish2(GState* __restrict__ st, double2* __restrict__ h,
+                                                      const double2* __restrict__ h2, HessArgs a, MemberArgs mb,
+                                                      int k, int M) {
+    finish2_body(st, h, h2, a, mb, k, M);
 }
 
 // ---- the Arnoldi step of few columns (M < 16) in three launches
@@ -581,10 +586,10 @@ __global__ void __launch_bounds__(256) k_seed_finish_givens(GState* __restrict__
 // launches separate (dots, finish, update, twice) a step took 44 to 66 us of
 // 5 to 15 us launches, all latency; 31 now (N = 4000, 3 columns, 5 steps).
 
-// pass 1: [V_0 .. V_k, u]^H u for u = w - V_k, then arn_finish_body pass 1
+// [V_0 .. V_k, u]^H u for u = w - V_k, then arn_finish1_body
 __global__ void __launch_bounds__(256) k_arn_dots(const double2* __restrict__ V, size_t vstride, int k, int rows,
                                                   int M, double2* __restrict__ partial, GState* __restrict__ st,
-                                                  double2* __restrict__ h, HessArgs a, unsigned int* __restrict__ done) {
+                                                  double2* __restrict__ h, unsigned int* __restrict__ done) {
     __shared__ double2 red[8][256];
     const int nvec = k + 2;
     const int L = (256 / M) * M;
@@ -612,12 +617,11 @@ __global__ void __launch_bounds__(256) k_arn_dots(const double2* __restrict__ V,
     if (!last_cta(done, gridDim.x * gridDim.z)) return;
     reduce_partials(partial, gridDim.x, nvec * M, h);
     __syncthreads();
-    arn_finish_body(st, h, nullptr, 1, 0, nullptr, a.inv_nu, nullptr, nullptr, nullptr, nullptr, k, a.restart, M, a.bn,
-                    a.tol, nullptr, a.maxiter, a.flag);
+    arn_finish1_body(st, h, k, M);
 }
 
-// w' = w - sum_{i <= k} V_i h_i (columns not cycling: 0), then pass 2:
-// [V_0 .. V_k, w']^H w' into h2, h += h2, the norm and the Givens updates
+// w' = w - sum_{i <= k} V_i h_i (columns not cycling: 0), [V_0 .. V_k, w']^H w'
+// into h2, then finish2_body
 __global__ void __launch_bounds__(256) k_arn_project(double2* __restrict__ V, size_t vstride, int k, int rows, int M,
                                                      double2* __restrict__ partial, GState* __restrict__ st,
                                                      double2* __restrict__ h, double2* __restrict__ h2, HessArgs a,
@@ -993,6 +997,33 @@ int BatchSolver::read_flags(const int* dflag, int M, cudaStream_t s) {
     return *flag_;
 }
 
+int* BatchSolver::poll_words(int M) {
+    const size_t bytes = sizeof(int) * (size_t(M) + 2);
+    if (!poll_.p || poll_.bytes < bytes) {
+        poll_.ensure(bytes);
+        poll_.as<int>()[0] = 0;        // no sequence number (they start at 1)
+    }
+    return poll_.as<int>();
+}
+
+// Waits for the flags of the Arnoldi step with the latest sequence number and
+// returns the count.  The kernel that makes them writes them to page-locked
+// memory, so the host need not wait for the step's last launch nor for a
+// copy; the stream is queried now and then, so that a failed launch ends the
+// wait with its error.
+int BatchSolver::wait_flags(cudaStream_t s) {
+    const volatile int* w = poll_.as<int>();
+    for (unsigned it = 1; w[0] != poll_seq_; ++it) {
+        if (it % 4096) continue;
+        const cudaError_t e = cudaStreamQuery(s);
+        if (e == cudaErrorNotReady) continue;
+        MPM_CUDA(e);
+        if (w[0] != poll_seq_) throw std::runtime_error("Krylov step ended without its flags");
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return w[1];
+}
+
 int BatchSolver::apply_cols(Field& F, const double2* X, double2* Y, int M, const double2* sc, bool jacobi,
                             bool r32, bool re32, const int* active, bool compact, cudaStream_t s) {
     if (!compact || !active) {
@@ -1013,7 +1044,7 @@ int BatchSolver::apply_cols(Field& F, const double2* X, double2* Y, int M, const
     if (cols != cur_cols_) {
         StageScope scope(ST_KRYLOV, s);
         // the previous upload from hidx_ has completed: every change of the
-        // column set follows a flag read, which synchronises the stream
+        // column set follows flags that were made after it on this stream
         hidx_.ensure(sizeof(int) * M);
         std::copy(cols.begin(), cols.end(), hidx_.as<int>());
         cidx_.ensure(sizeof(int) * M);
@@ -1119,7 +1150,7 @@ void BatchSolver::arnoldi(double2* V, int k, int rows, int M, void* state, const
         partial_.ensure(sizeof(double2) * size_t(gx) * (a.restart + 2) * M);
         double2* part = partial_.as<double2>();
         unsigned int* done = done_counter(s);
-        k_arn_dots<<<dim3(gx, 1, (k + 2 + 7) / 8), 256, 0, s>>>(V, n, k, rows, M, part, st, h, a, done);
+        k_arn_dots<<<dim3(gx, 1, (k + 2 + 7) / 8), 256, 0, s>>>(V, n, k, rows, M, part, st, h, done);
         MPM_LAUNCH();
         k_arn_project<<<gx, 256, 0, s>>>(V, n, k, rows, M, part, st, h, h2, a, mb, done);
         MPM_LAUNCH();
@@ -1128,18 +1159,12 @@ void BatchSolver::arnoldi(double2* V, int k, int rows, int M, void* state, const
         const bool seeds = mb.st != nullptr;
         const int fthr = std::min(256, ((std::max(M, seeds ? mb.M : M) + 31) / 32) * 32);
         dots(V, n, k + 2, w, rows, M, 1, h, s, k);
-        k_arn_finish<<<1, fthr, 0, s>>>(st, h, h2, 1, 0, nullptr, a.inv_nu, nullptr, nullptr, nullptr, nullptr, k,
-                                        a.restart, M, a.bn, a.tol, nullptr, a.maxiter, a.flag);
+        k_arn_finish1<<<1, fthr, 0, s>>>(st, h, k, M);
         MPM_LAUNCH();
         k_arn_update<<<vb, 256, 0, s>>>(V, n, k, h, st, a.inv_nu, rows, M, 1);
         MPM_LAUNCH();
         dots(V, n, k + 2, w, rows, M, 1, h2, s);
-        if (seeds) {
-            k_seed_finish_givens<<<1, fthr, 0, s>>>(st, h, h2, a, mb, k, M);
-        } else {
-            k_arn_finish<<<1, fthr, 0, s>>>(st, h, h2, 2, 1, nullptr, a.inv_nu, a.H, a.g, a.cs, a.sn, k, a.restart, M,
-                                            a.bn, a.tol, a.tolv, a.maxiter, a.flag);
-        }
+        k_arn_finish2<<<1, fthr, 0, s>>>(st, h, h2, a, mb, k, M);
         MPM_LAUNCH();
     }
     k_arn_update<<<vb, 256, 0, s>>>(V, n, k, h2, st, a.inv_nu, rows, M, 2);
@@ -1237,13 +1262,13 @@ void BatchSolver::gmres(Field& F, const double2* b, double2* x, int M, const dou
             st.column_matvecs += apply_cols(F, Vk, w, M, sc, opt.jacobi, r32, re32, cyc.data(), opt.compact, s);
             st.matvecs++;
             HessArgs ha{H_.as<double2>(), g_.as<double2>(), cs_.as<double>(), sn_.as<double2>(), bnorm_.as<double>(),
-                        opt.tol, tolv, opt.maxiter, restart, nullptr, rnorm_.as<double>(), dflag};
+                        opt.tol, tolv, opt.maxiter, restart, nullptr, rnorm_.as<double>(), dflag, poll_words(M), ++poll_seq_};
             arnoldi(V, k, rows, M, gs, ha, MemberArgs{}, s);
             st.reorth_steps++;
             // the count and the M column flags
-            const int left = read_flags(dflag, M, s);
+            const int left = wait_flags(s);
             if (left == 0) break;
-            cyc.assign(flag_ + 1, flag_ + 1 + M);
+            cyc.assign(poll_.as<int>() + 2, poll_.as<int>() + 2 + M);
         }
         backsub(gs, H_.as<double2>(), g_.as<double2>(), y_.as<double2>(), restart, M, kper, s);
         k_vupdate<<<vb, 256, 0, s>>>(x, V, n, restart, y_.as<double2>(), rows, M, 1.0, kper);
@@ -1371,12 +1396,12 @@ void BatchSolver::gmres_shifted(Field& F, const double2* b, double2* x, int M, c
         st.column_matvecs += apply_cols(F, Vk, w, G, scs, true, r32, re32, cyc.data(), opt.compact, s);
         st.matvecs++;
         HessArgs ha{H_.as<double2>(), g_.as<double2>(), cs_.as<double>(), sn_.as<double2>(), bs, opt.tol, nullptr,
-                    opt.maxiter, restart, nu, rnorm_.as<double>(), dflag};
+                    opt.maxiter, restart, nu, rnorm_.as<double>(), dflag, poll_words(G), ++poll_seq_};
         arnoldi(V, k, rows, G, sst, ha, MemberArgs{mst, dsig, dgrp, M, tolv, scyc}, s);
         st.reorth_steps++;
-        const int left = read_flags(dflag, G, s);
+        const int left = wait_flags(s);
         if (left == 0) break;
-        cyc.assign(flag_ + 1, flag_ + 1 + G);
+        cyc.assign(poll_.as<int>() + 2, poll_.as<int>() + 2 + G);
     }
     backsub(mst, H_.as<double2>(), g_.as<double2>(), y_.as<double2>(), restart, M, kper, s);
     k_shift_x<<<nblk((long long)rows * M, 256), 256, 0, s>>>(x, V, ns, G, y_.as<double2>(), dgrp, kper, skip, rows,

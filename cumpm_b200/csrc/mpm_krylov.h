@@ -126,6 +126,11 @@ private:
     DevBuf shf_, shflag_, shmeta_, shsc_, shb_, shst_;   // shifted solve: detection, seeds, members
     HostBuf flagbuf_, hidx_;             // count + per-column flags; column list for the gather
     int* flag_ = nullptr;                // the words of flagbuf_
+    // flags of the latest Arnoldi step: sequence number, count, column flags
+    HostBuf poll_;
+    int poll_seq_ = 0;
+    int* poll_words(int M);
+    int wait_flags(cudaStream_t s);
     std::vector<int> cur_cols_;          // column list the device buffers hold
     const double2* cur_sc_ = nullptr;    // self coefficients gathered into scc_
 };
