@@ -1543,7 +1543,7 @@ __global__ void __launch_bounds__(128) k_real(const double2* __restrict__ X, dou
 // where the columns are many, by the chain of a thread's sources where the
 // system is small: hence few targets per CTA there.  One thread per target
 // and column, each with its own geometry, took 1150 us for N = 2000 with 30
-// columns in fp64 (416 here) and 27 us for N = 100 with 3 in fp32
+// columns in fp64 (344 here) and 27 us for N = 100 with 3 in fp32
 // (8 us).
 constexpr int kDirectTile = 64;    // sources staged at a time
 

@@ -79,10 +79,16 @@ private:
     std::vector<cdouble> guess(const std::vector<cdouble>& fd, const std::vector<cdouble>& fq, size_t w) const;
     void solve_batch(const std::vector<size_t>& freqs, const std::vector<std::vector<cdouble>>& guesses,
                      std::vector<cdouble>& frame_cap, std::vector<cdouble>& frame_dip, std::vector<cdouble>& frame_quad);
-    // batch_all with dipoles and uniform incident fields: the mean-field
-    // guesses of frequencies 1..W-1 (and frequency 0's, from init) are built
-    // on the device and the solution is written into the frame layout there
-    bool device_batch_ok() const;
+    // dipoles and uniform incident fields: guesses, right-hand sides and self
+    // coefficients are built on the device and the solutions are put into the
+    // frame layout there, all frequencies as one batch (batch_all) or one
+    // after another
+    bool device_ok() const;
+    void upload_inputs();
+    SolveOptions solve_options() const;
+    void sweep_device(const std::vector<cdouble>& init, std::vector<cdouble>& frame_cap,
+                      std::vector<cdouble>& frame_dip);
+    void average(std::vector<cdouble>& frame_cap, const std::vector<cdouble>& frame_dip) const;
     void solve_all_device(const std::vector<cdouble>& init, std::vector<cdouble>& frame_cap,
                           std::vector<cdouble>& frame_dip);
     void print(const std::string& msg) const;
