@@ -453,6 +453,7 @@ __global__ void __launch_bounds__(256) k_spread_planned(const double2* __restric
     const int nb = min(bc, B - b0);
     const R* wTt = wT + trow * wlen;
     for (int t = threadIdx.x; t < ncol; t += blockDim.x) lnS[t] = lnT[size_t(tile) * ncol + t];
+#pragma unroll 4
     for (int t = threadIdx.x; t < nc * TZ; t += blockDim.x) {
         const int c = t / TZ;
         wz[t] = wTt[size_t(c) * wlen + TX + TY + (t - c * TZ)];
@@ -1575,17 +1576,31 @@ __global__ void __launch_bounds__(128) k_direct(const double2* __restrict__ X, d
     for (int t0 = 0; t0 < N; t0 += kDirectTile) {
         const int te = min(kDirectTile, N - t0);
         __syncthreads();
-        for (int t = threadIdx.x; t < te * 3 * CB; t += 128) {
+        // (fixed trip counts: all loads of a tile in flight together)
+        constexpr int kLoads = (kDirectTile * 3 * CB + 127) / 128;
+        double2 v[kLoads];
+#pragma unroll
+        for (int l = 0; l < kLoads; ++l) {
+            const int t = threadIdx.x + l * 128;
             const int b = t % CB, row = t / CB;                    // row = 3 source + component
-            sp[t] = b < mc ? to_r<R>(X[(size_t(3) * t0 + row) * M + m0 + b]) : mk<R>(R(0), R(0));
+            v[l] = b < mc && row < 3 * te ? X[(size_t(3) * t0 + row) * M + m0 + b] : make_double2(0.0, 0.0);
         }
-        for (int t = threadIdx.x; t < 4 * te; t += 128) {
-            const int c = t / te, i = t - c * te;
-            if (c < 3) sx[c * kDirectTile + i] = R(src[size_t(c) * N + t0 + i]);
-            else {
-                const R a = rad ? R(rad[t0 + i]) : R(0);
-                sx[c * kDirectTile + i] = a * a;
-            }
+        double g[4 * kDirectTile / 128];
+#pragma unroll
+        for (int l = 0; l < 4 * kDirectTile / 128; ++l) {
+            const int t = threadIdx.x + l * 128, c = t / kDirectTile, i = t - c * kDirectTile;
+            g[l] = i >= te ? 0.0 : c < 3 ? src[size_t(c) * N + t0 + i] : rad ? rad[t0 + i] : 0.0;
+        }
+#pragma unroll
+        for (int l = 0; l < kLoads; ++l) {
+            const int t = threadIdx.x + l * 128;
+            if (t < kDirectTile * 3 * CB) sp[t] = to_r<R>(v[l]);
+        }
+#pragma unroll
+        for (int l = 0; l < 4 * kDirectTile / 128; ++l) {
+            const int t = threadIdx.x + l * 128;
+            const R a = R(g[l]);
+            sx[t] = t < 3 * kDirectTile ? a : a * a;
         }
         __syncthreads();
         if (!live) continue;
@@ -2491,8 +2506,9 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
                                                spec_.solver_ax ? sources_.idx_sorted.as<int>() : nullptr, ov ? 1 : 0,
                                                ov ? ov->jacobi_sc : nullptr);
         };
-        // four warps per target below 16 warps per SM in all
-        const bool one = nt >= 16 * 148;
+        // four warps per target below 16 warps per SM in all (64 for one slot,
+        // where a lane then has all its loads in flight at once)
+        const bool one = nt >= (gv_.Sz == 1 ? 64 : 16) * 148;
         if (gv_.Sz == 1) one ? few(k_contract_few<R, 1, 1>, 4) : few(k_contract_few<R, 1, 4>, 1);
         else if (gv_.Sz <= 9) one ? few(k_contract_few<R, 9, 1>, 4) : few(k_contract_few<R, 9, 4>, 1);
         else one ? few(k_contract_few<R, 13, 1>, 4) : few(k_contract_few<R, 13, 4>, 1);
