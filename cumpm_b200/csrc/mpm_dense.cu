@@ -149,7 +149,9 @@ __device__ __forceinline__ void line_of(long long f, long long ntot, int ncols, 
 }
 
 // TS: the tables are staged in shared memory once per CTA, which then stays
-// for several tiles.  ONE: r1 = 1.  A tile is copied in with all its loads in
+// for several tiles.  KIND 0: r1 = 1; 1: r1 > 1; 2: m is an in-register radix
+// too, and takes the product's place (84 = 12 * 7 points of 9 columns, 43 MB:
+// 38 us with the product, 21).  A tile is copied in with all its loads in
 // flight (cp.async; loads of four at a time spent two thirds of the kernel
 // waiting), transformed in place by the radix pass, and read by the product
 // whose outputs go straight to global memory; the SM's other CTAs compute
@@ -158,7 +160,7 @@ __device__ __forceinline__ void line_of(long long f, long long ntot, int ncols, 
 // of 497 MB.  Forward, scale and inverse in one launch needs the outputs of a
 // whole tile in registers or a second tile: 2010 us at 109 points where two
 // launches take 1245.)
-template <typename R, bool SCALED, bool TS, bool ONE>
+template <typename R, bool SCALED, bool TS, int KIND>
 __global__ void __launch_bounds__(kDenseMaxThreads, 2) k_dense(DenseArgs<R> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int CW = 1 << a.cwl;
@@ -170,12 +172,12 @@ __global__ void __launch_bounds__(kDenseMaxThreads, 2) k_dense(DenseArgs<R> a) {
     constexpr int CT = dense_ct<R>();
     const int half = CW / CT;
     const bool inv = a.inv != 0;
-    if (TS) {
+    if (TS && KIND != 2) {
         const int nt = imax(1, a.H) * 2 * a.ld * int(sizeof(R)) / 16;
         const double2* g = reinterpret_cast<const double2*>(a.tab);
         for (int t = threadIdx.x; t < nt; t += blockDim.x) copy_async<double>(reinterpret_cast<double2*>(tabS) + t, g + t, true);
     }
-    if (!ONE)
+    if (KIND != 0)
         for (int t = threadIdx.x; t < a.n; t += blockDim.x) copy_async<R>(T + t, a.tw + t, true);
     const R* tab = TS ? tabS : a.tab;
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
@@ -190,7 +192,7 @@ __global__ void __launch_bounds__(kDenseMaxThreads, 2) k_dense(DenseArgs<R> a) {
         }
         copy_async_wait();
         __syncthreads();
-        if constexpr (!ONE) {
+        if constexpr (KIND != 0) {
             // radix-r1 butterflies over x[j + q m], times W_n^(j p), in place: S[p][j]
             radix_dispatch<16>(a.r1, [&](auto rc) {
                 constexpr int RAD = decltype(rc)::value;
@@ -213,25 +215,49 @@ __global__ void __launch_bounds__(kDenseMaxThreads, 2) k_dense(DenseArgs<R> a) {
             });
             __syncthreads();
         }
-        // the columns of this thread's work items
-        cplx<R>* oline[CT];
-        bool olive[CT];
-        const R* osc[CT];
+        if constexpr (KIND == 2) {
+            // radix-m butterflies over S[p1][j]: outputs p1 + r1 p (mirrored for the inverse)
+            const bool live = f0 + c < a.ntot;
+            int o = 0, cc = 0;
+            if (live) line_of(f0 + c, a.ntot, a.ncols, o, cc);
+            cplx<R>* line = a.data + size_t(o) * a.os + cc;
+            const R* sc = SCALED ? a.sc + size_t(o) * a.sz + cc / a.sb : nullptr;
+            if (live)
+                radix_dispatch<16>(a.m, [&](auto rc) {
+                    constexpr int RAD = decltype(rc)::value;
+                    for (int p1 = lane; p1 < a.r1; p1 += lanes) {
+                        cplx<R> x[RAD];
 #pragma unroll
-        for (int t = 0; t < CT; ++t) {
-            const long long g = f0 + (threadIdx.x & (half - 1)) + t * half;
-            olive[t] = g < a.ntot;
-            int go = 0, gc = 0;
-            if (olive[t]) line_of(g, a.ntot, a.ncols, go, gc);
-            oline[t] = a.data + size_t(go) * a.os + gc;
-            osc[t] = SCALED ? a.sc + size_t(go) * a.sz + gc / a.sb : nullptr;
+                        for (int q = 0; q < RAD; ++q) x[q] = S[(p1 * RAD + q) * CW + c];
+                        dft_small<R, false, RAD>(x);
+#pragma unroll
+                        for (int k = 0; k < RAD; ++k) {
+                            const int e = p1 + a.r1 * (inv && k ? RAD - k : k);
+                            line[size_t(e) * a.es] = SCALED ? x[k] * sc[size_t(e) * a.estep] : x[k];
+                        }
+                    }
+                });
+        } else {
+            // the columns of this thread's work items
+            cplx<R>* oline[CT];
+            bool olive[CT];
+            const R* osc[CT];
+#pragma unroll
+            for (int t = 0; t < CT; ++t) {
+                const long long g = f0 + (threadIdx.x & (half - 1)) + t * half;
+                olive[t] = g < a.ntot;
+                int go = 0, gc = 0;
+                if (olive[t]) line_of(g, a.ntot, a.ncols, go, gc);
+                oline[t] = a.data + size_t(go) * a.os + gc;
+                osc[t] = SCALED ? a.sc + size_t(go) * a.sz + gc / a.sb : nullptr;
+            }
+            dense_pass<R>(S, a, tab, inv, [&](int t, int p1, int p, cplx<R> v) {
+                if (!olive[t]) return;
+                const int e = p1 + a.r1 * p;
+                if constexpr (SCALED) v = v * osc[t][size_t(e) * a.estep];
+                oline[t][size_t(e) * a.es] = v;
+            });
         }
-        dense_pass<R>(S, a, tab, inv, [&](int t, int p1, int p, cplx<R> v) {
-            if (!olive[t]) return;
-            const int e = p1 + a.r1 * p;
-            if constexpr (SCALED) v = v * osc[t][size_t(e) * a.estep];
-            oline[t][size_t(e) * a.es] = v;
-        });
         __syncthreads();   // the tile's buffer is free
     }
 }
@@ -310,7 +336,8 @@ void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, si
     const size_t tabb = sizeof(R) * size_t(std::max(1, H_)) * 2 * ld_;
     const size_t twb = r1_ > 1 ? sizeof(cplx<R>) * size_t(n_) : 0;
     const size_t per_col = size_t(n_) * sizeof(cplx<R>);
-    const bool ts = tabb <= kDenseTableSmem && (per_col << 2) + tabb + twb <= kDenseSmemMax;
+    const bool radix2 = r1_ > 1 && m_ <= 16;       // no table
+    const bool ts = !radix2 && tabb <= kDenseTableSmem && (per_col << 2) + tabb + twb <= kDenseSmemMax;
     auto smem = [&](int cwl) { return (per_col << cwl) + (ts ? tabb : 0) + twb; };
     auto items = [&](int cwl) { return a.r1 * a.nch * ((1 << cwl) / CT); };
     // columns per tile: 64 (fp64: 32), so that a warp's lanes are the columns
@@ -324,7 +351,7 @@ void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, si
     a.cwl = cwl;
     a.ntiles = int((a.ntot + (1ll << cwl) - 1) >> cwl);
     // threads: the work items in equal rounds, a whole number of column rows
-    const int it = items(cwl), rounds = (it + kDenseMaxThreads - 1) / kDenseMaxThreads;
+    const int it = radix2 ? r1_ << cwl : items(cwl), rounds = (it + kDenseMaxThreads - 1) / kDenseMaxThreads;
     const int unit = std::max(32, 1 << cwl);
     int nt = ((it + rounds - 1) / rounds + unit - 1) / unit * unit;
     nt = std::min(kDenseMaxThreads, std::max(nt, 128));   // the copies and radix pass use them all
@@ -335,13 +362,14 @@ void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, si
         set_smem_limit(kern, shm);
         kern<<<grid, nt, shm, s>>>(a);
     };
-    auto pick = [&](auto scaled, auto one) {
-        constexpr bool SC = decltype(scaled)::value, ONE = decltype(one)::value;
-        if (ts) go(k_dense<R, SC, true, ONE>);
-        else go(k_dense<R, SC, false, ONE>);
+    auto pick = [&](auto scaled) {
+        constexpr bool SC = decltype(scaled)::value;
+        if (radix2) go(k_dense<R, SC, false, 2>);
+        else if (r1_ == 1) ts ? go(k_dense<R, SC, true, 0>) : go(k_dense<R, SC, false, 0>);
+        else ts ? go(k_dense<R, SC, true, 1>) : go(k_dense<R, SC, false, 1>);
     };
-    if (scale) r1_ == 1 ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{});
-    else r1_ == 1 ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{});
+    if (scale) pick(std::true_type{});
+    else pick(std::false_type{});
     MPM_LAUNCH();
 }
 
