@@ -203,7 +203,8 @@ __global__ void k_poly_cands(PolyTile t, const int* __restrict__ bin_start, cons
 // per ballot (a thread per tile walked its list alone: 421 us for 125 tiles
 // of 80 candidates).
 __global__ void k_poly_filter(PolyTile t, const int4* __restrict__ base, const int* __restrict__ off,
-                              const int* __restrict__ list, int* __restrict__ cnt, int* __restrict__ clist) {
+                              const int* __restrict__ list, int* __restrict__ cnt, int* __restrict__ clist,
+                              int* __restrict__ maxc) {
     const int tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const int ntile = t.nb[0] * t.nb[1] * t.nb[2];
@@ -229,7 +230,10 @@ __global__ void k_poly_filter(PolyTile t, const int4* __restrict__ base, const i
         if (all) clist[c0 + kept + __popc(hit & ((1u << lane) - 1u))] = i;
         kept += __popc(hit);
     }
-    if (lane == 0) cnt[tile] = kept;
+    if (lane == 0) {
+        cnt[tile] = kept;
+        atomicMax(maxc, kept);
+    }
 }
 
 // Spread onto one 8^3 voxel tile x CM consecutive columns per CTA, every
@@ -281,6 +285,7 @@ __global__ void __launch_bounds__(256) k_poly_spread(const double2* __restrict__
     const int nc = min(tcnt[tile], t.cap);
     const int P = t.P;
     const size_t P3 = size_t(P) * P * P;
+#pragma unroll 4
     for (int q = threadIdx.x; q < nc * 24; q += 256) {
         const int c = q / 24, r = q - c * 24, d = r >> 3, u = r & 7;
         const int i = clist[c0 + c];
@@ -291,6 +296,7 @@ __global__ void __launch_bounds__(256) k_poly_spread(const double2* __restrict__
         sup[q] = short(poly_support(tt + u, org, N, P));
         if (r == 0) cand[c] = i;
     }
+#pragma unroll 4
     for (int k = threadIdx.x; k < nc * 3 * CM; k += 256) {
         const int cm = k % CM, comp = (k / CM) % 3, c = k / (3 * CM);
         const int m = m0 + cm;
@@ -843,12 +849,18 @@ void Field::poly_weights(PointSet& ps, const double* radius_dev, cudaStream_t s,
     MPM_LAUNCH();
     ptcnt_.ensure(sizeof(int) * std::max(1, nbins));
     ptclist_.ensure(sizeof(int) * std::max(1, hv[1]));
+    MPM_CUDA(cudaMemsetAsync(ptmax_.p, 0, sizeof(int), s));
     k_poly_filter<<<nblk((long long)nbins * 32, 128), 128, 0, s>>>(t, ps.base.as<int4>(), ptoff_.as<int>(),
                                                                    ptlist_.as<int>(), ptcnt_.as<int>(),
-                                                                   ptclist_.as<int>());
+                                                                   ptclist_.as<int>(), ptmax_.as<int>());
     MPM_LAUNCH();
-    pcand_cap_ = std::max(1, h);
-    const size_t shm = 65536 + (3 * 128 + 9 * sizeof(int)) * size_t(pcand_cap_);
+    // the spread's shared memory holds the candidates that are left (the limit
+    // on a frame is that of the unfiltered lists)
+    int kept = 0;
+    MPM_CUDA(cudaMemcpyAsync(&kept, ptmax_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MPM_CUDA(cudaStreamSynchronize(s));
+    pcand_cap_ = std::max(1, kept);
+    const size_t shm = 65536 + (3 * 128 + 9 * sizeof(int)) * size_t(std::max(1, h));
     if (shm > 200 * 1024 || pgeom_.P > 255)
         throw std::runtime_error("polydisperse spread: " + std::to_string(h) +
                                  " particles reach one 8^3 voxel tile, more than the shared candidate list holds");
