@@ -102,7 +102,7 @@ __device__ __forceinline__ void reduce_partials(const double2* __restrict__ part
         const int o = o0 + g;
         double2 sum = make_double2(0, 0);
         if (o < n) {
-#pragma unroll 4
+#pragma unroll 8
             for (int b = sl; b < gx; b += 8) sum += __ldcg(&partial[size_t(b) * n + o]);
         }
         for (int off = 4; off > 0; off >>= 1) {
@@ -673,9 +673,19 @@ __global__ void __launch_bounds__(256) k_arn_project(double2* __restrict__ V, si
         cta_column_sums(acc, nv, M, L, red, partial + (size_t(blockIdx.x) * nvec + i0) * M);
     }
     if (!last_cta(done, gridDim.x)) return;
-    reduce_partials(partial, gridDim.x, nvec * M, h2);
+    // the finish on copies of h and h2 in shared memory (when they fit): it is
+    // a chain of dependent reads by a few threads
+    const int n2 = nvec * M;
+    const bool fits = 2 * n2 <= 8 * 256;
+    double2* hs = fits ? &red[0][0] : h;
+    double2* h2s = fits ? hs + n2 : h2;
+    reduce_partials(partial, gridDim.x, n2, h2s);
+    if (fits)
+        for (int t = j; t < n2 - M; t += 256) hs[t] = h[t];
     __syncthreads();
-    finish2_body(st, h, h2, a, mb, k, M);
+    if (fits)
+        for (int t = j; t < n2; t += 256) h2[t] = h2s[t];      // for k_arn_update
+    finish2_body(st, hs, h2s, a, mb, k, M);
 }
 
 // member states: active and cycling from the start, x0 = 0; g_m = (beta, 0..);

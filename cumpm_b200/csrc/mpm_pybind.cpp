@@ -181,16 +181,26 @@ public:
     }
     std::vector<double> calculate() {
         std::vector<double> out(nfp_);
-        int st;
-        {
-            py::gil_scoped_release nogil;
-            st = mpm_near_calculate(n_, out.data(), int(out.size()));
-        }
-        check(st);
+        fill(out.data(), out.size());
+        return out;
+    }
+    // the same as an array: a list of 10000 values and its conversion cost as
+    // much as the field itself
+    py::array_t<double> calculate_array() {
+        py::array_t<double> out{py::ssize_t(nfp_)};
+        fill(out.mutable_data(), nfp_);
         return out;
     }
 
 private:
+    void fill(double* out, size_t n) {
+        int st;
+        {
+            py::gil_scoped_release nogil;
+            st = mpm_near_calculate(n_, out, int(n));
+        }
+        check(st);
+    }
     mpm_near* n_ = nullptr;
     size_t npos_ = 0, nfp_ = 0;
 };
@@ -268,5 +278,6 @@ PYBIND11_MODULE(_cuMPM, m) {
         .def("set_dipoles", &PyNearField::set_dipoles, py::arg("dip"))
         .def("set_dipole_positions", &PyNearField::set_dipole_positions, py::arg("x"), py::arg("y"), py::arg("z"))
         .def("set_field_points", &PyNearField::set_field_points, py::arg("x"), py::arg("y"), py::arg("z"))
-        .def("calculate", &PyNearField::calculate);
+        .def("calculate", &PyNearField::calculate)
+        .def("calculate_array", &PyNearField::calculate_array);
 }

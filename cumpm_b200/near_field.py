@@ -49,4 +49,4 @@ class Near_Field:
         self._near_field.set_field_points(p[:, 0].tolist(), p[:, 1].tolist(), p[:, 2].tolist())
 
     def calculate(self):
-        return np.array(self._near_field.calculate())
+        return self._near_field.calculate_array()
