@@ -151,7 +151,7 @@ __device__ __forceinline__ void line_of(long long f, long long ntot, int ncols, 
 // TS: the tables are staged in shared memory once per CTA, which then stays
 // for several tiles.  KIND 0: r1 = 1; 1: r1 > 1; 2: m is an in-register radix
 // too, and takes the product's place (84 = 12 * 7 points of 9 columns, 43 MB:
-// 38 us with the product, 21).  A tile is copied in with all its loads in
+// 38 us with the product, 30).  A tile is copied in with all its loads in
 // flight (cp.async; loads of four at a time spent two thirds of the kernel
 // waiting), transformed in place by the radix pass, and read by the product
 // whose outputs go straight to global memory; the SM's other CTAs compute

@@ -1397,10 +1397,12 @@ __global__ void __launch_bounds__(128) k_real(const double2* __restrict__ X, dou
     const double sign = (a.solver_ax || a.pairs_plus) ? 1.0 : -1.0;
     const double selfc = selfv ? selfv[j] : a.selfo;  // polydisperse: self value of the particle's radius class
     const int qt = (QUADS && quad_map && j < a.N) ? quad_map[j] : -1;
-    // fewer than 32 columns: the warp splits into 32 / gsz groups of gsz lanes (gsz = M rounded up to a power of two); group g
-    // takes pairs p0 + g, p0 + g + 32/gsz, ... and the groups' sums meet in a
-    // fixed shuffle tree
-    const int gsz = M < 32 ? (M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16) : 32;
+    // few columns: the warp splits into 32 / gsz groups of gsz lanes (gsz = M
+    // rounded up to a power of two); group g takes pairs p0 + g, p0 + g +
+    // 32/gsz, ... and the groups' sums meet in a fixed shuffle tree.  With
+    // quadrupoles every M above four takes two groups, so that a column's sum
+    // has the same order in a sweep's blocks as in the whole sweep.
+    const int gsz = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : QUADS ? 16 : M <= 8 ? 8 : M < 32 ? 16 : 32;
     const int ng = 32 / gsz, grp = lane / gsz;
     for (int m0 = 0; m0 < M; m0 += gsz) {
         const int m = m0 + lane % gsz;
