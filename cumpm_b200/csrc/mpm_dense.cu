@@ -35,6 +35,9 @@ namespace {
 
 constexpr int kDenseMaxThreads = 256;
 constexpr int kPC = 8;    // output pairs per thread
+// CTAs per SM that the registers allow: the product's accumulators take 128 a
+// thread, two fp32 butterflies half of them
+template <typename R> __host__ __device__ constexpr int dense_ctas(bool radix2) { return radix2 && sizeof(R) == 4 ? 4 : 2; }
 
 template <typename R> constexpr int dense_ct() { return sizeof(R) == 4 ? 2 : 1; }   // columns per thread
 
@@ -151,7 +154,7 @@ __device__ __forceinline__ void line_of(long long f, long long ntot, int ncols, 
 // TS: the tables are staged in shared memory once per CTA, which then stays
 // for several tiles.  KIND 0: r1 = 1; 1: r1 > 1; 2: m is an in-register radix
 // too, and takes the product's place (84 = 12 * 7 points of 9 columns, 43 MB:
-// 38 us with the product, 30).  A tile is copied in with all its loads in
+// 38 us with the product, 26).  A tile is copied in with all its loads in
 // flight (cp.async; loads of four at a time spent two thirds of the kernel
 // waiting), transformed in place by the radix pass, and read by the product
 // whose outputs go straight to global memory; the SM's other CTAs compute
@@ -161,7 +164,7 @@ __device__ __forceinline__ void line_of(long long f, long long ntot, int ncols, 
 // whole tile in registers or a second tile: 2010 us at 109 points where two
 // launches take 1245.)
 template <typename R, bool SCALED, bool TS, int KIND>
-__global__ void __launch_bounds__(kDenseMaxThreads, 2) k_dense(DenseArgs<R> a) {
+__global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_dense(DenseArgs<R> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int CW = 1 << a.cwl;
     cplx<R>* S = reinterpret_cast<cplx<R>*>(smem_raw);                   // [n][CW]
@@ -345,7 +348,8 @@ void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, si
     // SM would not hold two CTAs, whose copies and products overlap, or the
     // tiles would not cover two per SM (few columns in all)
     int cwl = sizeof(R) == 4 ? 6 : 5;
-    while (cwl > 2 && (smem(cwl) > 112 * 1024 || (a.ntot >> cwl) < 2 * sm_count())) --cwl;
+    const int regs = 256 / dense_ctas<R>(radix2);
+    while (cwl > 2 && (smem(cwl) > size_t(224 * 1024 / dense_ctas<R>(radix2)) || (a.ntot >> cwl) < 2 * sm_count())) --cwl;
     const size_t shm = smem(cwl);
     if (shm > kDenseSmemMax) throw std::runtime_error("FFT line does not fit in shared memory");
     a.cwl = cwl;
@@ -355,8 +359,8 @@ void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, si
     const int unit = std::max(32, 1 << cwl);
     int nt = ((it + rounds - 1) / rounds + unit - 1) / unit * unit;
     nt = std::min(kDenseMaxThreads, std::max(nt, 128));   // the copies and radix pass use them all
-    // resident CTAs (128 registers a thread); each stays for its share of the tiles
-    const int per_sm = std::max(1, std::min({int(227 * 1024 / (shm + 1024)), 65536 / (128 * nt), 16}));
+    // resident CTAs; each stays for its share of the tiles
+    const int per_sm = std::max(1, std::min({int(227 * 1024 / (shm + 1024)), 65536 / (regs * nt), 16}));
     const int grid = std::min(a.ntiles, per_sm * sm_count());
     auto go = [&](auto kern) {
         set_smem_limit(kern, shm);

@@ -420,13 +420,24 @@ __global__ void __launch_bounds__(256) k_spread_plan(const int4* __restrict__ ba
 // a multiple of four; -1 marks a list that overflowed)
 __device__ __forceinline__ int list_padded(int n) { return n > 0 ? (n + 3) & ~3 : 0; }
 
+// four consecutive values from a 16-byte boundary of shared memory
+__device__ __forceinline__ void load4(const float* p, float* o) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+}
+__device__ __forceinline__ void load4(const double* p, double* o) {
+    const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
+}
+
 // Spread with the per-frame plan: CTA = one tile x one chunk of bc grid
 // columns; stages the tile's candidate moments and z weights and every (x, y)
 // column's contributor list in shared memory, then thread = one (x, y) column
 // x one grid column with the whole z run in registers.  The same contributors
 // in the same order as k_spread.  With the lists and weights read from global
 // memory in the loop it waited on one dependent load after another: 119 us
-// for 8000 particles, 84^3 voxels and 9 columns, 90 here.
+// for 8000 particles, 84^3 voxels and 9 columns, 65 here (91 with the lists and
+// z weights read from shared memory word by word).
 template <typename R, int ZMAX>
 __global__ void __launch_bounds__(256) k_spread_planned(const double2* __restrict__ X, int M, int N, int C,
                                                         const int* __restrict__ quad_map, GridView g, int TX,
@@ -437,11 +448,15 @@ __global__ void __launch_bounds__(256) k_spread_planned(const double2* __restric
                                                         cplx<R>* __restrict__ grid) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int ncol = TX * TY;
-    cplx<R>* pv = reinterpret_cast<cplx<R>*>(smem_raw);                  // [capT][bc]
-    R* wz = reinterpret_cast<R*>(pv + size_t(capT) * bc);                 // [capT][TZ]
-    R* lwS = wz + size_t(capT) * TZ;                                      // [ncol][kSpreadListCap]
+    R* lwS = reinterpret_cast<R*>(smem_raw);                              // [ncol][kSpreadListCap]
     int* lcS = reinterpret_cast<int*>(lwS + size_t(ncol) * kSpreadListCap);
-    int* lnS = lcS + size_t(ncol) * kSpreadListCap;                        // [ncol]
+    // [capT][bc] moments and [capT][TZ] z weights; rows of eight weights come
+    // first and are then 16-byte aligned
+    unsigned char* rest = reinterpret_cast<unsigned char*>(lcS + size_t(ncol) * kSpreadListCap);
+    const size_t wzb = sizeof(R) * size_t(capT) * TZ, pvb = sizeof(cplx<R>) * size_t(capT) * bc;
+    R* wz = reinterpret_cast<R*>(rest + (ZMAX == 8 ? 0 : pvb));
+    cplx<R>* pv = reinterpret_cast<cplx<R>*>(rest + (ZMAX == 8 ? wzb : 0));
+    int* lnS = reinterpret_cast<int*>(rest + wzb + pvb);                  // [ncol]
     const int zt = blockIdx.z % nzt, chunk = blockIdx.z / nzt;
     const int tile = (zt * nby + blockIdx.y) * nbx + blockIdx.x;
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = zt * TZ;
@@ -520,20 +535,27 @@ __global__ void __launch_bounds__(256) k_spread_planned(const double2* __restric
             const int* lc = lcS + col * kSpreadListCap;
             const R* lw = lwS + col * kSpreadListCap;
             for (int k = 0; k < nl; k += 4) {
-                int c[4];
+                const int4 c4 = *reinterpret_cast<const int4*>(lc + k);
+                const int c[4] = {c4.x, c4.y, c4.z, c4.w};
+                R wxy[4];
+                load4(lw + k, wxy);
                 cplx<R> v[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    c[u] = lc[k + u];
-                    v[u] = pv[c[u] * bc + bb];
-                }
+                for (int u = 0; u < 4; ++u) v[u] = pv[c[u] * bc + bb] * wxy[u];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const R wxy = lw[k + u];
                     const R* wzc = wz + c[u] * TZ;
+                    if constexpr (ZMAX == 8) {
+                        R w[8];
+                        load4(wz + c[u] * 8, w);
+                        load4(wz + c[u] * 8 + 4, w + 4);
 #pragma unroll
-                    for (int lz = 0; lz < ZMAX; ++lz)
-                        if (lz < TZ) fma_rc(acc[lz], wxy * wzc[lz], v[u]);
+                        for (int lz = 0; lz < ZMAX; ++lz) fma_rc(acc[lz], w[lz], v[u]);
+                    } else {
+#pragma unroll
+                        for (int lz = 0; lz < ZMAX; ++lz)
+                            if (lz < TZ) fma_rc(acc[lz], wzc[lz], v[u]);
+                    }
                 }
             }
         } else {   // list overflowed: every candidate, in order
@@ -576,10 +598,10 @@ __global__ void __launch_bounds__(256) k_spread_planned_1z(const double2* __rest
                                                            cplx<R>* __restrict__ grid) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int ncol = TX * TY;
-    cplx<R>* pv = reinterpret_cast<cplx<R>*>(smem_raw);             // [capT][bc]
-    R* lwS = reinterpret_cast<R*>(pv + size_t(capT) * bc);           // [ncol][kSpreadListCap]
+    R* lwS = reinterpret_cast<R*>(smem_raw);                          // [ncol][kSpreadListCap]
     int* lcS = reinterpret_cast<int*>(lwS + size_t(ncol) * kSpreadListCap);
-    int* lnS = lcS + size_t(ncol) * kSpreadListCap;                   // [ncol]
+    cplx<R>* pv = reinterpret_cast<cplx<R>*>(lcS + size_t(ncol) * kSpreadListCap);   // [capT][bc]
+    int* lnS = reinterpret_cast<int*>(pv + size_t(capT) * bc);        // [ncol]
     const int chunk = blockIdx.z;
     const int tile = blockIdx.y * nbx + blockIdx.x;
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
@@ -652,11 +674,15 @@ __global__ void __launch_bounds__(256) k_spread_planned_1z(const double2* __rest
             cplx<R> acc = mk<R>(0, 0);
             if (nl >= 0) {
                 for (int k = 0; k < nl; k += 4) {
+                    const int4 c4 = *reinterpret_cast<const int4*>(lc + k);
+                    const int c[4] = {c4.x, c4.y, c4.z, c4.w};
+                    R w[4];
+                    load4(lw + k, w);
                     cplx<R> v[4];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) v[u] = pv[lc[k + u] * bc + bb];
+                    for (int u = 0; u < 4; ++u) v[u] = pv[c[u] * bc + bb];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) fma_rc(acc, lw[k + u], v[u]);
+                    for (int u = 0; u < 4; ++u) fma_rc(acc, w[u], v[u]);
                 }
             } else {   // list overflowed: every candidate, in order
                 for (int c = 0; c < nc; ++c) {
@@ -2420,6 +2446,7 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
                                                           plan_cid_.as<int>(), wT, lw, plan_lc_.as<int>(),
                                                           plan_ln_.as<int>(), grid);
         }
+        else if (TZ == 8) go(k_spread_planned<R, 8>);
         else if (TZ <= 9) go(k_spread_planned<R, 9>);
         else go(k_spread_planned<R, kSpreadZMax>);
     } else {
