@@ -23,6 +23,7 @@
 // column), so a transform of few columns per line (the z axis of a solve's
 // three right-hand sides) still fills its tiles.
 #include "mpm_butterfly.cuh"
+#include "mpm_chain.cuh"
 #include "mpm_fft.h"
 
 #include <algorithm>
@@ -175,6 +176,7 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
     constexpr int CT = dense_ct<R>();
     const int half = CW / CT;
     const bool inv = a.inv != 0;
+    // (the tables are older than any launch of this stream)
     if (TS && KIND != 2) {
         const int nt = imax(1, a.H) * 2 * a.ld * int(sizeof(R)) / 16;
         const double2* g = reinterpret_cast<const double2*>(a.tab);
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
     if (KIND != 0)
         for (int t = threadIdx.x; t < a.n; t += blockDim.x) copy_async<R>(T + t, a.tw + t, true);
     const R* tab = TS ? tabS : a.tab;
+    chain_wait();
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
         const long long f0 = (long long)tile << a.cwl;
         {
@@ -193,6 +196,9 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
             const size_t es = live ? a.es : 0;
             for (int e = lane; e < a.n; e += lanes) copy_async<R>(S + e * CW + c, line + size_t(e) * es, live);
         }
+        // a successor that is scheduled earlier takes slots from work on other
+        // streams for as long as this CTA's tiles last
+        if (tile + gridDim.x >= a.ntiles) chain_release();
         copy_async_wait();
         __syncthreads();
         if constexpr (KIND != 0) {
@@ -364,7 +370,7 @@ void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, si
     const int grid = std::min(a.ntiles, per_sm * sm_count());
     auto go = [&](auto kern) {
         set_smem_limit(kern, shm);
-        kern<<<grid, nt, shm, s>>>(a);
+        launch_chained(kern, grid, nt, shm, s, a);
     };
     auto pick = [&](auto scaled) {
         constexpr bool SC = decltype(scaled)::value;
@@ -374,7 +380,6 @@ void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, si
     };
     if (scale) pick(std::true_type{});
     else pick(std::false_type{});
-    MPM_LAUNCH();
 }
 
 template void DenseDFT::run<float>(float2*, const float2*, size_t, int, size_t, int, int, const float*, int, int,

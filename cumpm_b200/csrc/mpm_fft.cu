@@ -1,6 +1,7 @@
 // Batched in-place 1-D DFT along a strided axis (see mpm_fft.h).
 #include "mpm_fft.h"
 #include "mpm_butterfly.cuh"
+#include "mpm_chain.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -316,6 +317,7 @@ template <typename R, int CW, int MODE, int CLS>
 __global__ void __launch_bounds__(kFft2MaxThreads) k_fft2(cplx<R>* __restrict__ data, const cplx<R>* __restrict__ tw,
                                                           int r1, int r2, size_t es, int ncols, size_t os,
                                                           int ngroups, LineScale<R> ks) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr bool INV = MODE == 1;
     const int n = r1 * r2;
@@ -436,7 +438,7 @@ void launch2_cw(int cls, int nblocks, int nthreads, size_t shm, cudaStream_t s, 
                 int r1, int r2, size_t es, int ncols, size_t os, int ngroups, const LineScale<R>& ks) {
     auto go = [&](auto kern) {
         set_smem_limit(kern, shm);
-        kern<<<nblocks, nthreads, shm, s>>>(data, tw, r1, r2, es, ncols, os, ngroups, ks);
+        launch_chained(kern, nblocks, nthreads, shm, s, data, tw, r1, r2, es, ncols, os, ngroups, ks);
     };
     if (cls == 8) go(k_fft2<R, CW, MODE, 8>);
     else if (cls == 12) go(k_fft2<R, CW, MODE, 12>);
@@ -515,6 +517,7 @@ template <typename R, int MC, int ZMAX, int CLS>
 __global__ void __launch_bounds__(kSlabThreads) k_slab(cplx<R>* __restrict__ data, const cplx<R>* __restrict__ tw,
                                                        const cplx<R>* __restrict__ taps, int r1, int r2,
                                                        SlabArgs a) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int n = r1 * r2;
     const int Zs = a.Zs, M = a.M, B = 3 * M;
@@ -813,7 +816,6 @@ void AxisFFT::launch_line(cplx<R>* data, size_t es, int ncols, size_t os, int no
         if (mode == 2) go(std::integral_constant<int, 2>{});
         else if (mode == 1) go(std::integral_constant<int, 1>{});
         else go(std::integral_constant<int, 0>{});
-        MPM_LAUNCH();
         return;
     }
     // the prime-pass tables go to shared memory when small (else the pass
@@ -882,7 +884,7 @@ void AxisFFT::run_slab(cplx<R>* data, int nx, int Zs, int M, const cplx<R>* taps
     const int cls = register_class(r1_);
     auto go = [&](auto kern) {
         set_smem_limit(kern, shm);
-        kern<<<nx * a.nchunk, kSlabThreads, shm, s>>>(data, tw, taps, r1_, r2_, a);
+        launch_chained(kern, nx * a.nchunk, kSlabThreads, shm, s, data, tw, taps, r1_, r2_, a);
     };
     if (Zs == 1) {
         if (cls == 8) go(k_slab<R, MC1, 1, 8>);
@@ -897,7 +899,6 @@ void AxisFFT::run_slab(cplx<R>* data, int nx, int Zs, int M, const cplx<R>* taps
         else if (cls == 12) go(k_slab<R, MCS, 16, 12>);
         else go(k_slab<R, MCS, 16, 16>);
     }
-    MPM_LAUNCH();
 }
 
 template void AxisFFT::run_slab<float>(float2*, int, int, int, const float2*, double, double, cudaStream_t) const;

@@ -22,6 +22,7 @@
 //    Jacobi scaling and the INTERACTION_FIELD sign are fused into it.
 #include "mpm_field.h"
 #include "mpm_bins.cuh"
+#include "mpm_chain.cuh"
 #include "mpm_profile.h"
 
 #include <cub/cub.cuh>
@@ -446,6 +447,7 @@ __global__ void __launch_bounds__(256) k_spread_planned(const double2* __restric
                                                         const R* __restrict__ wT, const R* __restrict__ lwT,
                                                         const int* __restrict__ lcT, const int* __restrict__ lnT,
                                                         cplx<R>* __restrict__ grid) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int ncol = TX * TY;
     R* lwS = reinterpret_cast<R*>(smem_raw);                              // [ncol][kSpreadListCap]
@@ -596,6 +598,7 @@ __global__ void __launch_bounds__(256) k_spread_planned_1z(const double2* __rest
                                                            const R* __restrict__ wT, const R* __restrict__ lwT,
                                                            const int* __restrict__ lcT, const int* __restrict__ lnT,
                                                            cplx<R>* __restrict__ grid) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int ncol = TX * TY;
     R* lwS = reinterpret_cast<R*>(smem_raw);                          // [ncol][kSpreadListCap]
@@ -715,6 +718,7 @@ __device__ __forceinline__ void khat_at(int ix, int iy, int iz, int Nx, int Ny, 
 template <typename R, bool QUADS>
 __global__ void k_scale(cplx<R>* __restrict__ grid, const R* __restrict__ sc, int Nx, int Ny, int Nz, double Lx,
                         double Ly, double Lz, int M, double bx, double by) {
+    chain_enter();
     const size_t V = size_t(Nx) * Ny * Nz;
     const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= V * M) return;
@@ -941,6 +945,7 @@ __global__ void k_build_layer_taps(ScaleArgs a, const double* __restrict__ w2, d
 // applied to all Z outputs (ZMAX bounds Z at compile time).
 template <typename R, int ZMAX>
 __global__ void k_column(cplx<R>* __restrict__ grid, const cplx<R>* __restrict__ K, int Z, int M) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int col = blockIdx.x;
     const int B = 3 * M;
@@ -998,6 +1003,7 @@ __global__ void k_contract(const cplx<R>* __restrict__ grid, GridView g, int M, 
                            const int4* __restrict__ base, const R* __restrict__ w1, double factor,
                            const int* __restrict__ quad_map, double2* __restrict__ Y,
                            const int* __restrict__ order, int accumulate, const double2* __restrict__ jsc) {
+    chain_enter();
     __shared__ R w[3 * kMaxStencil];
     __shared__ int idx[3 * kMaxStencil];
     __shared__ long long offxy[2 * kMaxStencil];   // x then y stencil offsets into the grid (elements)
@@ -1091,6 +1097,7 @@ __global__ void __launch_bounds__(128) k_contract_few(const cplx<R>* __restrict_
                                                       double factor, const int* __restrict__ quad_map,
                                                       double2* __restrict__ Y, const int* __restrict__ order,
                                                       int accumulate, const double2* __restrict__ jsc) {
+    chain_enter();
     constexpr int TPC = 4 / WPT;
     __shared__ R w[TPC][3 * kMaxStencil];
     __shared__ long long off[TPC][2 * kMaxStencil];    // x then y stencil offsets into the grid (elements)
@@ -1414,6 +1421,7 @@ __global__ void __launch_bounds__(128) k_real(const double2* __restrict__ X, dou
                                               const int* __restrict__ quad_map,
                                               const double2* __restrict__ sc, const double* __restrict__ selfv,
                                               const cplx<R>* __restrict__ ph) {
+    chain_enter();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= a.Nt) return;
@@ -1581,6 +1589,7 @@ __global__ void __launch_bounds__(128) k_direct(const double2* __restrict__ X, d
                                                 int Nt, const double* __restrict__ src,
                                                 const double* __restrict__ tgt, const double* __restrict__ rad,
                                                 const double2* __restrict__ sc, int solver_ax, int jacobi) {
+    chain_enter();
     constexpr int SL = 128 / TG;   // source slices
     constexpr int kStage = kDirectTile * (3 * CB * int(sizeof(cplx<R>)) + 4 * int(sizeof(R)));
     constexpr int kRed = 128 * 3 * CB * int(sizeof(cplx<R>));
@@ -2434,14 +2443,14 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
         const R* lw = f32 ? reinterpret_cast<const R*>(plan_lw32_.p) : reinterpret_cast<const R*>(plan_lw64_.p);
         auto go = [&](auto kern) {
             set_smem_limit(kern, pshm);
-            kern<<<grd, 256, pshm, s>>>(X, M, N_, C, quad_map_.as<int>(), gv_, TX, TY, TZ, ps.nb[0], ps.nb[1],
-                                        ps.nb[2], plan_cap_, bc, plan_nc_.as<int>(), plan_cid_.as<int>(), wT, lw,
+            launch_chained(kern, grd, 256, pshm, s, X, M, N_, C, quad_map_.as<int>(), gv_, TX, TY, TZ, ps.nb[0],
+                           ps.nb[1], ps.nb[2], plan_cap_, bc, plan_nc_.as<int>(), plan_cid_.as<int>(), wT, lw,
                                         plan_lc_.as<int>(), plan_ln_.as<int>(), grid);
         };
         // the tile's z run in registers: as many accumulators as it needs
         if (TZ == 1 && gv_.Zs == 1) {
             set_smem_limit(k_spread_planned_1z<R>, pshm);
-            k_spread_planned_1z<R><<<grd, 256, pshm, s>>>(X, M, N_, C, quad_map_.as<int>(), gv_, TX, TY, ps.nb[0],
+            launch_chained(k_spread_planned_1z<R>, grd, 256, pshm, s, X, M, N_, C, quad_map_.as<int>(), gv_, TX, TY, ps.nb[0],
                                                           ps.nb[1], plan_cap_, bc, plan_nc_.as<int>(),
                                                           plan_cid_.as<int>(), wT, lw, plan_lc_.as<int>(),
                                                           plan_ln_.as<int>(), grid);
@@ -2453,8 +2462,8 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
         k_spread<R><<<grd, 256, shm, s>>>(X, M, N_, C, quad_map_.as<int>(), ps.base.as<int4>(), w1,
                                           ps.bin_start.as<int>(), ps.bin_end.as<int>(), ps.idx_sorted.as<int>(),
                                           gv_, TX, TY, TZ, ps.nb[0], ps.nb[1], ps.nb[2], cap, bc, grid);
+        MPM_LAUNCH();
     }
-    MPM_LAUNCH();
     Profiler::get().end(ST_SPREAD, s);
     if (use_slab()) {
         // x forward; y forward, slab Green tensor and y inverse in one pass;
@@ -2491,23 +2500,21 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
                 throw std::runtime_error("column kernel not built for the current layout");
             auto go = [&](auto kern) {
                 set_smem_limit(kern, shm2);
-                kern<<<gv_.Nx * gv_.Ny, thr, shm2, s>>>(grid, K, Z, M);
+                launch_chained(kern, gv_.Nx * gv_.Ny, thr, shm2, s, grid, K, Z, M);
             };
             if (Z <= 9) go(k_column<R, 9>);
             else if (Z <= 16) go(k_column<R, 16>);
             else go(k_column<R, 24>);
-            MPM_LAUNCH();
         } else {
             const size_t V = size_t(gv_.Nx) * gv_.Ny * gv_.Zs;
             const R* sc = sizeof(R) == 4 ? reinterpret_cast<const R*>(scale32_.p) : reinterpret_cast<const R*>(scale64_.p);
             if (scale_built_ != (Nq_ ? 4 : 1) || !sc) throw std::runtime_error("k-space scale not built");
-            if (Nq_)
-                k_scale<R, true><<<nblk((long long)(V * M), 256), 256, 0, s>>>(grid, sc, gv_.Nx, gv_.Ny, gv_.Nz, spec_.box[0],
-                                                                               spec_.box[1], spec_.box[2], M, spec_.bloch[0], spec_.bloch[1]);
-            else
-                k_scale<R, false><<<nblk((long long)(V * M), 256), 256, 0, s>>>(grid, sc, gv_.Nx, gv_.Ny, gv_.Nz, spec_.box[0],
-                                                                                spec_.box[1], spec_.box[2], M, spec_.bloch[0], spec_.bloch[1]);
-            MPM_LAUNCH();
+            auto scale = [&](auto kern) {
+                launch_chained(kern, nblk((long long)(V * M), 256), 256, 0, s, grid, sc, gv_.Nx, gv_.Ny, gv_.Nz,
+                               spec_.box[0], spec_.box[1], spec_.box[2], M, spec_.bloch[0], spec_.bloch[1]);
+            };
+            if (Nq_) scale(k_scale<R, true>);
+            else scale(k_scale<R, false>);
         }
         Profiler::get().end(ST_KSPACE, s);
         Profiler::get().begin(ST_FFT_INV, s);
@@ -2523,14 +2530,14 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
     const int thr = std::min(256, ((B + 31) / 32) * 32);
     if (ov) MPM_CUDA(cudaStreamWaitEvent(s, ov->join, 0));   // the real-space part is in Y
     auto contract = [&](auto kern) {
-        kern<<<nt, thr, 0, s>>>(grid, gv_, M, C, nt, tg.base.as<int4>(), tw, factor,
+        launch_chained(kern, nt, thr, 0, s, grid, gv_, M, C, nt, tg.base.as<int4>(), tw, factor,
                                 spec_.solver_ax ? quad_map_.as<int>() : nullptr, Y,
                                 spec_.solver_ax ? sources_.idx_sorted.as<int>() : nullptr, ov ? 1 : 0,
                                 ov ? ov->jacobi_sc : nullptr);
     };
     if (B <= 16 && gv_.Sz <= 13) {
         auto few = [&](auto kern, int tpc) {
-            kern<<<nblk(nt, tpc), 128, 0, s>>>(grid, gv_, M, C, nt, tg.base.as<int4>(), tw, factor,
+            launch_chained(kern, nblk(nt, tpc), 128, 0, s, grid, gv_, M, C, nt, tg.base.as<int4>(), tw, factor,
                                                spec_.solver_ax ? quad_map_.as<int>() : nullptr, Y,
                                                spec_.solver_ax ? sources_.idx_sorted.as<int>() : nullptr, ov ? 1 : 0,
                                                ov ? ov->jacobi_sc : nullptr);
@@ -2552,7 +2559,6 @@ void Field::recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cudaStr
     } else {
         contract(k_contract<R, 0, 0>);
     }
-    MPM_LAUNCH();
 }
 
 void Field::real_part(const double2* X, double2* Y, int M, const double2* sc, bool jacobi, bool fp32, bool add_recip,
@@ -2580,7 +2586,7 @@ void Field::real_part(const double2* X, double2* Y, int M, const double2* sc, bo
     if (ph && num_pairs_ > 0 && pair_ph64_.bytes < sizeof(double2) * size_t(num_pairs_))
         throw std::runtime_error("Bloch pair phases not built for the current pairs");
     auto go = [&](auto kern, const auto* T, const auto* P) {
-        kern<<<blocks, thr, 0, s>>>(X, Y, a, pair_off_.as<int>(), pair_src_.as<int>(), T, pair_Q_.as<double>(),
+        launch_chained(kern, blocks, thr, 0, s, X, Y, a, pair_off_.as<int>(), pair_src_.as<int>(), T, pair_Q_.as<double>(),
                                     quad_map_.as<int>(), sc, selfv, P);
     };
     if (fp32) {
@@ -2592,7 +2598,6 @@ void Field::real_part(const double2* X, double2* Y, int M, const double2* sc, bo
         if (a.quads) go(k_real<double, true>, pair_T64_.as<double>(), P);
         else go(k_real<double, false>, pair_T64_.as<double>(), P);
     }
-    MPM_LAUNCH();
 }
 
 void Field::direct(const double2* X, double2* Y, int M, const double2* sc, bool jacobi, bool fp32, cudaStream_t s) {
@@ -2613,8 +2618,8 @@ void Field::direct(const double2* X, double2* Y, int M, const double2* sc, bool 
         return;
     }
     auto go = [&](auto kern, int cb, int tgs) {
-        kern<<<dim3(nblk(nt, tgs), nblk(M, cb)), 128, 0, s>>>(X, Y, M, N_, nt, src, tg, rad, sc, spec_.solver_ax,
-                                                              jacobi);
+        launch_chained(kern, dim3(nblk(nt, tgs), nblk(M, cb)), 128, 0, s, X, Y, M, N_, nt, src, tg, rad, sc,
+                       int(spec_.solver_ax), int(jacobi));
     };
     // columns per CTA: one or three (a frequency's polarisations) in one CTA,
     // else six, the most whose sums stay in registers.  Targets per CTA: 32,
@@ -2630,7 +2635,6 @@ void Field::direct(const double2* X, double2* Y, int M, const double2* sc, bool 
     };
     if (fp32) pick(float{});
     else pick(double{});
-    MPM_LAUNCH();
 }
 
 void Field::apply(const double2* X, double2* Y, int M, const double2* sc, bool jacobi, bool recip_fp32,

@@ -1,5 +1,6 @@
 // Batched device Krylov solvers (see mpm_krylov.h).
 #include "mpm_krylov.h"
+#include "mpm_chain.cuh"
 #include "mpm_profile.h"
 
 #include <algorithm>
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(256) k_dots1s(const double2* __restrict__ V, s
                                                 const double2* __restrict__ w, int rows, int M, int conj,
                                                 double2* __restrict__ partial, double2* __restrict__ out,
                                                 double* __restrict__ nrm, unsigned int* __restrict__ done) {
+    chain_enter();
     __shared__ double2 red[8][256];
     const int L = (256 / M) * M;
     const int j = threadIdx.x;
@@ -406,6 +408,7 @@ __global__ void __launch_bounds__(256) k_arn_finish1(GState* __restrict__ st, do
 __global__ void k_arn_update(double2* __restrict__ V, size_t vstride, int k, const double2* __restrict__ h,
                              const GState* __restrict__ st, const double* __restrict__ inv_nu, int rows, int M,
                              int pass) {
+    chain_enter();
     const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= size_t(rows) * M) return;
     const int m = int(t % M);
@@ -590,6 +593,7 @@ __global__ void __launch_bounds__(256) k_arn_finish2(GState* __restrict__ st, do
 __global__ void __launch_bounds__(256) k_arn_dots(const double2* __restrict__ V, size_t vstride, int k, int rows,
                                                   int M, double2* __restrict__ partial, GState* __restrict__ st,
                                                   double2* __restrict__ h, unsigned int* __restrict__ done) {
+    chain_enter();
     __shared__ double2 red[8][256];
     const int nvec = k + 2;
     const int L = (256 / M) * M;
@@ -626,6 +630,7 @@ __global__ void __launch_bounds__(256) k_arn_project(double2* __restrict__ V, si
                                                      double2* __restrict__ partial, GState* __restrict__ st,
                                                      double2* __restrict__ h, double2* __restrict__ h2, HessArgs a,
                                                      MemberArgs mb, unsigned int* __restrict__ done) {
+    chain_enter();
     __shared__ double2 red[8][256];
     const int nvec = k + 2;
     const int L = (256 / M) * M;
@@ -962,6 +967,7 @@ __global__ void k_axpy1(double2* __restrict__ x, const double2* __restrict__ d, 
 // dst[row][j] = src[row][idx[j]]  (compact batch of the listed columns)
 __global__ void k_gather_cols(const double2* __restrict__ src, int M, double2* __restrict__ dst, int Ma,
                               const int* __restrict__ idx, int rows) {
+    chain_enter();
     const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= size_t(rows) * Ma) return;
     const size_t row = t / Ma;
@@ -972,6 +978,7 @@ __global__ void k_gather_cols(const double2* __restrict__ src, int M, double2* _
 // dst[row][idx[j]] = src[row][j]
 __global__ void k_scatter_cols(const double2* __restrict__ src, int Ma, double2* __restrict__ dst, int M,
                                const int* __restrict__ idx, int rows) {
+    chain_enter();
     const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= size_t(rows) * Ma) return;
     const size_t row = t / Ma;
@@ -1071,16 +1078,14 @@ int BatchSolver::apply_cols(Field& F, const double2* X, double2* Y, int M, const
     yc_.ensure(sizeof(double2) * size_t(rout) * M);
     {
         StageScope scope(ST_KRYLOV, s);
-        k_gather_cols<<<nblk((long long)rin * Ma, 256), 256, 0, s>>>(X, M, xc_.as<double2>(), Ma, cidx_.as<int>(),
-                                                                     rin);
-        MPM_LAUNCH();
+        launch_chained(k_gather_cols, nblk((long long)rin * Ma, 256), 256, 0, s, X, M, xc_.as<double2>(), Ma,
+                       cidx_.as<int>(), rin);
     }
     F.apply(xc_.as<double2>(), yc_.as<double2>(), Ma, sc ? scc_.as<double2>() : nullptr, jacobi, r32, re32, s);
     {
         StageScope scope(ST_KRYLOV, s);
-        k_scatter_cols<<<nblk((long long)rout * Ma, 256), 256, 0, s>>>(yc_.as<double2>(), Ma, Y, M,
-                                                                       cidx_.as<int>(), rout);
-        MPM_LAUNCH();
+        launch_chained(k_scatter_cols, nblk((long long)rout * Ma, 256), 256, 0, s, yc_.as<double2>(), Ma, Y, M,
+                       cidx_.as<int>(), rout);
     }
     return Ma;
 }
@@ -1160,10 +1165,8 @@ void BatchSolver::arnoldi(double2* V, int k, int rows, int M, void* state, const
         partial_.ensure(sizeof(double2) * size_t(gx) * (a.restart + 2) * M);
         double2* part = partial_.as<double2>();
         unsigned int* done = done_counter(s);
-        k_arn_dots<<<dim3(gx, 1, (k + 2 + 7) / 8), 256, 0, s>>>(V, n, k, rows, M, part, st, h, done);
-        MPM_LAUNCH();
-        k_arn_project<<<gx, 256, 0, s>>>(V, n, k, rows, M, part, st, h, h2, a, mb, done);
-        MPM_LAUNCH();
+        launch_chained(k_arn_dots, dim3(gx, 1, (k + 2 + 7) / 8), 256, 0, s, V, n, k, rows, M, part, st, h, done);
+        launch_chained(k_arn_project, gx, 256, 0, s, V, n, k, rows, M, part, st, h, h2, a, mb, done);
     } else {
         double2* w = V + size_t(k + 1) * n;
         const bool seeds = mb.st != nullptr;
@@ -1177,8 +1180,7 @@ void BatchSolver::arnoldi(double2* V, int k, int rows, int M, void* state, const
         k_arn_finish2<<<1, fthr, 0, s>>>(st, h, h2, a, mb, k, M);
         MPM_LAUNCH();
     }
-    k_arn_update<<<vb, 256, 0, s>>>(V, n, k, h2, st, a.inv_nu, rows, M, 2);
-    MPM_LAUNCH();
+    launch_chained(k_arn_update, vb, 256, 0, s, V, n, k, h2, st, a.inv_nu, rows, M, 2);
 }
 
 void BatchSolver::true_residual(Field& F, const double2* b, const double2* x, int M, const double2* sc,

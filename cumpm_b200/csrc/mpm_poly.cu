@@ -26,6 +26,7 @@
 //    reads are evaluated on the fly, so no table is stored: a continuous
 //    radius distribution (one class per particle) costs nothing extra.
 #include "mpm_bins.cuh"
+#include "mpm_chain.cuh"
 #include "mpm_field.h"
 #include "mpm_poly.cuh"
 #include "mpm_profile.h"
@@ -271,6 +272,7 @@ __global__ void __launch_bounds__(256) k_poly_spread(const double2* __restrict__
                                                      const int4* __restrict__ base, const int* __restrict__ toff,
                                                      const int* __restrict__ tcnt, const int* __restrict__ clist,
                                                      PolyTile t, cplx<R>* __restrict__ grid) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char shraw[];
     R* wb = reinterpret_cast<R*>(shraw);                                    // [stages][kPolyPer][64 rows][8 z][3]
     cplx<R>* pm = reinterpret_cast<cplx<R>*>(wb + kPolyStages * kPolyPer * 64 * 24);   // [cap][3][CM]
@@ -433,6 +435,7 @@ __global__ void __launch_bounds__(256) k_poly_contract(const cplx<R>* __restrict
                                                        const int4* __restrict__ base, const R* __restrict__ w, int P,
                                                        int Nx, int Ny, int Nz, double factor,
                                                        double2* __restrict__ Y) {
+    chain_enter();
     constexpr int CW = 8, NG = 32 / GS;
     __shared__ cplx<R> red[CW][3][GS];
     const int j = blockIdx.x;
@@ -931,7 +934,7 @@ void Field::poly_recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cu
             constexpr int CM = decltype(cmc)::value;
             const size_t shm = poly_spread_smem<R>(t.cap, CM);
             set_smem_limit(k_poly_spread<R, CM>, shm);
-            k_poly_spread<R, CM><<<ntile * ((M + CM - 1) / CM), 256, shm, s>>>(
+            launch_chained(k_poly_spread<R, CM>, ntile * ((M + CM - 1) / CM), 256, shm, s,
                 X, M, w1, ps.base.as<int4>(), ptoff_.as<int>(), ptcnt_.as<int>(), ptclist_.as<int>(), t, grid);
         };
         auto ctas = [&](int cm) { return (long long)ntile * ((M + cm - 1) / cm); };
@@ -943,7 +946,6 @@ void Field::poly_recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cu
             if (M > 4 && ctas(8) >= 2 * 148) go(std::integral_constant<int, 8>{});
             else go(std::integral_constant<int, 4>{});
         }
-        MPM_LAUNCH();
     }
     const R* scl = sizeof(R) == 4 ? reinterpret_cast<const R*>(scale32_.p) : reinterpret_cast<const R*>(scale64_.p);
     const size_t V = size_t(gv_.Nx) * gv_.Ny * gv_.Nz;
@@ -1017,7 +1019,7 @@ void Field::poly_recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cu
     const double factor = pgeom_.h[0] * pgeom_.h[1] * pgeom_.h[2];
     auto contract = [&](auto gsc, auto mcc) {
         constexpr int GS = decltype(gsc)::value, MC = decltype(mcc)::value;
-        k_poly_contract<R, GS, MC><<<dim3(tg.n, (M + GS * MC - 1) / (GS * MC)), 256, 0, s>>>(
+        launch_chained(k_poly_contract<R, GS, MC>, dim3(tg.n, (M + GS * MC - 1) / (GS * MC)), 256, 0, s,
             grid, M, tg.base.as<int4>(), tw, pgeom_.P, gv_.Nx, gv_.Ny, gv_.Nz, factor, Y);
     };
     using std::integral_constant;
@@ -1027,7 +1029,6 @@ void Field::poly_recip_on(const double2* X, double2* Y, int M, cplx<R>* grid, cu
     else if (M <= 32) contract(integral_constant<int, 16>{}, integral_constant<int, 2>{});
     else if (M <= 48) contract(integral_constant<int, 16>{}, integral_constant<int, 3>{});
     else contract(integral_constant<int, 32>{}, integral_constant<int, 3>{});
-    MPM_LAUNCH();
     if (Nq_) {
         k_poly_quad_contract<R><<<Nq_, 128, 0, s>>>(gq, M, tg.base.as<int4>(), qw, pgeom_.P, gv_.Nx, gv_.Ny, gv_.Nz,
                                                    quad_idx_.as<int>(), tg.n, Y);
