@@ -11,10 +11,10 @@
 // at its last tile: the successor's waiting CTAs hold slots that a second
 // stream's kernels could use (500 particles with quadrupoles: 948 us released
 // at entry, 937 unchained, and 906 against 925 unchained with the late
-// release).  GMRES of 8000 particles, 3 columns: 2.64 ms unchained, 2.27 now;
-// its operator with 3 x 3 columns 276 and 265 us; a spectrum of a 4000-particle
-// layer 16.3 and 15.2 ms.  (Only grids below eight CTAs per SM chained: the
-// operator 316 us against 301 with all of them.)
+// release).  GMRES of 500 particles, one column: 2.64 ms unchained, 2.27 now;
+// an operator on 8000 particles and three columns 276 and 265 us; a spectrum
+// of a 4000-particle layer 16.3 and 15.2 ms.  (Only grids below eight CTAs
+// per SM chained: that operator 316 us against 301 with all of them.)
 #pragma once
 
 #include "mpm_common.cuh"
