@@ -42,6 +42,15 @@ inline void set_smem_limit(K* kernel, size_t bytes) {
 void note_launch();
 #define MPM_LAUNCH() (::mpm::note_launch(), ::mpm::cuda_check(cudaGetLastError(), "kernel launch", __FILE__, __LINE__))
 
+// Host data for kernels on any stream.  cudaMemcpy from pageable memory may
+// return once the data are staged, and a stream made with
+// cudaStreamNonBlocking does not wait for the legacy stream that carries them,
+// so that stream is waited for here.
+inline void upload(void* dst, const void* src, size_t bytes) {
+    MPM_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+    MPM_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+}
+
 // --------------------------------------------------------------- complex --
 
 template <typename R> struct CTraits;

@@ -307,8 +307,8 @@ void DenseDFT::init(int n, int r1) {
     std::vector<float> tf(t.begin(), t.end());
     t64_.ensure(sizeof(double) * t.size());
     t32_.ensure(sizeof(float) * tf.size());
-    MPM_CUDA(cudaMemcpy(t64_.p, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice));
-    MPM_CUDA(cudaMemcpy(t32_.p, tf.data(), sizeof(float) * tf.size(), cudaMemcpyHostToDevice));
+    upload(t64_.p, t.data(), sizeof(double) * t.size());
+    upload(t32_.p, tf.data(), sizeof(float) * tf.size());
 }
 
 bool DenseDFT::fits(bool fp64) const {

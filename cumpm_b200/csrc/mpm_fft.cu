@@ -744,8 +744,8 @@ void AxisFFT::init(int n) {
     }
     tw64_.ensure(sizeof(double2) * n);
     tw32_.ensure(sizeof(float2) * n);
-    MPM_CUDA(cudaMemcpy(tw64_.p, t64.data(), sizeof(double2) * n, cudaMemcpyHostToDevice));
-    MPM_CUDA(cudaMemcpy(tw32_.p, t32.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
+    upload(tw64_.p, t64.data(), sizeof(double2) * n);
+    upload(tw32_.p, t32.data(), sizeof(float2) * n);
     // W_r^(p q) tables of the general kernel's streamed (r > 16) passes
     std::vector<double2> p64;
     for (int i = 0; i < f_.nf; ++i) {
@@ -773,8 +773,8 @@ void AxisFFT::upload_table(std::vector<double2> t64, DevBuf& d64, DevBuf& d32) {
     for (size_t k = 0; k < t64.size(); ++k) t32[k] = make_float2(float(t64[k].x), float(t64[k].y));
     d64.ensure(sizeof(double2) * t64.size());
     d32.ensure(sizeof(float2) * t32.size());
-    MPM_CUDA(cudaMemcpy(d64.p, t64.data(), sizeof(double2) * t64.size(), cudaMemcpyHostToDevice));
-    MPM_CUDA(cudaMemcpy(d32.p, t32.data(), sizeof(float2) * t32.size(), cudaMemcpyHostToDevice));
+    upload(d64.p, t64.data(), sizeof(double2) * t64.size());
+    upload(d32.p, t32.data(), sizeof(float2) * t32.size());
 }
 
 template <typename R>

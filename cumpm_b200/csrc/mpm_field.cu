@@ -1855,10 +1855,10 @@ Field::Field(const FieldSpec& spec) : spec_(spec) {
         tables_ = build_mono_tables(spec_.xi, spec_.quads);
         tab_r_.ensure(sizeof(double) * kTableSize);
         tab_f_.ensure(sizeof(double) * kTableSize * T_COUNT);
-        MPM_CUDA(cudaMemcpy(tab_r_.p, tables_.r.data(), sizeof(double) * kTableSize, cudaMemcpyHostToDevice));
+        upload(tab_r_.p, tables_.r.data(), sizeof(double) * kTableSize);
         for (int f = 0; f < (spec_.quads ? int(T_COUNT) : int(T_FD2) + 1); ++f)
-            MPM_CUDA(cudaMemcpy(tab_f_.as<double>() + size_t(f) * kTableSize, tables_.f[f].data(),
-                                sizeof(double) * kTableSize, cudaMemcpyHostToDevice));
+            upload(tab_f_.as<double>() + size_t(f) * kTableSize, tables_.f[f].data(),
+                   sizeof(double) * kTableSize);
     } else if (spec_.kind == FIELD_POLY) {
         poly_init();
     } else if (spec_.kind != FIELD_DIRECT) {
@@ -1905,10 +1905,10 @@ void Field::set_positions(const double* x, const double* y, const double* z, int
         for (int q = 0; q < Nq_; ++q)
             if (qidx[q] >= 0 && qidx[q] < N_) qmap[qidx[q]] = q;
         quad_map_.ensure(sizeof(int) * N_);
-        MPM_CUDA(cudaMemcpy(quad_map_.p, qmap.data(), sizeof(int) * N_, cudaMemcpyHostToDevice));
+        upload(quad_map_.p, qmap.data(), sizeof(int) * N_);
         if (Nq_) {
             quad_idx_.ensure(sizeof(int) * Nq_);
-            MPM_CUDA(cudaMemcpy(quad_idx_.p, qidx.data(), sizeof(int) * Nq_, cudaMemcpyHostToDevice));
+            upload(quad_idx_.p, qidx.data(), sizeof(int) * Nq_);
         }
         if (spec_.kind == FIELD_POLY && int(spec_.radius.size()) != N_)
             throw std::invalid_argument("Polydisperse field: radius size must match num_particles.");
@@ -1917,7 +1917,7 @@ void Field::set_positions(const double* x, const double* y, const double* z, int
             if (rad.empty()) rad.assign(N_, 0.0);
             if (int(rad.size()) != N_) throw std::invalid_argument("Direct field: radius size must match num_particles.");
             radius_.ensure(sizeof(double) * N_);
-            MPM_CUDA(cudaMemcpy(radius_.p, rad.data(), sizeof(double) * N_, cudaMemcpyHostToDevice));
+            upload(radius_.p, rad.data(), sizeof(double) * N_);
         }
     }
     sources_.n = n;

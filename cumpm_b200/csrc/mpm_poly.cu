@@ -719,18 +719,17 @@ void Field::poly_init() {
     prad_.ensure(sizeof(double) * nu);
     pself_.ensure(sizeof(double) * n);
     radius_.ensure(sizeof(double) * n);
-    MPM_CUDA(cudaMemcpy(pcls_.p, pgeom_.cls.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    MPM_CUDA(cudaMemcpy(prad_.p, pgeom_.unique.data(), sizeof(double) * nu, cudaMemcpyHostToDevice));
-    MPM_CUDA(cudaMemcpy(pself_.p, selfv.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-    MPM_CUDA(cudaMemcpy(radius_.p, spec_.radius.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
+    upload(pcls_.p, pgeom_.cls.data(), sizeof(int) * n);
+    upload(prad_.p, pgeom_.unique.data(), sizeof(double) * nu);
+    upload(pself_.p, selfv.data(), sizeof(double) * n);
+    upload(radius_.p, spec_.radius.data(), sizeof(double) * n);
     if (spec_.quads) {
         const int qn = pgeom_.table_n;
         const auto QT = build_poly_quad_tables(spec_.xi, qn);
         pqtab_.ensure(sizeof(double) * 8 * size_t(qn));
-        MPM_CUDA(cudaMemcpy(pqtab_.p, QT.r.data(), sizeof(double) * qn, cudaMemcpyHostToDevice));
+        upload(pqtab_.p, QT.r.data(), sizeof(double) * qn);
         for (int f = 0; f < PQ_COUNT; ++f)
-            MPM_CUDA(cudaMemcpy(pqtab_.as<double>() + size_t(f + 1) * qn, QT.f[f].data(), sizeof(double) * qn,
-                                cudaMemcpyHostToDevice));
+            upload(pqtab_.as<double>() + size_t(f + 1) * qn, QT.f[f].data(), sizeof(double) * qn);
         // a from the particle, the self value from its radius class (:1171-1177)
         std::vector<double> a2(n), g2(n);
         for (int i = 0; i < n; ++i) {
@@ -739,8 +738,8 @@ void Field::poly_init() {
         }
         pqa2_.ensure(sizeof(double) * n);
         pqg2_.ensure(sizeof(double) * n);
-        MPM_CUDA(cudaMemcpy(pqa2_.p, a2.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-        MPM_CUDA(cudaMemcpy(pqg2_.p, g2.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
+        upload(pqa2_.p, a2.data(), sizeof(double) * n);
+        upload(pqg2_.p, g2.data(), sizeof(double) * n);
     }
     gv_.Nx = pgeom_.ng[0];
     gv_.Ny = pgeom_.ng[1];

@@ -266,7 +266,9 @@ bool DipoleSolver::device_ok() const {
     return true;
 }
 
-// permittivities [W][N], radii and incident fields, once per solver
+// permittivities [W][N], radii and incident fields, once per solver.  On the
+// solve's own stream: it does not wait for the legacy stream, and a copy from
+// pageable memory may have left its source before it has reached the device.
 void DipoleSolver::upload_inputs() {
     const size_t K = E0_.size(), W = eps_p_.size();
     if (!dev_eps_) {
@@ -278,9 +280,9 @@ void DipoleSolver::upload_inputs() {
         dEps_.ensure(sizeof(double2) * W * N_);
         dRad_.ensure(sizeof(double) * N_);
         dE0_.ensure(sizeof(double2) * K * 3);
-        MPM_CUDA(cudaMemcpy(dEps_.p, e.data(), sizeof(double2) * W * N_, cudaMemcpyHostToDevice));
-        MPM_CUDA(cudaMemcpy(dRad_.p, radius_.data(), sizeof(double) * N_, cudaMemcpyHostToDevice));
-        MPM_CUDA(cudaMemcpy(dE0_.p, e0.data(), sizeof(double2) * K * 3, cudaMemcpyHostToDevice));
+        MPM_CUDA(cudaMemcpyAsync(dEps_.p, e.data(), sizeof(double2) * W * N_, cudaMemcpyHostToDevice, stream_));
+        MPM_CUDA(cudaMemcpyAsync(dRad_.p, radius_.data(), sizeof(double) * N_, cudaMemcpyHostToDevice, stream_));
+        MPM_CUDA(cudaMemcpyAsync(dE0_.p, e0.data(), sizeof(double2) * K * 3, cudaMemcpyHostToDevice, stream_));
         dev_eps_ = true;
     }
 }
