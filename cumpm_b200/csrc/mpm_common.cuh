@@ -106,6 +106,7 @@ __host__ __device__ __forceinline__ int cyc_diff(int a, int b, int n) {
 }
 
 constexpr double kPi = 3.14159265358979323846;
+constexpr long double kPiL = 3.14159265358979323846264338327950288L;   // (host)
 
 // --------------------------------------------------------------- buffers --
 

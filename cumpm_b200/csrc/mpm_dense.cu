@@ -8,16 +8,16 @@
 //   A_p = sum_q (x_q + x_(m-q)) cos(2 pi p q / m),
 //   B_p = sum_q (x_q - x_(m-q)) sin(2 pi p q / m),
 //   y_p = x_0 + A_p - i B_p,  y_(m-p) = x_0 + A_p + i B_p,
-// m real FMAs per element.  A thread holds eight p of two fp32 columns (one
-// fp64 column) in registers, so a step over q costs 64 (32) FMAs against 8
-// (10) shared loads: at one FMA per lane and clock an element of m = 109 costs 3 ps
-// of this GPU, against the 2.5 ps that its trip through HBM takes, and m = 53
-// is bound by that trip.  (Packed fp32 pairs, fma.rn.f32x2, halve the FMA
-// instructions but took more to arrange their operands: slower.)  The
-// alternative for primes, Rader's convolution through two (p-1)-point
-// transforms, needs a quarter of the arithmetic but three more shared round
-// trips and gathers by g^q: it ran at 12 ps per element where this kernel
-// takes 8.9 (109^3 x 48 columns, fp32).
+// m real FMAs per element.  A thread holds A or B (fp64: A and B) of eight p
+// and two columns (fp64: one) in registers, so a step over q costs 32 FMAs
+// against 4 (10) shared loads: at one FMA per lane and clock an element of
+// m = 109 costs 3 ps of this GPU, against the 2.5 ps that its trip through HBM
+// takes, and m = 53 is bound by that trip.  (Packed fp32 pairs, fma.rn.f32x2,
+// halve the FMA instructions but took more to arrange their operands: slower.)
+// The alternative for primes, Rader's convolution (mpm_rader.cu), needs a
+// quarter of the arithmetic but three more shared round trips and gathers by
+// g^q: 736 us for a 109-point pass of 497 MB (48 fp32 columns) that takes 558
+// here; see AxisFFT::path for where it is the faster one.
 //
 // Columns are enumerated over lines and columns together (f = line * ncols +
 // column), so a transform of few columns per line (the z axis of a solve's
@@ -40,14 +40,25 @@ constexpr int kPC = 8;    // output pairs per thread
 // thread, two fp32 butterflies half of them
 template <typename R> __host__ __device__ constexpr int dense_ctas(bool radix2) { return radix2 && sizeof(R) == 4 ? 4 : 2; }
 
-template <typename R> constexpr int dense_ct() { return sizeof(R) == 4 ? 2 : 1; }   // columns per thread
+constexpr int kChunk = 2 * kPC;   // eight pairs' table entries: cosines, sines
+
+// where row q - 1's entries of chunk ch begin (s = 0: cosines, 1: sines).  In
+// fp32 a warp reads both of one chunk, in fp64 one of up to four chunks: beside
+// one another they meet no bank twice (fp64 beside as in fp32: 366 points, 90
+// columns 54 us, 41 so)
+template <typename R>
+__host__ __device__ constexpr int tab_at(int nch, int ch, int s) {
+    return sizeof(R) == 4 ? ch * kChunk + s * kPC : (s * nch + ch) * kPC;
+}
+
+template <typename R> __host__ __device__ constexpr int dense_ct() { return sizeof(R) == 4 ? 2 : 1; }   // columns per thread
 
 template <typename R>
 struct DenseArgs {
     cplx<R>* data;
     const cplx<R>* tw;    // W_n^t, t < n
-    const R* tab;         // [H][2][ld]: cos, sin of 2 pi p q / m (row q = m/2 of an even m holds halves)
-    int n, r1, m, H, ld, nch;
+    const R* tab;         // [H] rows of cos, sin of 2 pi p q / m (tab_at)
+    int n, r1, m, H, nch;
     size_t es, os;
     int ncols, ntiles, cwl, inv;
     long long ntot;
@@ -56,9 +67,24 @@ struct DenseArgs {
     int sz, sb;
 };
 
-// One work item: the output pairs p0 .. p0 + 7 of the m-point DFT of CT
-// columns whose inputs are S[q * CW + t * half]; A and B above per pair.
-template <typename R, int CT> struct DenseAcc { cplx<R> a[CT][kPC], b[CT][kPC]; };
+// fp32: bits of a thread's number within its work items: the low lhb (at most
+// four) bits of its columns, the half (A or B), the rest of the columns.
+struct ItemBits {
+    int lgh, lhb;     // log2 of the columns per thread row, of those beside one another in a warp
+    __device__ __forceinline__ explicit ItemBits(int cwl) : lgh(cwl - 1), lhb(lgh < 4 ? lgh : 4) {}
+    __device__ __forceinline__ bool second(int u) const { return (u >> lhb) & 1; }
+    // its t-th column in the tile (a B lane has them in the other order: of the
+    // halves of a row that each kind reads, no bank twice)
+    __device__ __forceinline__ int column(int u, int t) const {
+        return ((u & ((1 << lhb) - 1)) | (((u >> (lhb + 1)) & ((1 << (lgh - lhb)) - 1)) << lhb)) +
+               ((second(u) ? 1 - t : t) << lgh);
+    }
+};
+template <typename R>
+__device__ __forceinline__ int column_of(int cwl, int u, int t) {
+    if constexpr (sizeof(R) == 4) return ItemBits(cwl).column(u, t);
+    else return u & ((1 << cwl) - 1);
+}
 
 // eight table entries as 16-byte words
 __device__ __forceinline__ void load8(const float* t, float (&v)[8]) {
@@ -74,67 +100,140 @@ __device__ __forceinline__ void load8(const double* t, double (&v)[8]) {
     }
 }
 
-template <typename R, int CT>
-__device__ __forceinline__ void dense_dot(const cplx<R>* S, int CW, int half, int m, int H, const R* tab, int ld,
-                                          DenseAcc<R, CT>& o) {
-#pragma unroll
-    for (int t = 0; t < CT; ++t)
-#pragma unroll
-        for (int k = 0; k < kPC; ++k) o.a[t][k] = o.b[t][k] = mk<R>(R(0), R(0));
-    const cplx<R>* lo = S + CW;
-    const cplx<R>* hi = S + (m - 1) * CW;
+// One half of an fp32 work item: x_0 + A_p (tab the cosines, S the sums x_q +
+// x_(m-q), o = x_0) or -i B_p (the sines, S the differences times -i, o = 0)
+// above for p = p0 .. p0 + 7 and the columns S, S + cs, added to o; rows of S
+// and tab are rs and ts apart.  Sums of 16
+// terms that are then added up: one running sum over m / 2 terms had up to 2.4
+// times the largest error of transforms in short radices (241 points); so the
+// rms error is 0.5 to 0.9 and the largest error 0.4 to 1.0 of theirs at the
+// primes from 17 to 257 (1.1 at 89).
+constexpr int kSumBlock = 16;
+
+__device__ __forceinline__ void dense_sums(const float2* S, int rs, int cs, int H, const float* tab, int ts,
+                                           float2 (&o)[2][kPC]) {
+    const float2* S1 = S + cs;
 #pragma unroll 1
-    for (int q = 1; q <= H; ++q, lo += CW, hi -= CW, tab += 2 * ld) {
-        cplx<R> p[CT], d[CT];
+    for (int q = 0; q < H; q += kSumBlock) {
+        const int n = min(kSumBlock, H - q);
+        float2 a[2][kPC];
+        auto term = [&](auto first) {
+            float w[kPC];
+            load8(tab, w);
+            const float2 x[2] = {*S, *S1};
 #pragma unroll
-        for (int t = 0; t < CT; ++t) {
-            const cplx<R> u = lo[t * half], v = hi[t * half];
-            p[t] = u + v;
-            d[t] = u - v;
-        }
-        R w[kPC];
-        load8(tab, w);
+            for (int t = 0; t < 2; ++t)
 #pragma unroll
-        for (int t = 0; t < CT; ++t)
+                for (int k = 0; k < kPC; ++k) {
+                    if constexpr (decltype(first)::value) a[t][k] = x[t] * w[k];
+                    else fma_rc(a[t][k], w[k], x[t]);
+                }
+            S += rs;
+            S1 += rs;
+            tab += ts;
+        };
+        term(std::true_type{});
+#pragma unroll 5
+        for (int e = 1; e < n; ++e) term(std::false_type{});
 #pragma unroll
-            for (int k = 0; k < kPC; ++k) fma_rc(o.a[t][k], w[k], p[t]);
-        load8(tab + ld, w);
+        for (int t = 0; t < 2; ++t)
 #pragma unroll
-        for (int t = 0; t < CT; ++t)
-#pragma unroll
-            for (int k = 0; k < kPC; ++k) fma_rc(o.b[t][k], w[k], d[t]);
+            for (int k = 0; k < kPC; ++k) o[t][k] += a[t][k];
     }
 }
 
-// The m-point DFTs of every sub-line p1 < r1 of the tile S ([r1][m][CW]);
-// put(t, p1, output index, value) takes each output once, t the thread's
-// column (threadIdx mod half + t half).
-template <typename R, typename Put>
-__device__ __forceinline__ void dense_pass(const cplx<R>* S, const DenseArgs<R>& a, const R* tab, bool inv, Put&& put) {
-    constexpr int CT = dense_ct<R>();
-    const int CW = 1 << a.cwl, half = CW / CT;
-    const int lgh = a.cwl - (CT == 2 ? 1 : 0);
-    const int items = (a.r1 * a.nch) << lgh;
-    for (int u = threadIdx.x; u < items; u += blockDim.x) {
-        const int c = u & (half - 1);
-        const int w = u >> lgh;
-        const int p1 = w / a.nch, p0 = (w - p1 * a.nch) * kPC;
-        const cplx<R>* Sp = S + p1 * a.m * CW + c;
-        DenseAcc<R, CT> o;
-        dense_dot<R, CT>(Sp, CW, half, a.m, a.H, tab + p0, a.ld, o);
+// The m-point DFTs of every sub-line p1 < r1 of the tile S ([r1][m][CW]; fp32:
+// of each sub-line x_0, then x_q + x_(m-q) at q <= m / 2, -i (x_q - x_(m-q)) at
+// m - q); put(t, p1, output index, value) takes each output once, t the
+// thread's column (column_of).  (The block is a multiple of CW threads: a
+// thread's columns, and its half, are the same in every round.)
+//
+// fp32: a work item is eight output pairs of two columns, its A and its B in
+// two lanes of a warp (so that the sums and block sums of one of them fit in a
+// thread's registers): they exchange their sums, and the A lane puts y_p, the
+// B lane y_(m-p).
+template <typename Put>
+__device__ __forceinline__ void dense_pass(const float2* S, const DenseArgs<float>& a, const float* tab, bool inv,
+                                           Put&& put) {
+    const int CW = 1 << a.cwl, half = CW / 2;
+    const ItemBits ib(a.cwl);
+    const bool second = ib.second(threadIdx.x);
+    const float sg = second ? -1.0f : 1.0f;
+    const int items = (a.r1 * a.nch) << a.cwl;
+    for (int u0 = 0; u0 < items; u0 += blockDim.x) {
+        const int u = u0 + threadIdx.x;
+        const bool act = u < items;
+        const int w = act ? u >> a.cwl : 0;
+        const int p1 = w / a.nch, ch = w - p1 * a.nch, p0 = ch * kPC;
+        const float2* Sp = S + p1 * a.m * CW;
+        float2 o[2][kPC];
 #pragma unroll
-        for (int t = 0; t < CT; ++t) {
-            const cplx<R> x0 = Sp[t * half];
+        for (int t = 0; t < 2; ++t) {
+            const float2 x0 = second ? make_float2(0.0f, 0.0f) : Sp[ib.column(threadIdx.x, t)];
+#pragma unroll
+            for (int k = 0; k < kPC; ++k) o[t][k] = x0;
+        }
+        if (act)
+            dense_sums(Sp + (second ? a.m - 1 : 1) * CW + ib.column(threadIdx.x, 0), second ? -CW : CW,
+                       second ? -half : half, a.H, tab + tab_at<float>(a.nch, ch, second), a.nch * kChunk, o);
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
 #pragma unroll
             for (int k = 0; k < kPC; ++k) {
                 const int p = p0 + k;
-                if (p > a.H) continue;
-                const cplx<R> e = x0 + o.a[t][k], f = o.b[t][k];
-                const cplx<R> y = mk<R>(e.x + f.y, e.y - f.x), z = mk<R>(e.x - f.y, e.y + f.x);
+                // (1 - t: the other lane's number of this column)
+                const float2 v = make_float2(__shfl_xor_sync(0xffffffffu, o[1 - t][k].x, 1 << ib.lhb),
+                                             __shfl_xor_sync(0xffffffffu, o[1 - t][k].y, 1 << ib.lhb));
                 const int pr = p == 0 ? 0 : a.m - p;     // the mirrored output (itself for p = 0 and p = m / 2)
-                put(t, p1, inv ? pr : p, y);
-                if (pr != p) put(t, p1, inv ? p : pr, z);
+                if (!act || p > a.H || (second && pr == p)) continue;
+                // y_p = (x_0 + A) + (-i B), y_(m-p) = (x_0 + A) - (-i B)
+                put(t, p1, inv == second ? p : pr, make_float2(fmaf(sg, o[t][k].x, v.x), fmaf(sg, o[t][k].y, v.y)));
             }
+        }
+    }
+}
+
+// fp64: a work item is eight output pairs of one column, A and B together in
+// one running sum each: its rms error is 0.3 to 0.5 of that of transforms in
+// short radices whose twiddles come from angles rounded to 64 bits.
+template <typename Put>
+__device__ __forceinline__ void dense_pass(const double2* S, const DenseArgs<double>& a, const double* tab, bool inv,
+                                           Put&& put) {
+    const int CW = 1 << a.cwl;
+    const int items = (a.r1 * a.nch) << a.cwl;
+    for (int u = threadIdx.x; u < items; u += blockDim.x) {
+        const int w = u >> a.cwl;
+        const int p1 = w / a.nch, ch = w - p1 * a.nch, p0 = ch * kPC;
+        const double2* Sp = S + p1 * a.m * CW + (u & (CW - 1));
+        double2 A[kPC], B[kPC];
+#pragma unroll
+        for (int k = 0; k < kPC; ++k) A[k] = B[k] = make_double2(0.0, 0.0);
+        const double2* lo = Sp + CW;
+        const double2* hi = Sp + (a.m - 1) * CW;
+        const double* tq = tab + tab_at<double>(a.nch, ch, 0);
+        const int sines = tab_at<double>(a.nch, ch, 1) - tab_at<double>(a.nch, ch, 0);
+#pragma unroll 1
+        for (int q = 1; q <= a.H; ++q, lo += CW, hi -= CW, tq += a.nch * kChunk) {
+            const double2 x = *lo + *hi, y = *lo - *hi;
+            double v[kPC];
+            load8(tq, v);
+#pragma unroll
+            for (int k = 0; k < kPC; ++k) fma_rc(A[k], v[k], x);
+            load8(tq + sines, v);
+#pragma unroll
+            for (int k = 0; k < kPC; ++k) fma_rc(B[k], v[k], y);
+        }
+        const double2 x0 = *Sp;
+#pragma unroll
+        for (int k = 0; k < kPC; ++k) {
+            const int p = p0 + k;
+            if (p > a.H) continue;
+            const double2 e = x0 + A[k], f = B[k];
+            const double2 y = make_double2(e.x + f.y, e.y - f.x), z = make_double2(e.x - f.y, e.y + f.x);
+            const int pr = p == 0 ? 0 : a.m - p;
+            put(0, p1, inv ? pr : p, y);
+            if (pr != p) put(0, p1, inv ? p : pr, z);
         }
     }
 }
@@ -163,28 +262,28 @@ __device__ __forceinline__ void line_of(long long f, long long ntot, int ncols, 
 // product, left half the warps: 601 us against 555 for a 109-point pass
 // of 497 MB.  Forward, scale and inverse in one launch needs the outputs of a
 // whole tile in registers or a second tile: 2010 us at 109 points where two
-// launches take 1245.)
+// launches take 1247.)
 template <typename R, bool SCALED, bool TS, int KIND>
 __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_dense(DenseArgs<R> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int CW = 1 << a.cwl;
     cplx<R>* S = reinterpret_cast<cplx<R>*>(smem_raw);                   // [n][CW]
     R* tabS = reinterpret_cast<R*>(S + size_t(a.n) * CW);
-    cplx<R>* T = reinterpret_cast<cplx<R>*>(tabS + (TS ? imax(1, a.H) * 2 * a.ld : 0));   // [n], r1 > 1
+    cplx<R>* T = reinterpret_cast<cplx<R>*>(tabS + (TS ? imax(1, a.H) * a.nch * kChunk : 0));   // [n], r1 > 1
     const int c = threadIdx.x & (CW - 1);
     const int lane = threadIdx.x >> a.cwl, lanes = blockDim.x >> a.cwl;
-    constexpr int CT = dense_ct<R>();
-    const int half = CW / CT;
     const bool inv = a.inv != 0;
     // (the tables are older than any launch of this stream)
     if (TS && KIND != 2) {
-        const int nt = imax(1, a.H) * 2 * a.ld * int(sizeof(R)) / 16;
+        const int nt = imax(1, a.H) * a.nch * kChunk * int(sizeof(R)) / 16;
         const double2* g = reinterpret_cast<const double2*>(a.tab);
         for (int t = threadIdx.x; t < nt; t += blockDim.x) copy_async<double>(reinterpret_cast<double2*>(tabS) + t, g + t, true);
     }
     if (KIND != 0)
         for (int t = threadIdx.x; t < a.n; t += blockDim.x) copy_async<R>(T + t, a.tw + t, true);
     const R* tab = TS ? tabS : a.tab;
+    // fp32: the product's inputs are sums and differences of pairs of rows
+    constexpr bool FOLD = sizeof(R) == 4 && KIND != 2;
     chain_wait();
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
         const long long f0 = (long long)tile << a.cwl;
@@ -194,19 +293,36 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
             if (live) line_of(f0 + c, a.ntot, a.ncols, o, cc);
             const cplx<R>* line = a.data + size_t(o) * a.os + cc;
             const size_t es = live ? a.es : 0;
-            for (int e = lane; e < a.n; e += lanes) copy_async<R>(S + e * CW + c, line + size_t(e) * es, live);
+            if (FOLD && KIND == 0) {   // a thread copies the rows that it pairs
+                for (int e = lane; e <= a.H; e += lanes) {
+                    copy_async<R>(S + e * CW + c, line + size_t(e) * es, live);
+                    if (e && 2 * e < a.m) copy_async<R>(S + (a.m - e) * CW + c, line + size_t(a.m - e) * es, live);
+                }
+            } else {
+                for (int e = lane; e < a.n; e += lanes) copy_async<R>(S + e * CW + c, line + size_t(e) * es, live);
+            }
         }
         // a successor that is scheduled earlier takes slots from work on other
         // streams for as long as this CTA's tiles last
         if (tile + gridDim.x >= a.ntiles) chain_release();
         copy_async_wait();
+        // rows q and m - q of a column: their sum, and -i times their difference
+        auto fold = [&](cplx<R>* col, int q) {
+            cplx<R>&u = col[q * CW], &v = col[(a.m - q) * CW];
+            const cplx<R> x = u, y = v;
+            u = x + y;
+            v = mk<R>(x.y - y.y, y.x - x.x);
+        };
+        if constexpr (FOLD && KIND == 0)
+            for (int e = lane ? lane : lanes; 2 * e < a.m; e += lanes) fold(S + c, e);
         __syncthreads();
         if constexpr (KIND != 0) {
-            // radix-r1 butterflies over x[j + q m], times W_n^(j p), in place: S[p][j]
+            // radix-r1 butterflies over x[j + q m], times W_n^(j p), in place:
+            // S[p][j] (FOLD: of the pair j, m - j the sum and the difference)
             radix_dispatch<16>(a.r1, [&](auto rc) {
                 constexpr int RAD = decltype(rc)::value;
                 if constexpr (RAD > 1) {
-                    for (int j = lane; j < a.m; j += lanes) {
+                    auto butterfly = [&](int j) {
                         cplx<R> x[RAD];
 #pragma unroll
                         for (int q = 0; q < RAD; ++q) x[q] = S[(j + q * a.m) * CW + c];
@@ -218,6 +334,19 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
                             cplx<R> w = T[j * p];
                             if (inv) w.y = -w.y;
                             S[(p * a.m + j) * CW + c] = k == 0 ? x[k] : x[k] * w;
+                        }
+                    };
+                    if constexpr (!FOLD) {
+                        for (int j = lane; j < a.m; j += lanes) butterfly(j);
+                    } else {
+                        for (int j = lane; j <= a.H; j += lanes) {
+                            const bool pair = j && 2 * j < a.m;
+#pragma unroll 1
+                            for (int h = 0; h <= int(pair); ++h) butterfly(h ? a.m - j : j);
+                            if (pair) {
+#pragma unroll 2
+                                for (int p = 0; p < RAD; ++p) fold(S + p * a.m * CW + c, j);
+                            }
                         }
                     }
                 }
@@ -248,19 +377,19 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
                 });
         } else {
             // the columns of this thread's work items
-            cplx<R>* oline[CT];
-            bool olive[CT];
-            const R* osc[CT];
+            cplx<R>* oline[dense_ct<R>()];
+            bool olive[dense_ct<R>()];
+            const R* osc[dense_ct<R>()];
 #pragma unroll
-            for (int t = 0; t < CT; ++t) {
-                const long long g = f0 + (threadIdx.x & (half - 1)) + t * half;
+            for (int t = 0; t < dense_ct<R>(); ++t) {
+                const long long g = f0 + column_of<R>(a.cwl, threadIdx.x, t);
                 olive[t] = g < a.ntot;
                 int go = 0, gc = 0;
                 if (olive[t]) line_of(g, a.ntot, a.ncols, go, gc);
                 oline[t] = a.data + size_t(go) * a.os + gc;
                 osc[t] = SCALED ? a.sc + size_t(go) * a.sz + gc / a.sb : nullptr;
             }
-            dense_pass<R>(S, a, tab, inv, [&](int t, int p1, int p, cplx<R> v) {
+            dense_pass(S, a, tab, inv, [&](int t, int p1, int p, cplx<R> v) {
                 if (!olive[t]) return;
                 const int e = p1 + a.r1 * p;
                 if constexpr (SCALED) v = v * osc[t][size_t(e) * a.estep];
@@ -270,6 +399,10 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
         __syncthreads();   // the tile's buffer is free
     }
 }
+
+constexpr size_t kDenseSmemMax = 220 * 1024;
+
+}  // namespace
 
 int sm_count() {
     static const int sms = [] {
@@ -281,10 +414,6 @@ int sm_count() {
     return sms;
 }
 
-constexpr size_t kDenseSmemMax = 220 * 1024;
-
-}  // namespace
-
 // Tables longer than this stay in global memory (L1): m above 131.
 constexpr size_t kDenseTableSmem = 72 * 1024;
 
@@ -294,21 +423,30 @@ void DenseDFT::init(int n, int r1) {
     n_ = n;
     if (!r1) return;
     H_ = m_ / 2;
-    ld_ = (H_ + 1 + kPC - 1) / kPC * kPC;
-    std::vector<double> t(size_t(std::max(1, H_)) * 2 * ld_, 0.0);
-    for (int q = 1; q <= H_; ++q) {
-        const double f = 2 * q == m_ ? 0.5 : 1.0;     // x_q + x_(m-q) counts the middle input twice
-        for (int p = 0; p <= H_; ++p) {
-            const double w = 2.0 * kPi * double((long long)p * q % m_) / m_;
-            t[(size_t(q - 1) * 2) * ld_ + p] = f * std::cos(w);
-            t[(size_t(q - 1) * 2 + 1) * ld_ + p] = 2 * q == m_ ? 0.0 : std::sin(w);
-        }
+    nch_ = (H_ + 1 + kPC - 1) / kPC;
+    // (an angle rounded to 64 bits would cost the fp64 tables a digit)
+    std::vector<double> c(m_), d(m_);
+    for (int j = 0; j < m_; ++j) {
+        const long double w = 2.0L * kPiL * j / m_;
+        c[j] = double(std::cos(w));
+        d[j] = double(std::sin(w));
     }
-    std::vector<float> tf(t.begin(), t.end());
-    t64_.ensure(sizeof(double) * t.size());
-    t32_.ensure(sizeof(float) * tf.size());
-    upload(t64_.p, t.data(), sizeof(double) * t.size());
-    upload(t32_.p, tf.data(), sizeof(float) * tf.size());
+    auto fill = [&](auto zero, DevBuf& buf) {
+        using R = decltype(zero);
+        std::vector<R> t(size_t(std::max(1, H_)) * nch_ * kChunk, zero);
+        for (int q = 1; q <= H_; ++q)
+            for (int p = 0; p <= H_; ++p) {
+                const size_t j = size_t(p) * q % m_;
+                R* e = t.data() + size_t(q - 1) * nch_ * kChunk + p % kPC;
+                // (in fp64 the middle row of an even m meets itself as a pair)
+                e[tab_at<R>(nch_, p / kPC, 0)] = R(sizeof(R) == 8 && 2 * q == m_ ? 0.5 * c[j] : c[j]);
+                e[tab_at<R>(nch_, p / kPC, 1)] = 2 * q == m_ ? zero : R(d[j]);
+            }
+        buf.ensure(sizeof(R) * t.size());
+        upload(buf.p, t.data(), sizeof(R) * t.size());
+    };
+    fill(0.0, t64_);
+    fill(0.0f, t32_);
 }
 
 bool DenseDFT::fits(bool fp64) const {
@@ -330,41 +468,54 @@ void DenseDFT::run(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, size_
 template <typename R>
 void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, size_t os, int nouter, bool inverse,
                       const R* scale, int sz, int sb, cudaStream_t s) const {
-    constexpr int CT = dense_ct<R>();
     DenseArgs<R> a{};
     a.data = data;
     a.tw = tw;
     a.tab = sizeof(R) == 4 ? reinterpret_cast<const R*>(t32_.p) : reinterpret_cast<const R*>(t64_.p);
-    a.n = n_; a.r1 = r1_; a.m = m_; a.H = H_; a.ld = ld_; a.nch = ld_ / kPC;
+    a.n = n_; a.r1 = r1_; a.m = m_; a.H = H_; a.nch = nch_;
     a.es = es; a.os = os; a.ncols = ncols; a.inv = inverse;
     a.ntot = (long long)nouter * ncols;
     a.sc = scale;
     a.estep = size_t(nouter) * sz;
     a.sz = sz;
     a.sb = sb;
-    const size_t tabb = sizeof(R) * size_t(std::max(1, H_)) * 2 * ld_;
+    const size_t tabb = sizeof(R) * size_t(std::max(1, H_)) * nch_ * kChunk;
     const size_t twb = r1_ > 1 ? sizeof(cplx<R>) * size_t(n_) : 0;
     const size_t per_col = size_t(n_) * sizeof(cplx<R>);
     const bool radix2 = r1_ > 1 && m_ <= 16;       // no table
     const bool ts = !radix2 && tabb <= kDenseTableSmem && (per_col << 2) + tabb + twb <= kDenseSmemMax;
     auto smem = [&](int cwl) { return (per_col << cwl) + (ts ? tabb : 0) + twb; };
-    auto items = [&](int cwl) { return a.r1 * a.nch * ((1 << cwl) / CT); };
+    // threads: a work item (fp32: the A or B of one) each
+    auto items = [&](int cwl) { return a.r1 * a.nch << cwl; };
     // columns per tile: 64 (fp64: 32), so that a warp's lanes are the columns
     // of one p range and read its table entries as one word; fewer while the
-    // SM would not hold two CTAs, whose copies and products overlap, or the
+    // SM would not hold `ctas` CTAs, whose copies and products overlap, or the
     // tiles would not cover two per SM (few columns in all)
-    int cwl = sizeof(R) == 4 ? 6 : 5;
+    auto widest = [&](int ctas) {
+        int l = sizeof(R) == 4 ? 6 : 5;
+        while (l > 2 && (smem(l) > size_t(224 * 1024 / ctas) || (a.ntot >> l) < 2 * sm_count())) --l;
+        return l;
+    };
+    int maxthr = kDenseMaxThreads, cwl = widest(dense_ctas<R>(radix2));
     const int regs = 256 / dense_ctas<R>(radix2);
-    while (cwl > 2 && (smem(cwl) > size_t(224 * 1024 / dense_ctas<R>(radix2)) || (a.ntot >> cwl) < 2 * sm_count())) --cwl;
+    // four CTAs of 128 threads instead of two of 256 where their tiles, of
+    // eight columns at least, are no smaller than the tables beside them
+    // (109-point pass of 48 columns, fp32: 558 us against 597; 366 points, 90
+    // columns: 34 against 37; with four
+    // columns per tile 151 points would take 145 against 93)
+    if (const int l = widest(4); sizeof(R) == 4 && !radix2 && l > 2 && smem(l) <= 56 * 1024 && (per_col << l) >= (ts ? tabb : 0)) {
+        cwl = l;
+        maxthr = 128;
+    }
     const size_t shm = smem(cwl);
     if (shm > kDenseSmemMax) throw std::runtime_error("FFT line does not fit in shared memory");
     a.cwl = cwl;
     a.ntiles = int((a.ntot + (1ll << cwl) - 1) >> cwl);
     // threads: the work items in equal rounds, a whole number of column rows
-    const int it = radix2 ? r1_ << cwl : items(cwl), rounds = (it + kDenseMaxThreads - 1) / kDenseMaxThreads;
+    const int it = radix2 ? r1_ << cwl : items(cwl), rounds = (it + maxthr - 1) / maxthr;
     const int unit = std::max(32, 1 << cwl);
     int nt = ((it + rounds - 1) / rounds + unit - 1) / unit * unit;
-    nt = std::min(kDenseMaxThreads, std::max(nt, 128));   // the copies and radix pass use them all
+    nt = std::min(maxthr, std::max(nt, 128));   // the copies and radix pass use them all
     // resident CTAs; each stays for its share of the tiles
     const int per_sm = std::max(1, std::min({int(227 * 1024 / (shm + 1024)), 65536 / (regs * nt), 16}));
     const int grid = std::min(a.ntiles, per_sm * sm_count());

@@ -30,6 +30,9 @@ struct FftFactors {
     int pt_total = 0;     // entries of all tables together
 };
 
+// SMs of the first device used (the rules that share work between CTAs)
+int sm_count();
+
 // Line transform of n = r1 * m points by an in-register radix-r1 pass and
 // m-point DFTs as products with their tables (mpm_dense.cu).  r1 = 0: off.
 class DenseDFT {
@@ -46,8 +49,8 @@ private:
     template <typename R>
     void launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, size_t os, int nouter, bool inverse,
                 const R* scale, int sz, int sb, cudaStream_t s) const;
-    int n_ = 0, r1_ = 0, m_ = 0, H_ = 0, ld_ = 0;
-    DevBuf t64_, t32_;   // [H][2][ld]: cos, sin of 2 pi p q / m
+    int n_ = 0, r1_ = 0, m_ = 0, H_ = 0, nch_ = 0;
+    DevBuf t64_, t32_;   // cosines and sines of 2 pi p q / m, see mpm_dense.cu
 };
 
 class AxisFFT {
@@ -74,8 +77,8 @@ public:
     void set_force_general(bool v) { force_general_ = v; }
     // kernel a transform of ncols columns takes: 1 two-pass in registers (both
     // factors in-register radices, at least half a tile of columns per line),
-    // 2 in-register radix times table product (mpm_dense.cu: lengths with one
-    // prime above 16, few columns per line, other lengths with a short rest),
+    // 2 in-register radix times table product or a second one (mpm_dense.cu:
+    // lengths with one prime above 16, two radices with few columns per line),
     // 0 general multi-pass
     int path(int ncols, bool fp64) const {
         if (force_general_) return 0;
