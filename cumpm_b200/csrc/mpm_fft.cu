@@ -759,6 +759,8 @@ void AxisFFT::init(int n) {
     // as fast or faster, 8.9 us against 19.4 for 300 points, 9 columns and 80
     // lines, and its largest errors smaller)
     dense_.init(n, r1_);
+    const std::pair<int, int> ab = kind_ == 2 ? fft2_split(r2_ - 1) : std::pair<int, int>{0, 0};
+    rader_.init(n, r1_, r2_, ab.first, ab.second);
 }
 
 void AxisFFT::upload_table(std::vector<double2> t64, DevBuf& d64, DevBuf& d32) {
@@ -783,7 +785,11 @@ void AxisFFT::launch_line(cplx<R>* data, size_t es, int ncols, size_t os, int no
     ks.sb = sb;
     const cplx<R>* tw = sizeof(R) == 4 ? reinterpret_cast<const cplx<R>*>(tw32_.p)
                                        : reinterpret_cast<const cplx<R>*>(tw64_.p);
-    const int kind = path(ncols, sizeof(R) == 8);
+    const int kind = path(ncols, sizeof(R) == 8, mode);
+    if (kind == 3) {
+        rader_.run<R>(data, tw, es, ncols, os, nouter, mode == 1, s);
+        return;
+    }
     if (kind == 2) {
         dense_.run<R>(data, tw, es, ncols, os, nouter, mode, scale, sz, sb, s);
         return;

@@ -53,6 +53,24 @@ private:
     DevBuf t64_, t32_;   // cosines and sines of 2 pi p q / m, see mpm_dense.cu
 };
 
+// Line transform of n = r1 * p points, p a prime with p - 1 = A * B, by an
+// in-register radix-r1 pass and Rader's convolution (mpm_rader.cu).
+class RaderDFT {
+public:
+    void init(int n, int r1, int p, int A, int B);
+    // false: not set up (A = 0, or a tile does not fit in shared memory)
+    bool usable() const { return n_ != 0; }
+    // as AxisFFT::run
+    template <typename R>
+    void run(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, size_t os, int nouter, bool inverse,
+             cudaStream_t s) const;
+
+private:
+    int n_ = 0, r1_ = 0, p_ = 0, a_ = 0, b_ = 0;
+    DevBuf t64_, t32_;   // W_N^t, N = p - 1, then the forward and the inverse Bh
+    DevBuf perm_;        // g^-q, then g^m
+};
+
 class AxisFFT {
 public:
     void init(int n);
@@ -79,10 +97,13 @@ public:
     // factors in-register radices, at least half a tile of columns per line),
     // 2 in-register radix times table product or a second one (mpm_dense.cu:
     // lengths with one prime above 16, two radices with few columns per line),
-    // 0 general multi-pass
-    int path(int ncols, bool fp64) const {
+    // 3 in-register radix and Rader's convolution (mpm_rader.cu: one prime too
+    // long for the product, at least half a tile of columns per line, no
+    // fused scale), 0 general multi-pass
+    int path(int ncols, bool fp64, int mode) const {
         if (force_general_) return 0;
         if (kind_ == 1 && ncols >= 16) return 1;
+        if (kind_ == 2 && ncols >= 16 && mode != 2 && rader_.usable() && rader_faster(fp64)) return 3;
         return dense_.fits(fp64) ? 2 : 0;
     }
     // the split as mpm_line_fft reports it
@@ -116,11 +137,21 @@ private:
                      int sb, cudaStream_t s) const;
     static void upload_table(std::vector<double2> t64, DevBuf& d64, DevBuf& d32);
     FftFactors f_;
+    // the length's own split n = r1 * r2: kind 1 both in-register radices (r1 >=
+    // r2), kind 2 r1 in-register and r2 a prime above 16; (0, 0) if neither
     int kind_ = 0, r1_ = 0, r2_ = 0;
     bool force_general_ = false;
     DevBuf tw64_, tw32_;
     DevBuf pt64_, pt32_;   // prime-pass twiddle tables (see FftFactors)
     DenseDFT dense_;
+    RaderDFT rader_;
+    // The product's m FMAs per element against Rader's fixed cost (us per pass
+    // of 46 MB, product and Rader: fp64 127 points 58 and 91, 131 113 and 89,
+    // 257 211 and 84; fp32 181 points 88 and 139, 197 136 and 138, 211 160 and
+    // 139, 257 177 and 131; 2 * 157 points 99 and 100, 2 * 181 104 and 98,
+    // 2 * 193 142 and 93).  With the fused scale the product's two launches
+    // are the faster ones (181 points, fp32: 200 and 2 x 139).
+    bool rader_faster(bool fp64) const { return fp64 ? r2_ > 128 : r2_ > 200 || (r1_ > 1 && r2_ > 180); }
 };
 
 }  // namespace mpm
