@@ -562,9 +562,9 @@ int mpm_line_fft(void* data, int fp64, int n, size_t es, int ncols, size_t os, i
         fft.init(n);
         fft.set_force_general(general != 0);
         if (split) {
-            const bool two = fft.reports_split(ncols, mode);
-            split[0] = two ? fft.split_r1() : 0;
-            split[1] = two ? fft.split_r2() : 0;
+            const auto sp = fft.split(ncols, fp64 != 0, mode);
+            split[0] = sp.first;
+            split[1] = sp.second;
         }
         const auto st = static_cast<cudaStream_t>(stream);
         if (fp64) {

@@ -87,10 +87,6 @@ public:
                     cudaStream_t s) const;
     // whether one line of this length fits in shared memory
     static bool fits(int n, bool fp64);
-    // the split n = r1 * r2: both in-register radices (r1 >= r2), or r1
-    // in-register and r2 a prime above 16; (0, 0) if neither
-    int split_r1() const { return r1_; }
-    int split_r2() const { return r2_; }
     // run every length through the general multi-pass kernel (tests)
     void set_force_general(bool v) { force_general_ = v; }
     // kernel a transform of ncols columns takes: 1 two-pass in registers (both
@@ -106,9 +102,10 @@ public:
         if (kind_ == 2 && ncols >= 16 && mode != 2 && rader_.usable() && rader_faster(fp64)) return 3;
         return dense_.fits(fp64) ? 2 : 0;
     }
-    // the split as mpm_line_fft reports it
-    bool reports_split(int ncols, int mode) const {
-        return r1_ && !force_general_ && ncols >= 16 && !(kind_ == 2 && mode == 2);
+    // the split of the kernel that such a transform takes, (0, 0) for the
+    // general one
+    std::pair<int, int> split(int ncols, bool fp64, int mode) const {
+        return path(ncols, fp64, mode) ? std::pair<int, int>{r1_, r2_} : std::pair<int, int>{0, 0};
     }
 
     // The k-space step of the pruned (z-slab) monodisperse grid fused with

@@ -1,7 +1,7 @@
 """The in-house batched line DFT (the grid transform of the spectral-Ewald
 fields, replacing the reference's cuFFT plans) against numpy's FFT, through
-the C-ABI entry mpm_line_fft: both kernels (two-pass in-register and general
-multi-pass), both precisions, forward, inverse and the fused
+the C-ABI entry mpm_line_fft: the length's own kernels and the general
+multi-pass one, both precisions, forward, inverse and the fused
 forward-scale-inverse pass, for the line layouts the fields use (lines
 contiguous: z axis; lines strided across the outer index: x axis)."""
 import numpy as np
@@ -11,11 +11,9 @@ torch = pytest.importorskip("torch")
 
 pytestmark = pytest.mark.gpu
 
-# two-pass splits in registers: 2 = 2x1, 16 = 4x4, 49 = 7x7, 80 = 10x8,
-# 108 = 12x9, 112 = 14x8, 143 = 13x11, 256 = 16x16; with a Rader prime pass
-# (p - 1 = A x B in registers): 34 = 2x17 (16 = 4x4, radix <= 8 class),
-# 97 = 1x97 (96 = 12x8), 238 = 14x17 (16 = 4x4), 366 = 6x61 (60 = 10x6); with
-# a streamed prime pass: 206 = 2x103 (102 has no such split); general only:
+# two radices in registers: 2 = 2x1, 16 = 4x4, 49 = 7x7, 80 = 10x8,
+# 108 = 12x9, 112 = 14x8, 143 = 13x11, 256 = 16x16; a radix and a prime:
+# 34 = 2x17, 97 = 1x97, 206 = 2x103, 238 = 14x17, 366 = 6x61; general only:
 # 289 = 17*17
 LENGTHS = [2, 16, 34, 49, 80, 97, 108, 112, 143, 206, 238, 256, 289, 366]
 SPLITS = {2: (2, 1), 16: (4, 4), 34: (2, 17), 49: (7, 7), 80: (10, 8), 108: (12, 9), 112: (14, 8),
@@ -64,8 +62,6 @@ def test_line_fft_matches_numpy(n, fp64):
                 err, split = run_case(n, layout, 40, 3, fp64, mode, general)
                 assert err < tol, (layout, general, mode, err)
                 want = (0, 0) if general else SPLITS.get(n, (0, 0))
-                if mode == 2 and want[1] > 16:
-                    want = (0, 0)   # the fused pass has no streamed-prime variant
                 assert split == want, (split, want)
 
 
@@ -87,11 +83,13 @@ def test_line_fft_tuner_lengths(n):
 @pytest.mark.parametrize("ncols", [1, 5, 17, 33, 70])
 def test_line_fft_ragged_column_groups(ncols):
     """Column counts that leave the last CTA's column group partly empty, and
-    fewer columns than one group (general kernel below 16 columns)."""
-    for n in (108, 206, 366):
+    fewer columns than one group (the table product and its two-radix form
+    below 16 columns, with the same split)."""
+    for n in (108, 206, 289, 366):
         for mode in (0, 1, 2):
-            err, _ = run_case(n, "x", ncols, 5, True, mode, False, seed=ncols)
+            err, split = run_case(n, "x", ncols, 5, True, mode, False, seed=ncols)
             assert err < 1e-12, (n, mode, err)
+            assert split == SPLITS.get(n, (0, 0)), (n, ncols, mode, split)
 
 
 def test_line_fft_rejects_bad_arguments():
