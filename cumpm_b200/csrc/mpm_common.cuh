@@ -8,6 +8,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <stdexcept>
@@ -107,6 +108,17 @@ __host__ __device__ __forceinline__ int cyc_diff(int a, int b, int n) {
 
 constexpr double kPi = 3.14159265358979323846;
 constexpr long double kPiL = 3.14159265358979323846264338327950288L;   // (host)
+
+// exp(2 pi i j / n), 0 <= j < n, to all digits of a double: from an angle of at
+// most pi / 4 (one of up to 2 pi, rounded to a double, loses three bits)
+inline double2 unit_root(long long j, long long n) {
+    const long long q = 4 * j / n, r = 4 * j - q * n;     // quarters of a turn, and r / n of one
+    const bool hi = 2 * r > n;
+    const double x = double(kPiL / 2 * (hi ? n - r : r) / n);
+    const double c = hi ? std::sin(x) : std::cos(x), s = hi ? std::cos(x) : std::sin(x);
+    return q == 0 ? make_double2(c, s) : q == 1 ? make_double2(-s, c) : q == 2 ? make_double2(-c, -s)
+                                                                               : make_double2(s, -c);
+}
 
 // --------------------------------------------------------------- buffers --
 

@@ -8,15 +8,15 @@
 //   A_p = sum_q (x_q + x_(m-q)) cos(2 pi p q / m),
 //   B_p = sum_q (x_q - x_(m-q)) sin(2 pi p q / m),
 //   y_p = x_0 + A_p - i B_p,  y_(m-p) = x_0 + A_p + i B_p,
-// m real FMAs per element.  A thread holds A or B (fp64: A and B) of eight p
-// and two columns (fp64: one) in registers, so a step over q costs 32 FMAs
-// against 4 (10) shared loads: at one FMA per lane and clock an element of
+// m real FMAs per element.  A thread holds A and B (BLK: A or B) of eight p and
+// two columns (fp64: one) in registers, so a step over q costs 64 (32) FMAs
+// against 8 (4) shared loads: at one FMA per lane and clock an element of
 // m = 109 costs 3 ps of this GPU, against the 2.5 ps that its trip through HBM
 // takes, and m = 53 is bound by that trip.  (Packed fp32 pairs, fma.rn.f32x2,
 // halve the FMA instructions but took more to arrange their operands: slower.)
 // The alternative for primes, Rader's convolution (mpm_rader.cu), needs a
 // quarter of the arithmetic but three more shared round trips and gathers by
-// g^q: 736 us for a 109-point pass of 497 MB (48 fp32 columns) that takes 558
+// g^q: 736 us for a 109-point pass of 497 MB (48 fp32 columns) that takes 515
 // here; see AxisFFT::path for where it is the faster one.
 //
 // Columns are enumerated over lines and columns together (f = line * ncols +
@@ -43,12 +43,12 @@ template <typename R> __host__ __device__ constexpr int dense_ctas(bool radix2) 
 constexpr int kChunk = 2 * kPC;   // eight pairs' table entries: cosines, sines
 
 // where row q - 1's entries of chunk ch begin (s = 0: cosines, 1: sines).  In
-// fp32 a warp reads both of one chunk, in fp64 one of up to four chunks: beside
-// one another they meet no bank twice (fp64 beside as in fp32: 366 points, 90
-// columns 54 us, 41 so)
-template <typename R>
+// blocks (BLK below) a warp reads both of one chunk, else one of up to four
+// chunks: what it reads lies side by side and meets no bank twice (366 points,
+// 90 columns, fp64: 54 us with a chunk's sines behind its cosines, 42 so)
+template <bool BLK>
 __host__ __device__ constexpr int tab_at(int nch, int ch, int s) {
-    return sizeof(R) == 4 ? ch * kChunk + s * kPC : (s * nch + ch) * kPC;
+    return BLK ? ch * kChunk + s * kPC : (s * nch + ch) * kPC;
 }
 
 template <typename R> __host__ __device__ constexpr int dense_ct() { return sizeof(R) == 4 ? 2 : 1; }   // columns per thread
@@ -67,7 +67,7 @@ struct DenseArgs {
     int sz, sb;
 };
 
-// fp32: bits of a thread's number within its work items: the low lhb (at most
+// BLK: bits of a thread's number within its work items: the low lhb (at most
 // four) bits of its columns, the half (A or B), the rest of the columns.
 struct ItemBits {
     int lgh, lhb;     // log2 of the columns per thread row, of those beside one another in a warp
@@ -80,10 +80,11 @@ struct ItemBits {
                ((second(u) ? 1 - t : t) << lgh);
     }
 };
-template <typename R>
+template <typename R, bool BLK>
 __device__ __forceinline__ int column_of(int cwl, int u, int t) {
-    if constexpr (sizeof(R) == 4) return ItemBits(cwl).column(u, t);
-    else return u & ((1 << cwl) - 1);
+    if constexpr (BLK) return ItemBits(cwl).column(u, t);
+    const int half = (1 << cwl) / dense_ct<R>();
+    return (u & (half - 1)) + t * half;
 }
 
 // eight table entries as 16-byte words
@@ -100,22 +101,28 @@ __device__ __forceinline__ void load8(const double* t, double (&v)[8]) {
     }
 }
 
-// One half of an fp32 work item: x_0 + A_p (tab the cosines, S the sums x_q +
+// One half of a blocked work item: x_0 + A_p (tab the cosines, S the sums x_q +
 // x_(m-q), o = x_0) or -i B_p (the sines, S the differences times -i, o = 0)
 // above for p = p0 .. p0 + 7 and the columns S, S + cs, added to o; rows of S
-// and tab are rs and ts apart.  Sums of 16
-// terms that are then added up: one running sum over m / 2 terms had up to 2.4
-// times the largest error of transforms in short radices (241 points); so the
-// rms error is 0.5 to 0.9 and the largest error 0.4 to 1.0 of theirs at the
-// primes from 17 to 257 (1.1 at 89).
-constexpr int kSumBlock = 16;
+// and tab are rs and ts apart.  Sums of some 20 terms that are then added up:
+// one running sum over m / 2 terms had up to 2.4 times the largest error of
+// transforms in short radices (241 points) and 1.4 times their rms error; so
+// both are 0.5 to 0.9 and 0.4 to 1.1 of theirs at the primes from 53 to 257.
+constexpr int kSumBlock = 20;
+// Shorter products are summed at once: up to 47 points the largest error was no
+// larger than that of short radices either, and the split of the work items
+// costs more (43 points, 46 MB: 37 us, 42 in blocks; 53 points, 229 MB: 87 and
+// 92 us, but with 1.2 times the largest error).
+constexpr int kPlainTerms = 24;
+template <typename R> __host__ __device__ constexpr bool blocked(int H) { return sizeof(R) == 4 && H > kPlainTerms; }
 
 __device__ __forceinline__ void dense_sums(const float2* S, int rs, int cs, int H, const float* tab, int ts,
                                            float2 (&o)[2][kPC]) {
     const float2* S1 = S + cs;
+    const int len = H / ((H + kSumBlock - 1) / kSumBlock) + 1;    // blocks of about the same length
 #pragma unroll 1
-    for (int q = 0; q < H; q += kSumBlock) {
-        const int n = min(kSumBlock, H - q);
+    for (int q = 0; q < H; q += len) {
+        const int n = min(len, H - q);
         float2 a[2][kPC];
         auto term = [&](auto first) {
             float w[kPC];
@@ -133,7 +140,8 @@ __device__ __forceinline__ void dense_sums(const float2* S, int rs, int cs, int 
             tab += ts;
         };
         term(std::true_type{});
-#pragma unroll 5
+// (unrolled by 3, 4 and 5: 515, 534 and 540 us for the 109-point pass)
+#pragma unroll 3
         for (int e = 1; e < n; ++e) term(std::false_type{});
 #pragma unroll
         for (int t = 0; t < 2; ++t)
@@ -142,19 +150,19 @@ __device__ __forceinline__ void dense_sums(const float2* S, int rs, int cs, int 
     }
 }
 
-// The m-point DFTs of every sub-line p1 < r1 of the tile S ([r1][m][CW]; fp32:
+// The m-point DFTs of every sub-line p1 < r1 of the tile S ([r1][m][CW]; BLK:
 // of each sub-line x_0, then x_q + x_(m-q) at q <= m / 2, -i (x_q - x_(m-q)) at
 // m - q); put(t, p1, output index, value) takes each output once, t the
 // thread's column (column_of).  (The block is a multiple of CW threads: a
 // thread's columns, and its half, are the same in every round.)
 //
-// fp32: a work item is eight output pairs of two columns, its A and its B in
+// BLK: a work item is eight output pairs of two columns, its A and its B in
 // two lanes of a warp (so that the sums and block sums of one of them fit in a
 // thread's registers): they exchange their sums, and the A lane puts y_p, the
 // B lane y_(m-p).
 template <typename Put>
 __device__ __forceinline__ void dense_pass(const float2* S, const DenseArgs<float>& a, const float* tab, bool inv,
-                                           Put&& put) {
+                                           Put&& put, std::true_type) {
     const int CW = 1 << a.cwl, half = CW / 2;
     const ItemBits ib(a.cwl);
     const bool second = ib.second(threadIdx.x);
@@ -175,7 +183,7 @@ __device__ __forceinline__ void dense_pass(const float2* S, const DenseArgs<floa
         }
         if (act)
             dense_sums(Sp + (second ? a.m - 1 : 1) * CW + ib.column(threadIdx.x, 0), second ? -CW : CW,
-                       second ? -half : half, a.H, tab + tab_at<float>(a.nch, ch, second), a.nch * kChunk, o);
+                       second ? -half : half, a.H, tab + tab_at<true>(a.nch, ch, second), a.nch * kChunk, o);
         __syncwarp();
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
@@ -194,46 +202,62 @@ __device__ __forceinline__ void dense_pass(const float2* S, const DenseArgs<floa
     }
 }
 
-// fp64: a work item is eight output pairs of one column, A and B together in
-// one running sum each: its rms error is 0.3 to 0.5 of that of transforms in
-// short radices whose twiddles come from angles rounded to 64 bits.
-template <typename Put>
-__device__ __forceinline__ void dense_pass(const double2* S, const DenseArgs<double>& a, const double* tab, bool inv,
-                                           Put&& put) {
-    const int CW = 1 << a.cwl;
-    const int items = (a.r1 * a.nch) << a.cwl;
+// One running sum: a work item is eight output pairs of the columns of
+// dense_ct, A and B together.  fp64 (rms error 0.3 to 0.5 of that of transforms
+// in short radices whose twiddles come from angles rounded to 64 bits), and fp32
+// products of at most kPlainTerms terms.
+template <typename R, typename Put>
+__device__ __forceinline__ void dense_pass(const cplx<R>* S, const DenseArgs<R>& a, const R* tab, bool inv, Put&& put,
+                                           std::false_type) {
+    constexpr int CT = dense_ct<R>();
+    const int CW = 1 << a.cwl, half = CW / CT, lgh = a.cwl - (CT == 2 ? 1 : 0);
+    const int items = (a.r1 * a.nch) << lgh;
+    const int sines = tab_at<false>(a.nch, 0, 1);
     for (int u = threadIdx.x; u < items; u += blockDim.x) {
-        const int w = u >> a.cwl;
+        const int w = u >> lgh;
         const int p1 = w / a.nch, ch = w - p1 * a.nch, p0 = ch * kPC;
-        const double2* Sp = S + p1 * a.m * CW + (u & (CW - 1));
-        double2 A[kPC], B[kPC];
+        const cplx<R>* Sp = S + p1 * a.m * CW + (u & (half - 1));
+        cplx<R> A[CT][kPC], B[CT][kPC];
 #pragma unroll
-        for (int k = 0; k < kPC; ++k) A[k] = B[k] = make_double2(0.0, 0.0);
-        const double2* lo = Sp + CW;
-        const double2* hi = Sp + (a.m - 1) * CW;
-        const double* tq = tab + tab_at<double>(a.nch, ch, 0);
-        const int sines = tab_at<double>(a.nch, ch, 1) - tab_at<double>(a.nch, ch, 0);
+        for (int t = 0; t < CT; ++t)
+#pragma unroll
+            for (int k = 0; k < kPC; ++k) A[t][k] = B[t][k] = mk<R>(R(0), R(0));
+        const cplx<R>* lo = Sp + CW;
+        const cplx<R>* hi = Sp + (a.m - 1) * CW;
+        const R* tq = tab + tab_at<false>(a.nch, ch, 0);
 #pragma unroll 1
         for (int q = 1; q <= a.H; ++q, lo += CW, hi -= CW, tq += a.nch * kChunk) {
-            const double2 x = *lo + *hi, y = *lo - *hi;
-            double v[kPC];
+            cplx<R> x[CT], y[CT];
+#pragma unroll
+            for (int t = 0; t < CT; ++t) {
+                x[t] = lo[t * half] + hi[t * half];
+                y[t] = lo[t * half] - hi[t * half];
+            }
+            R v[kPC];
             load8(tq, v);
 #pragma unroll
-            for (int k = 0; k < kPC; ++k) fma_rc(A[k], v[k], x);
+            for (int t = 0; t < CT; ++t)
+#pragma unroll
+                for (int k = 0; k < kPC; ++k) fma_rc(A[t][k], v[k], x[t]);
             load8(tq + sines, v);
 #pragma unroll
-            for (int k = 0; k < kPC; ++k) fma_rc(B[k], v[k], y);
-        }
-        const double2 x0 = *Sp;
+            for (int t = 0; t < CT; ++t)
 #pragma unroll
-        for (int k = 0; k < kPC; ++k) {
-            const int p = p0 + k;
-            if (p > a.H) continue;
-            const double2 e = x0 + A[k], f = B[k];
-            const double2 y = make_double2(e.x + f.y, e.y - f.x), z = make_double2(e.x - f.y, e.y + f.x);
-            const int pr = p == 0 ? 0 : a.m - p;
-            put(0, p1, inv ? pr : p, y);
-            if (pr != p) put(0, p1, inv ? p : pr, z);
+                for (int k = 0; k < kPC; ++k) fma_rc(B[t][k], v[k], y[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < CT; ++t) {
+            const cplx<R> x0 = Sp[t * half];
+#pragma unroll
+            for (int k = 0; k < kPC; ++k) {
+                const int p = p0 + k;
+                if (p > a.H) continue;
+                const cplx<R> e = x0 + A[t][k], f = B[t][k];
+                const cplx<R> y = mk<R>(e.x + f.y, e.y - f.x), z = mk<R>(e.x - f.y, e.y + f.x);
+                const int pr = p == 0 ? 0 : a.m - p;     // the mirrored output (itself for p = 0 and p = m / 2)
+                put(t, p1, inv ? pr : p, y);
+                if (pr != p) put(t, p1, inv ? p : pr, z);
+            }
         }
     }
 }
@@ -262,8 +286,8 @@ __device__ __forceinline__ void line_of(long long f, long long ntot, int ncols, 
 // product, left half the warps: 601 us against 555 for a 109-point pass
 // of 497 MB.  Forward, scale and inverse in one launch needs the outputs of a
 // whole tile in registers or a second tile: 2010 us at 109 points where two
-// launches take 1247.)
-template <typename R, bool SCALED, bool TS, int KIND>
+// launches take 1189.)
+template <typename R, bool SCALED, bool TS, int KIND, bool BLK>
 __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_dense(DenseArgs<R> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int CW = 1 << a.cwl;
@@ -282,8 +306,6 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
     if (KIND != 0)
         for (int t = threadIdx.x; t < a.n; t += blockDim.x) copy_async<R>(T + t, a.tw + t, true);
     const R* tab = TS ? tabS : a.tab;
-    // fp32: the product's inputs are sums and differences of pairs of rows
-    constexpr bool FOLD = sizeof(R) == 4 && KIND != 2;
     chain_wait();
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
         const long long f0 = (long long)tile << a.cwl;
@@ -293,7 +315,7 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
             if (live) line_of(f0 + c, a.ntot, a.ncols, o, cc);
             const cplx<R>* line = a.data + size_t(o) * a.os + cc;
             const size_t es = live ? a.es : 0;
-            if (FOLD && KIND == 0) {   // a thread copies the rows that it pairs
+            if (BLK && KIND == 0) {   // a thread copies the rows that it pairs
                 for (int e = lane; e <= a.H; e += lanes) {
                     copy_async<R>(S + e * CW + c, line + size_t(e) * es, live);
                     if (e && 2 * e < a.m) copy_async<R>(S + (a.m - e) * CW + c, line + size_t(a.m - e) * es, live);
@@ -313,12 +335,12 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
             u = x + y;
             v = mk<R>(x.y - y.y, y.x - x.x);
         };
-        if constexpr (FOLD && KIND == 0)
+        if constexpr (BLK && KIND == 0)
             for (int e = lane ? lane : lanes; 2 * e < a.m; e += lanes) fold(S + c, e);
         __syncthreads();
         if constexpr (KIND != 0) {
             // radix-r1 butterflies over x[j + q m], times W_n^(j p), in place:
-            // S[p][j] (FOLD: of the pair j, m - j the sum and the difference)
+            // S[p][j] (BLK: of the pair j, m - j the sum and the difference)
             radix_dispatch<16>(a.r1, [&](auto rc) {
                 constexpr int RAD = decltype(rc)::value;
                 if constexpr (RAD > 1) {
@@ -336,7 +358,7 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
                             S[(p * a.m + j) * CW + c] = k == 0 ? x[k] : x[k] * w;
                         }
                     };
-                    if constexpr (!FOLD) {
+                    if constexpr (!BLK) {
                         for (int j = lane; j < a.m; j += lanes) butterfly(j);
                     } else {
                         for (int j = lane; j <= a.H; j += lanes) {
@@ -382,7 +404,7 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
             const R* osc[dense_ct<R>()];
 #pragma unroll
             for (int t = 0; t < dense_ct<R>(); ++t) {
-                const long long g = f0 + column_of<R>(a.cwl, threadIdx.x, t);
+                const long long g = f0 + column_of<R, BLK>(a.cwl, threadIdx.x, t);
                 olive[t] = g < a.ntot;
                 int go = 0, gc = 0;
                 if (olive[t]) line_of(g, a.ntot, a.ncols, go, gc);
@@ -394,7 +416,7 @@ __global__ void __launch_bounds__(kDenseMaxThreads, dense_ctas<R>(KIND == 2)) k_
                 const int e = p1 + a.r1 * p;
                 if constexpr (SCALED) v = v * osc[t][size_t(e) * a.estep];
                 oline[t][size_t(e) * a.es] = v;
-            });
+            }, std::bool_constant<BLK>{});
         }
         __syncthreads();   // the tile's buffer is free
     }
@@ -424,23 +446,20 @@ void DenseDFT::init(int n, int r1) {
     if (!r1) return;
     H_ = m_ / 2;
     nch_ = (H_ + 1 + kPC - 1) / kPC;
-    // (an angle rounded to 64 bits would cost the fp64 tables a digit)
-    std::vector<double> c(m_), d(m_);
-    for (int j = 0; j < m_; ++j) {
-        const long double w = 2.0L * kPiL * j / m_;
-        c[j] = double(std::cos(w));
-        d[j] = double(std::sin(w));
-    }
+    std::vector<double2> w(m_);
+    for (int j = 0; j < m_; ++j) w[j] = unit_root(j, m_);
     auto fill = [&](auto zero, DevBuf& buf) {
         using R = decltype(zero);
+        const bool blk = blocked<R>(H_);
+        auto at = [&](int ch, int s) { return blk ? tab_at<true>(nch_, ch, s) : tab_at<false>(nch_, ch, s); };
         std::vector<R> t(size_t(std::max(1, H_)) * nch_ * kChunk, zero);
         for (int q = 1; q <= H_; ++q)
             for (int p = 0; p <= H_; ++p) {
                 const size_t j = size_t(p) * q % m_;
                 R* e = t.data() + size_t(q - 1) * nch_ * kChunk + p % kPC;
-                // (in fp64 the middle row of an even m meets itself as a pair)
-                e[tab_at<R>(nch_, p / kPC, 0)] = R(sizeof(R) == 8 && 2 * q == m_ ? 0.5 * c[j] : c[j]);
-                e[tab_at<R>(nch_, p / kPC, 1)] = 2 * q == m_ ? zero : R(d[j]);
+                // (without blocks the middle row of an even m meets itself as a pair)
+                e[at(p / kPC, 0)] = R(!blk && 2 * q == m_ ? 0.5 * w[j].x : w[j].x);
+                e[at(p / kPC, 1)] = 2 * q == m_ ? zero : R(w[j].y);
             }
         buf.ensure(sizeof(R) * t.size());
         upload(buf.p, t.data(), sizeof(R) * t.size());
@@ -485,8 +504,9 @@ void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, si
     const bool radix2 = r1_ > 1 && m_ <= 16;       // no table
     const bool ts = !radix2 && tabb <= kDenseTableSmem && (per_col << 2) + tabb + twb <= kDenseSmemMax;
     auto smem = [&](int cwl) { return (per_col << cwl) + (ts ? tabb : 0) + twb; };
-    // threads: a work item (fp32: the A or B of one) each
-    auto items = [&](int cwl) { return a.r1 * a.nch << cwl; };
+    const bool blk = blocked<R>(H_) && !radix2;
+    // threads: a work item (in blocks: the A or B of one) each
+    auto items = [&](int cwl) { return (a.r1 * a.nch << cwl) / (blk ? 1 : dense_ct<R>()); };
     // columns per tile: 64 (fp64: 32), so that a warp's lanes are the columns
     // of one p range and read its table entries as one word; fewer while the
     // SM would not hold `ctas` CTAs, whose copies and products overlap, or the
@@ -500,11 +520,12 @@ void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, si
     const int regs = 256 / dense_ctas<R>(radix2);
     // four CTAs of 128 threads instead of two of 256 where their tiles, of
     // eight columns at least, are no smaller than the tables beside them
-    // (109-point pass of 48 columns, fp32: 558 us against 597; 366 points, 90
-    // columns: 34 against 37; with four
-    // columns per tile 151 points would take 145 against 93)
-    if (const int l = widest(4); sizeof(R) == 4 && !radix2 && l > 2 && smem(l) <= 56 * 1024 && (per_col << l) >= (ts ? tabb : 0)) {
-        cwl = l;
+    // (before the inner loop was unrolled by three: 109 points and 48 columns
+    // 558 us against 597, 366 points and 90 columns 34 against 37; with four
+    // columns per tile 151 points took 145 against 93)
+    const int l4 = widest(4);
+    if (blk && l4 > 2 && smem(l4) <= 56 * 1024 && (per_col << l4) >= (ts ? tabb : 0)) {
+        cwl = l4;
         maxthr = 128;
     }
     const size_t shm = smem(cwl);
@@ -523,14 +544,26 @@ void DenseDFT::launch(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, si
         set_smem_limit(kern, shm);
         launch_chained(kern, grid, nt, shm, s, a);
     };
-    auto pick = [&](auto scaled) {
-        constexpr bool SC = decltype(scaled)::value;
-        if (radix2) go(k_dense<R, SC, false, 2>);
-        else if (r1_ == 1) ts ? go(k_dense<R, SC, true, 0>) : go(k_dense<R, SC, false, 0>);
-        else ts ? go(k_dense<R, SC, true, 1>) : go(k_dense<R, SC, false, 1>);
+    auto pick = [&](auto scaled, auto blkc) {
+        constexpr bool SC = decltype(scaled)::value, BLK = decltype(blkc)::value;
+        if (r1_ == 1) ts ? go(k_dense<R, SC, true, 0, BLK>) : go(k_dense<R, SC, false, 0, BLK>);
+        else ts ? go(k_dense<R, SC, true, 1, BLK>) : go(k_dense<R, SC, false, 1, BLK>);
     };
-    if (scale) pick(std::true_type{});
-    else pick(std::false_type{});
+    auto kind = [&](auto scaled) {
+        if (radix2) {
+            go(k_dense<R, decltype(scaled)::value, false, 2, false>);
+            return;
+        }
+        if constexpr (sizeof(R) == 4) {
+            if (blk) {
+                pick(scaled, std::true_type{});
+                return;
+            }
+        }
+        pick(scaled, std::false_type{});
+    };
+    if (scale) kind(std::true_type{});
+    else kind(std::false_type{});
 }
 
 template void DenseDFT::run<float>(float2*, const float2*, size_t, int, size_t, int, int, const float*, int, int,

@@ -2,7 +2,7 @@
 cosine and sine tables (mpm_dense.cu), against numpy in more bits.  A rounding
 is at most u, of variance u^2 / 3 of its value.  Of a sum of H terms the partial
 sums have variance q = 1 .. H of a term's:
-* fp32, sums of 16 terms and then the sum of those B = H / 16: (16 + 1) / 2 + B / 2
+* fp32, sums of 20 terms and then the sum of those B = H / 20: (20 + 1) / 2 + B / 2
   roundings of a term per term, and two more for the pair's sum and the table;
 * fp64, one sum: H / 2, and two more; a table entry from an angle rounded to 64
   bits would bring in about two more by itself, and the twiddles likewise.
@@ -30,7 +30,7 @@ def rms_error(n, fp64, ncols=18, nouter=48):
 @pytest.mark.parametrize("n", [109, 151, 199, 251, 277])
 def test_fp32_product_sums_in_blocks(n):
     H = n // 2
-    assert rms_error(n, False) < 2.0 ** -24 * np.sqrt((8.5 + H / 32 + 2) / 3)
+    assert rms_error(n, False) < 2.0 ** -24 * np.sqrt((10.5 + H / 40 + 2) / 3)
 
 
 @pytest.mark.parametrize("n", [37, 61, 109])
