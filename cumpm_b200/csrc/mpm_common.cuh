@@ -45,12 +45,12 @@ void note_launch();
 
 // Host data for kernels on any stream.  cudaMemcpy from pageable memory may
 // return once the data are staged, and a stream made with
-// cudaStreamNonBlocking does not wait for the legacy stream that carries them,
-// so that stream is waited for here.
+// cudaStreamNonBlocking does not wait for the legacy stream that carries them:
+// uploads_done(), after the last of a set, waits for that stream.
 inline void upload(void* dst, const void* src, size_t bytes) {
     MPM_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
-    MPM_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
 }
+inline void uploads_done() { MPM_CUDA(cudaStreamSynchronize(cudaStreamLegacy)); }
 
 // --------------------------------------------------------------- complex --
 

@@ -758,6 +758,7 @@ void AxisFFT::init(int n) {
     const std::pair<int, int> ab =
         kind_ == 2 && (rader_faster(true) || rader_faster(false)) ? fft2_split(r2_ - 1) : std::pair<int, int>{0, 0};
     rader_.init(n, r1_, r2_, ab.first, ab.second);
+    uploads_done();
 }
 
 void AxisFFT::upload_table(std::vector<double2> t64, DevBuf& d64, DevBuf& d32) {

@@ -37,7 +37,7 @@ int sm_count();
 // m-point DFTs as products with their tables (mpm_dense.cu).  r1 = 0: off.
 class DenseDFT {
 public:
-    void init(int n, int r1);
+    void init(int n, int r1);     // (the caller waits for the uploads, uploads_done)
     // whether a tile of four columns fits in shared memory
     bool fits(bool fp64) const;
     // as AxisFFT::run / run_scaled (mode 2: two launches); tw: W_n^t, t < n
@@ -57,7 +57,7 @@ private:
 // in-register radix-r1 pass and Rader's convolution (mpm_rader.cu).
 class RaderDFT {
 public:
-    void init(int n, int r1, int p, int A, int B);
+    void init(int n, int r1, int p, int A, int B);     // (likewise)
     // false: not set up (A = 0, or a tile does not fit in shared memory)
     bool usable() const { return n_ != 0; }
     // as AxisFFT::run

@@ -1859,6 +1859,7 @@ Field::Field(const FieldSpec& spec) : spec_(spec) {
         for (int f = 0; f < (spec_.quads ? int(T_COUNT) : int(T_FD2) + 1); ++f)
             upload(tab_f_.as<double>() + size_t(f) * kTableSize, tables_.f[f].data(),
                    sizeof(double) * kTableSize);
+        uploads_done();
     } else if (spec_.kind == FIELD_POLY) {
         poly_init();
     } else if (spec_.kind != FIELD_DIRECT) {
@@ -1910,6 +1911,7 @@ void Field::set_positions(const double* x, const double* y, const double* z, int
             quad_idx_.ensure(sizeof(int) * Nq_);
             upload(quad_idx_.p, qidx.data(), sizeof(int) * Nq_);
         }
+        uploads_done();
         if (spec_.kind == FIELD_POLY && int(spec_.radius.size()) != N_)
             throw std::invalid_argument("Polydisperse field: radius size must match num_particles.");
         if (spec_.kind == FIELD_DIRECT) {
@@ -1918,6 +1920,7 @@ void Field::set_positions(const double* x, const double* y, const double* z, int
             if (int(rad.size()) != N_) throw std::invalid_argument("Direct field: radius size must match num_particles.");
             radius_.ensure(sizeof(double) * N_);
             upload(radius_.p, rad.data(), sizeof(double) * N_);
+            uploads_done();
         }
     }
     sources_.n = n;

@@ -741,6 +741,7 @@ void Field::poly_init() {
         upload(pqa2_.p, a2.data(), sizeof(double) * n);
         upload(pqg2_.p, g2.data(), sizeof(double) * n);
     }
+    uploads_done();
     gv_.Nx = pgeom_.ng[0];
     gv_.Ny = pgeom_.ng[1];
     gv_.Nz = pgeom_.ng[2];
