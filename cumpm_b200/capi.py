@@ -37,6 +37,7 @@ EXPORTS = [
     "mpm_field_apply_noalloc", "mpm_noalloc_scratch_bytes", "mpm_field_grad", "mpm_line_fft",
     "mpm_field_create_tuned", "mpm_field_autotune", "mpm_tune_xi_candidates", "mpm_tune_next_size",
     "mpm_solver_set_tuning", "mpm_solver_autotune", "mpm_field_set_bloch",
+    "mpm_empty_cache", "mpm_buffer_stats",
 ]
 
 STAGES = ["spread", "fft_fwd", "kspace", "fft_inv", "contract", "real", "direct", "krylov", "precalc"]
@@ -117,6 +118,9 @@ def lib():
         L.mpm_field_grad.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p,
                                      C.c_void_p]
         L.mpm_kernel_launches.restype = C.c_longlong
+        L.mpm_empty_cache.restype = None
+        L.mpm_buffer_stats.restype = C.c_longlong
+        L.mpm_buffer_stats.argtypes = [C.POINTER(C.c_size_t)] * 4
         L.mpm_line_fft.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_size_t, C.c_int, C.c_size_t, C.c_int, C.c_int,
                                    C.c_void_p, C.c_int, C.c_int, C.c_int, _ip, C.c_void_p]
         L.mpm_field_create_tuned.argtypes = [C.POINTER(C.c_void_p), C.c_int, C.c_int, _dp, C.c_double,
@@ -260,6 +264,21 @@ def profile_read():
 
 def kernel_launches():
     return int(lib().mpm_kernel_launches())
+
+
+def empty_cache():
+    """Gives the buffers that dropped solvers and near fields left for the next
+    ones (at most 256 MB of device and 64 MB of page-locked memory) back to the
+    driver."""
+    lib().mpm_empty_cache()
+
+
+def buffer_stats():
+    """Buffers asked for since the start, and bytes in use and kept."""
+    v = [C.c_size_t() for _ in range(4)]
+    n = lib().mpm_buffer_stats(*(C.byref(x) for x in v))
+    return dict(zip(("requests", "live_device", "live_host", "kept_device", "kept_host"),
+                    [int(n)] + [int(x.value) for x in v]))
 
 
 def _stream_ptr(stream):

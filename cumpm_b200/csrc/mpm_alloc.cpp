@@ -10,12 +10,12 @@
 // size:
 //  * bounded: at most 256 MB of device and 64 MB of host memory, no block
 //    above a quarter of that, and a block that kMaxAge later releases did not
-//    reuse is freed;
+//    reuse is freed; empty_buffer_cache() frees them all;
 //  * a block is kept only after the device that may still be using it has
 //    been waited for, as cudaFree does, so the next owner may be any thread
 //    and any stream;
 //  * when the driver is out of memory the kept blocks are freed first.
-#include "mpm_common.cuh"
+#include "mpm_alloc.h"
 
 #include <list>
 #include <mutex>
@@ -35,8 +35,9 @@ struct Pool {
     std::mutex mu;
     std::list<Block> kept;                                   // oldest first
     std::unordered_map<void*, std::pair<size_t, int>> live;  // size, device
-    size_t total = 0;
+    size_t total = 0, used = 0;                              // bytes kept, bytes in use
     unsigned long long clock = 0;
+    long long requests = 0;
     const bool host;
     const size_t cap;
     Pool(bool h, size_t c) : host(h), cap(c) {}
@@ -77,6 +78,7 @@ void* buf_alloc(size_t n, bool host) {
     MPM_CUDA(cudaGetDevice(&dev));
     const size_t want = rounded(n);
     std::lock_guard<std::mutex> lock(P.mu);
+    ++P.requests;
     auto best = P.kept.end();
     for (auto it = P.kept.begin(); it != P.kept.end(); ++it)
         if (it->bytes >= want && it->bytes <= want + want / 4 + 4096 && (host || it->dev == dev) &&
@@ -100,6 +102,7 @@ void* buf_alloc(size_t n, bool host) {
         MPM_CUDA(e);
     }
     P.live[p] = {got, dev};
+    P.used += got;
     return p;
 }
 
@@ -113,6 +116,7 @@ void buf_free(void* p, bool host) {
         if (it == P.live.end()) return;
         b = it->second;
         P.live.erase(it);
+        P.used -= b.first;
     }
     // wait for whatever still uses the block (outside the lock)
     bool idle = b.first <= P.cap / 4;
@@ -132,6 +136,26 @@ void buf_free(void* p, bool host) {
     P.kept.push_back({p, b.first, b.second, ++P.clock});
     P.total += b.first;
     P.trim(false);
+}
+
+BufferStats buffer_stats() {
+    BufferStats s{};
+    for (int host = 0; host < 2; ++host) {
+        Pool& P = pool(host != 0);
+        std::lock_guard<std::mutex> lock(P.mu);
+        s.requests += P.requests;
+        (host ? s.live_host : s.live_device) = P.used;
+        (host ? s.kept_host : s.kept_device) = P.total;
+    }
+    return s;
+}
+
+void empty_buffer_cache() {
+    for (int host = 0; host < 2; ++host) {
+        Pool& P = pool(host != 0);
+        std::lock_guard<std::mutex> lock(P.mu);
+        P.trim(true);
+    }
 }
 
 }  // namespace mpm

@@ -8,6 +8,7 @@
 #include <cstring>
 #include <string>
 
+#include "mpm_alloc.h"
 #include "mpm_field.h"
 #include "mpm_fft.h"
 #include "mpm_krylov.h"
@@ -634,5 +635,16 @@ int mpm_profile_read(double* ms, long long* count, int n) {
     return guard([&] { mpm::Profiler::get().read(ms, count, n); });
 }
 long long mpm_kernel_launches(void) { return mpm::Profiler::get().launches(); }
+
+void mpm_empty_cache(void) { mpm::empty_buffer_cache(); }
+
+long long mpm_buffer_stats(size_t* live_device, size_t* live_host, size_t* kept_device, size_t* kept_host) {
+    const mpm::BufferStats s = mpm::buffer_stats();
+    if (live_device) *live_device = s.live_device;
+    if (live_host) *live_host = s.live_host;
+    if (kept_device) *kept_device = s.kept_device;
+    if (kept_host) *kept_host = s.kept_host;
+    return s.requests;
+}
 
 }  // extern "C"

@@ -278,6 +278,15 @@ MPM_API int mpm_profile_read(double* ms, long long* count, int n);
 /* kernel launches issued by this library since the last reset */
 MPM_API long long mpm_kernel_launches(void);
 
+/* ---- memory (no counterpart in the reference) ----------------------------
+ * Dipole solvers and near fields keep the buffers that they release for the
+ * next one (at most 256 MB of device and 64 MB of page-locked memory in the
+ * whole process); this gives them back to the driver. */
+MPM_API void mpm_empty_cache(void);
+/* Buffers asked for since the start (the return value), and bytes in use and
+ * kept, device and page-locked; each pointer may be NULL. */
+MPM_API long long mpm_buffer_stats(size_t* live_device, size_t* live_host, size_t* kept_device, size_t* kept_host);
+
 /* ---- host-only helpers (no GPU needed) ---------------------------------- */
 /* real-space tables: out has 10 x 9001 doubles (r, fd1, fd2, fq1, fq2, fq3,
  * gq1, gq2, gq3, gq4); selfo/self_grad may be NULL */
