@@ -8,12 +8,17 @@
 // second for the driver's allocator when other processes use it).
 // Released blocks are therefore kept for the next request of about the same
 // size:
+//  * a block is kept only after the work that used it has been waited for, so
+//    the next owner may be any thread and any stream.  The work is known by
+//    stream: a solver's and a near field's own one, and those on which a
+//    caller applied a field (ReuseScope).  Waiting for the whole device would
+//    break a graph capture that runs in another thread, which cudaFree does
+//    not;
+//  * a block whose work is not known (a field whose call was captured or has
+//    thrown, the tuner's trials) goes back to the driver at once;
 //  * bounded: at most 256 MB of device and 64 MB of host memory, no block
 //    above a quarter of that, and a block that kMaxAge later releases did not
 //    reuse is freed; empty_buffer_cache() frees them all;
-//  * a block is kept only after the device that may still be using it has
-//    been waited for, as cudaFree does, so the next owner may be any thread
-//    and any stream;
 //  * when the driver is out of memory the kept blocks are freed first.
 #include "mpm_alloc.h"
 
@@ -42,6 +47,7 @@ struct Pool {
     const size_t cap;
     Pool(bool h, size_t c) : host(h), cap(c) {}
 
+    size_t largest() const { return cap / 4; }
     void drop(const Block& b) {
         if (host) cudaFreeHost(b.p);
         else cudaFree(b.p);
@@ -64,6 +70,8 @@ Pool& pool(bool host) {
     return host ? *hst : *dev;
 }
 
+thread_local const ReuseScope* t_scope = nullptr;
+
 size_t rounded(size_t n) {
     size_t unit = 512;
     while (unit * 8 < n) unit *= 2;      // steps of an eighth
@@ -71,6 +79,61 @@ size_t rounded(size_t n) {
 }
 
 }  // namespace
+
+namespace {
+// an error that only means that a block cannot be kept
+bool ok(cudaError_t e) {
+    if (e == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+}  // namespace
+
+StreamUses::~StreamUses() {
+    for (const Use& u : uses_) cudaEventDestroy(u.done);
+}
+
+void StreamUses::record(cudaStream_t s) {
+    if (unknown_) return;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (!ok(cudaStreamIsCapturing(s, &cap)) || cap != cudaStreamCaptureStatusNone || !ok(cudaStreamGetId(s, &id))) {
+        unknown_ = true;
+        return;
+    }
+    for (const Use& u : uses_)
+        if (u.stream == id) {
+            if (!ok(cudaEventRecord(u.done, s))) unknown_ = true;
+            return;
+        }
+    Use u{id, nullptr};
+    if (uses_.size() >= 16) {          // a caller that makes a stream per call: wait for the oldest
+        u.done = uses_.front().done;
+        uses_.erase(uses_.begin());
+        if (!ok(cudaEventSynchronize(u.done))) unknown_ = true;
+    } else if (!ok(cudaEventCreateWithFlags(&u.done, cudaEventDisableTiming))) {
+        unknown_ = true;
+        return;
+    }
+    uses_.push_back(u);
+    if (!ok(cudaEventRecord(u.done, s))) unknown_ = true;
+}
+
+bool StreamUses::wait() const {
+    if (unknown_) return false;
+    for (const Use& u : uses_)
+        if (!ok(cudaEventSynchronize(u.done))) return false;
+    return true;
+}
+
+ReuseScope::ReuseScope(bool own, cudaStream_t s, const StreamUses* uses)
+    : own_(own), s_(s), uses_(uses), outer_(t_scope) {
+    t_scope = this;
+}
+ReuseScope::~ReuseScope() { t_scope = outer_; }
+bool ReuseScope::idle() const {
+    return (!own_ || ok(cudaStreamSynchronize(s_))) && (!uses_ || uses_->wait());
+}
 
 void* buf_alloc(size_t n, bool host) {
     Pool& P = pool(host);
@@ -118,16 +181,8 @@ void buf_free(void* p, bool host) {
         P.live.erase(it);
         P.used -= b.first;
     }
-    // wait for whatever still uses the block (outside the lock)
-    bool idle = b.first <= P.cap / 4;
-    if (idle) {
-        int cur = 0;
-        idle = cudaGetDevice(&cur) == cudaSuccess;
-        if (idle && cur != b.second) idle = cudaSetDevice(b.second) == cudaSuccess;
-        if (idle) idle = cudaDeviceSynchronize() == cudaSuccess;
-        if (cur != b.second) cudaSetDevice(cur);
-    }
-    if (!idle) {       // too large, or the device is not in a state to keep anything
+    // (the wait is outside the lock)
+    if (!t_scope || b.first > P.largest() || !t_scope->idle()) {
         if (host) cudaFreeHost(p);
         else cudaFree(p);
         return;

@@ -296,7 +296,7 @@ int mpm_field_create(mpm_field** out, int kind, int mode, const double box[3], d
         const mpm::FieldSpec fs =
             field_spec(kind, mode, box, errortol, xi, radius, n_radius, solve_quads, quad_idxs, n_quad_idxs);
         auto* f = new mpm::Field(fs);
-        *out = new mpm_field{f, nullptr};
+        *out = new mpm_field{f, nullptr, {}};
     });
 }
 int mpm_field_create_tuned(mpm_field** out, int kind, int mode, const double box[3], double errortol,
@@ -309,7 +309,7 @@ int mpm_field_create_tuned(mpm_field** out, int kind, int mode, const double box
         const mpm::FieldSpec fs = mpm::apply_tuning(
             field_spec(kind, mode, box, errortol, t.xi, radius, n_radius, solve_quads, quad_idxs, n_quad_idxs), t);
         auto* f = new mpm::Field(fs);
-        *out = new mpm_field{f, nullptr};
+        *out = new mpm_field{f, nullptr, {}};
     });
 }
 int mpm_field_autotune(int kind, const double box[3], double errortol, double xi, const double* radius, int n_radius,
@@ -355,8 +355,12 @@ int mpm_tune_next_size(int n, int smooth23) {
 }
 void mpm_field_destroy(mpm_field* f) {
     if (!f) return;
-    delete f->solver;
-    delete f->impl;
+    {
+        std::optional<mpm::ReuseScope> reuse;
+        if (!f->uses.unknown()) reuse.emplace(f->uses);
+        delete f->solver;
+        delete f->impl;
+    }
     delete f;
 }
 int mpm_field_set_positions(mpm_field* f, const double* x, const double* y, const double* z, int n, void* stream) {
@@ -365,14 +369,18 @@ int mpm_field_set_positions(mpm_field* f, const double* x, const double* y, cons
         if (f->impl->spec().kind == mpm::FIELD_DIRECT && !f->impl->spec().radius.empty() &&
             int(f->impl->spec().radius.size()) != n && f->impl->spec().radius.size() != 1)
             throw std::invalid_argument("Direct field: radius size must match num_particles.");
+        FieldCall call(f, static_cast<cudaStream_t>(stream));
         f->impl->set_positions(x, y, z, n, static_cast<cudaStream_t>(stream));
+        call.done();
     });
 }
 int mpm_field_set_field_points(mpm_field* f, const double* x, const double* y, const double* z, int n,
                                void* stream) {
     return guard([&] {
         need(f, "field");
+        FieldCall call(f, static_cast<cudaStream_t>(stream));
         f->impl->set_field_points(x, y, z, n, static_cast<cudaStream_t>(stream));
+        call.done();
     });
 }
 int mpm_field_apply(mpm_field* f, const void* X, void* Y, int M, const void* sc, int jacobi, int recip_fp32,
@@ -383,8 +391,10 @@ int mpm_field_apply(mpm_field* f, const void* X, void* Y, int M, const void* sc,
         need(Y, "Y");
         if (M < 1) throw std::invalid_argument("M must be >= 1");
         if (jacobi && !sc) throw std::invalid_argument("jacobi scaling needs self coefficients");
+        FieldCall call(f, static_cast<cudaStream_t>(stream));
         f->impl->apply(static_cast<const double2*>(X), static_cast<double2*>(Y), M, static_cast<const double2*>(sc),
                        jacobi != 0, recip_fp32 != 0, real_fp32 != 0, static_cast<cudaStream_t>(stream));
+        call.done();
     });
 }
 int mpm_field_apply_part(mpm_field* f, const void* X, void* Y, int M, const void* sc, int recip_fp32, int real_fp32,
@@ -393,9 +403,11 @@ int mpm_field_apply_part(mpm_field* f, const void* X, void* Y, int M, const void
         need(f, "field");
         need(X, "X");
         need(Y, "Y");
+        FieldCall call(f, static_cast<cudaStream_t>(stream));
         f->impl->apply_part(static_cast<const double2*>(X), static_cast<double2*>(Y), M,
                             static_cast<const double2*>(sc), recip_fp32 != 0, real_fp32 != 0, part,
                             static_cast<cudaStream_t>(stream));
+        call.done();
     });
 }
 int mpm_field_set_bloch(mpm_field* f, double kx, double ky) {
@@ -458,8 +470,10 @@ int mpm_batch_solve(mpm_field* f, const void* B, void* X, int M, const void* sc,
         o.shifted = opt->shifted != 0;
         if (!(o.inner_tol >= 0.0)) throw std::invalid_argument("inner_tol must be >= 0");
         mpm::SolveStats st;
+        FieldCall call(f, static_cast<cudaStream_t>(stream));
         f->solver->solve(*f->impl, static_cast<const double2*>(B), static_cast<double2*>(X), M,
                          static_cast<const double2*>(sc), o, st, static_cast<cudaStream_t>(stream));
+        call.done();
         if (rep) {
             std::memset(rep, 0, sizeof(*rep));
             rep->matvecs = st.matvecs;
@@ -545,9 +559,11 @@ int mpm_field_grad(mpm_field* f, const void* lam, const void* p, int M, void* gx
         need(p, "p");
         need(gx, "gx");
         need(ga, "ga");
+        FieldCall call(f, static_cast<cudaStream_t>(stream));
         f->impl->grad_bilinear(static_cast<const double2*>(lam), static_cast<const double2*>(p), M,
                                static_cast<double2*>(gx), static_cast<double2*>(ga),
                                static_cast<cudaStream_t>(stream));
+        call.done();
     });
 }
 

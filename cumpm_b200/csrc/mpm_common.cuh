@@ -123,7 +123,7 @@ inline double2 unit_root(long long j, long long n) {
 // --------------------------------------------------------------- buffers --
 
 // device (or page-locked host) memory from / to the bounded cache of
-// mpm_alloc.cpp; buf_free waits for the device, as cudaFree does
+// mpm_alloc.cpp; buf_free waits for the work that uses it, as cudaFree does
 void* buf_alloc(size_t n, bool host);
 void buf_free(void* p, bool host);
 

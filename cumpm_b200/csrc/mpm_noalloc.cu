@@ -64,9 +64,11 @@ int mpm_field_apply_noalloc(mpm_field* f, const void* X, void* Y, int M, const v
                                             "-byte static scratch; use fewer right-hand sides or mpm_field_apply");
         }
         void* scratch = scratch_on_current_device();
+        FieldCall call(f, static_cast<cudaStream_t>(stream));
         f->impl->apply_scratch(static_cast<const double2*>(X), static_cast<double2*>(Y), M,
                                static_cast<const double2*>(self_coef), jacobi != 0, recip_fp32 != 0, real_fp32 != 0,
                                scratch, kNoAllocScratchBytes, static_cast<cudaStream_t>(stream));
+        call.done();
     });
 }
 

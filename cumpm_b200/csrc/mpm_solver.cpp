@@ -1,9 +1,11 @@
 // Host driver (see mpm_solver.h).  Reference semantics cited per function.
 #include "mpm_solver.h"
+#include "mpm_alloc.h"
 
 #include <algorithm>
 #include <cmath>
 #include <iostream>
+#include <optional>
 #include <stdexcept>
 
 namespace mpm {
@@ -33,8 +35,14 @@ DipoleSolver::DipoleSolver(std::vector<double> box, std::vector<std::vector<cdou
 }
 
 DipoleSolver::~DipoleSolver() {
-    field_.reset();
-    solver_.reset();
+    {
+        std::optional<ReuseScope> reuse;
+        if (stream_ && !failed_) reuse.emplace(stream_);
+        field_.reset();
+        solver_.reset();
+        for (DevBuf* b : {&dB_, &dX_, &dSC_, &dEps_, &dRad_, &dE0_, &dInit_, &dFrame_}) b->release();
+        for (HostBuf* b : {&hB_, &hX_, &hSC_}) b->release();
+    }
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -600,6 +608,11 @@ void DipoleSolver::compute(const std::vector<double>& x, const std::vector<doubl
     if (n == 0) return;
     if (N_ == 0) setup(n);
     else if (N_ != n) throw std::runtime_error("The number of particles has changed!");
+    // (a computation that throws may leave work on the field's second stream)
+    std::optional<ReuseScope> reuse;
+    const bool clean = !failed_;
+    if (clean) reuse.emplace(stream_);
+    failed_ = true;
     if (!field_) field_ = std::make_unique<Field>(tuned_ ? apply_tuning(field_spec(), tuning_) : field_spec());
     num_frames_++;
     const std::vector<double> sx = scaled(x), sy = scaled(y), sz = scaled(z);
@@ -647,6 +660,7 @@ void DipoleSolver::compute(const std::vector<double>& x, const std::vector<doubl
     avg_dips_.insert(avg_dips_.end(), frame_cap.begin(), frame_cap.end());
     dip_frames_.push_back(std::move(frame_dip));
     quad_frames_.push_back(solve_quads_ && Nq_ ? std::move(frame_quad) : std::vector<cdouble>());
+    failed_ = !clean;
 }
 
 // dipole_solver.cu:613-647
@@ -709,7 +723,13 @@ NearField::NearField(std::vector<double> box, std::vector<cdouble> E0, std::vect
 }
 
 NearField::~NearField() {
-    field_.reset();
+    {
+        std::optional<ReuseScope> reuse;
+        if (stream_) reuse.emplace(stream_);
+        field_.reset();
+        dX_.release();
+        dY_.release();
+    }
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -767,6 +787,7 @@ std::vector<double> NearField::calculate() {
         if (!stream_) MPM_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
         field_ = std::make_unique<Field>(fs);
     }
+    const ReuseScope reuse(stream_);
     const size_t M = fx_.size();
     std::vector<double> x(N_), y(N_), z(N_), a(M), b(M), c(M);
     for (size_t i = 0; i < N_; ++i) { x[i] = px_[i] / length_scale_; y[i] = py_[i] / length_scale_; z[i] = pz_[i] / length_scale_; }

@@ -127,6 +127,7 @@ private:
     // depend on nothing that changes between frames)
     std::vector<size_t> dev_freqs_;
     int indent_ = 0;
+    bool failed_ = false;     // a computation has thrown: buffers go back to the driver
 };
 
 class NearField {

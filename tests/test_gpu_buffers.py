@@ -1,5 +1,7 @@
 """Kept buffers (mpm_alloc.cpp): a dropped solver's are reused and given back on
-request."""
+request, and dropping objects leaves graph captures of other threads alone."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -43,3 +45,63 @@ def test_a_solvers_buffers_are_kept_within_bounds_and_given_back():
     capi.empty_cache()
     none = capi.buffer_stats()
     assert none["kept_device"] == none["kept_host"] == 0
+
+
+def test_a_fields_buffers_are_kept_unless_a_graph_may_use_them():
+    from cumpm_b200 import capi
+
+    X = torch.ones((42, 3), dtype=torch.complex128, device="cuda")
+    Y = torch.empty_like(X)
+    capi.empty_cache()
+    f = field()
+    other = torch.cuda.Stream()
+    for s in (torch.cuda.current_stream(), other):           # on two streams
+        f.apply(X, Y, stream=s)
+    del f
+    assert capi.buffer_stats()["kept_device"] > 0
+    torch.cuda.synchronize()
+    f = field()
+    f.apply(X, Y)
+    torch.cuda.synchronize()
+    ref = Y.clone()
+    capi.empty_cache()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        f.apply(X, Y)
+    Y.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert (Y == ref).all()
+    del f
+    assert capi.buffer_stats()["kept_device"] == 0
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+@pytest.mark.parametrize("make", [field, solver])
+def test_dropping_an_object_leaves_a_capture_of_another_thread_alone(make, mode):
+    held = [make()]
+    go, done = threading.Event(), threading.Event()
+
+    def drop():
+        go.wait(30)
+        held.pop()
+        done.set()
+
+    t = threading.Thread(target=drop)
+    t.start()
+    a = torch.ones(1024, device="cuda")
+    b = torch.zeros_like(a)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    try:
+        with torch.cuda.graph(g, capture_error_mode=mode):
+            b.copy_(a * 2)
+            go.set()
+            assert done.wait(30)
+            b.add_(1)
+    finally:
+        go.set()
+        t.join()
+    g.replay()
+    torch.cuda.synchronize()
+    assert (b == 3).all()
