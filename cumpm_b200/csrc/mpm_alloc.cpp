@@ -72,9 +72,11 @@ Pool& pool(bool host) {
 
 thread_local const ReuseScope* t_scope = nullptr;
 
-size_t rounded(size_t n) {
+// steps of an eighth to a quarter, so that a kept block fits its next request;
+// blocks too large to be kept are not enlarged
+size_t rounded(size_t n, size_t largest) {
     size_t unit = 512;
-    while (unit * 8 < n) unit *= 2;      // steps of an eighth
+    while (n <= largest && unit * 8 < n) unit *= 2;
     return (n + unit - 1) / unit * unit;
 }
 
@@ -139,7 +141,7 @@ void* buf_alloc(size_t n, bool host) {
     Pool& P = pool(host);
     int dev = 0;
     MPM_CUDA(cudaGetDevice(&dev));
-    const size_t want = rounded(n);
+    const size_t want = rounded(n, P.largest());
     std::lock_guard<std::mutex> lock(P.mu);
     ++P.requests;
     auto best = P.kept.end();

@@ -1,5 +1,6 @@
 """Kept buffers (mpm_alloc.cpp): a dropped solver's are reused and given back on
-request, and dropping objects leaves graph captures of other threads alone."""
+request, large ones are not enlarged, and dropping objects leaves graph captures
+of other threads alone."""
 import threading
 
 import numpy as np
@@ -74,6 +75,21 @@ def test_a_fields_buffers_are_kept_unless_a_graph_may_use_them():
     assert (Y == ref).all()
     del f
     assert capi.buffer_stats()["kept_device"] == 0
+
+
+def test_large_buffers_are_not_enlarged():
+    """A grid of 1.1 GB: what a field holds beyond its requests is less than the
+    quarter by which small blocks may be rounded up."""
+    from cumpm_b200 import capi
+
+    box, m = 180.0, 12
+    f = field(box, 50)
+    before = capi.buffer_stats()["live_device"]
+    f.apply(torch.zeros((150, m), dtype=torch.complex128, device="cuda"), recip_fp32=True)
+    g = f.info()["grid"]
+    grid = 8 * 3 * m * g[0] * g[1] * g[2]
+    assert grid > 256 << 20
+    assert grid <= capi.buffer_stats()["live_device"] - before < grid + (64 << 20)
 
 
 @pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
