@@ -69,10 +69,12 @@ def _fresh(kind):
 @pytest.mark.parametrize("kind", ["mono", "poly", "direct"])
 def test_noalloc_first_call_on_a_fresh_field_allocates_nothing(kind):
     """Called before any mpm_field_apply on a new field, the entry point
-    leaves the device's free memory where it was, and then agrees with
-    mpm_field_apply.  A warm-up call on another field of the same kind loads
+    asks for no buffer (the library's count of requests, which kept blocks
+    could serve without the device's free memory changing), leaves the device's
+    free memory where it was, and then agrees with mpm_field_apply.  A warm-up call on another field of the same kind loads
     the kernels first (module loading may take device memory)."""
     import torch
+    from cumpm_b200 import capi
     rng = np.random.default_rng(9)
     W, Nw = _fresh(kind)
     F, N = _fresh(kind)
@@ -85,10 +87,12 @@ def test_noalloc_first_call_on_a_fresh_field_allocates_nothing(kind):
         _call_noalloc(W, Xw, Yw, Sw, fp32)
     torch.cuda.synchronize()
     free0 = torch.cuda.mem_get_info()[0]
+    asked0 = capi.buffer_stats()["requests"]
     for fp32 in (False, True):   # nothing is allocated inside this window, by torch or by the library
         _call_noalloc(F, X, got[fp32], S, fp32)
     torch.cuda.synchronize()
     free1 = torch.cuda.mem_get_info()[0]
+    assert capi.buffer_stats()["requests"] == asked0
     assert free1 == free0, f"free device memory changed by {free0 - free1} bytes"
     for fp32 in (False, True):
         ref = F.apply(X, self_coef=S, recip_fp32=fp32).cpu().numpy()
