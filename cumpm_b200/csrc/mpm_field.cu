@@ -2337,11 +2337,9 @@ void Field::precalc(cudaStream_t s) {
             if (!gv_.pruned) fftz_.init(gv_.Nz);
         }
         build_stencil(sources_, s, true);
-        // a solve applies the operator many times per frame; a field at points
-        // is applied once, and the plan costs several spreads (near field of
-        // 1000 particles on 185 x 41 x 240: 2 x 165 us against 70 us more
-        // per spread without it)
-        if (spec_.solver_ax) build_spread_plan(s);
+        // the plan costs several spreads (1000 particles on 185 x 41 x 240:
+        // 2 x 165 us against 70 us more per spread without it)
+        if (!spec_.once) build_spread_plan(s);
         else plan_cap_ = 0;
         if (!spec_.solver_ax) build_stencil(targets_, s, false);  // SOLVER_AX: targets share the source stencil
         build_pairs(s);

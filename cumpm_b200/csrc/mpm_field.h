@@ -46,6 +46,9 @@ struct FieldSpec {
     // Bloch wavevector (x, y) of the periodic images (EELS zone sum):
     // k-space at k - b, a phase on every real-space pair; dipoles only
     double bloch[2] = {0.0, 0.0};
+    // applied once per set of positions: no per-frame tables that only pay
+    // over several applications (the spread plan)
+    bool once = false;
 };
 
 // Spectral-Ewald parameters (monodisperse_ewald_electric_field.cu:546-616).

@@ -767,6 +767,7 @@ std::vector<double> NearField::calculate() {
         length_scale_ = radius_[0];
         FieldSpec fs;
         fs.solver_ax = false;
+        fs.once = true;
         for (int d = 0; d < 3; ++d) fs.box[d] = box_[d] / length_scale_;
         fs.errortol = errortol_;
         fs.xi = xi_;
