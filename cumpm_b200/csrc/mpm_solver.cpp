@@ -190,9 +190,14 @@ __global__ void k_batch_guess(double2* __restrict__ X, int M, int N, int K, cons
 // s = -3 / (4 pi (1 - eps) a^3) (dipole_solver.cu:452-460) and initial guesses
 // (dipole_solver.cu:233-346) on the device.
 
+// a / b, b scaled by a power of two so that its square neither overflows nor
+// vanishes (as std::complex division does)
 __device__ __forceinline__ double2 quot(double2 a, double2 b) {
+    const double m = fmax(fabs(b.x), fabs(b.y));
+    const int e = m > 0.0 && isfinite(m) ? -ilogb(m) : 0;
+    b = make_double2(scalbn(b.x, e), scalbn(b.y, e));
     const double d = b.x * b.x + b.y * b.y;
-    return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
+    return make_double2(scalbn((a.x * b.x + a.y * b.y) / d, e), scalbn((a.y * b.x - a.x * b.y) / d, e));
 }
 
 __global__ void k_sweep_rhs(double2* __restrict__ B, int N, int K, const double2* __restrict__ E0) {

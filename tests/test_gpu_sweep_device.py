@@ -41,6 +41,17 @@ def test_sweep_matches_single_frequencies(W, solver, guess, field_type):
     np.testing.assert_allclose(a, d.mean(axis=(0, 2)), rtol=1e-10, atol=1e-10 * np.abs(a).max())
 
 
+def test_extrapolation_from_an_epsilon_close_to_the_mediums():
+    """(eps + 2) / (eps - 1) whose divisor's square vanishes in 64 bits."""
+    g = np.stack(np.meshgrid(np.arange(2), np.arange(2), np.arange(2)), axis=-1).reshape(-1, 3) * 3.0
+    eps = 1.2 * np.array([1.0 + 0.5j, 1.0 + 1e-170j, 1.0 + 2e-170j, 2.0 + 0.1j])
+    d, _ = run(eps, g, guess_type="derivative", field_type="direct")
+    d = d.reshape(4, 8, 3, 3)
+    assert np.isfinite(d).all()
+    ref = run(eps[3:], g, field_type="direct")[0].reshape(8, 3, 3)
+    assert np.abs(d[3] - ref).max() < 1e-6 * np.abs(ref).max()
+
+
 def test_unknown_guess_is_refused_at_the_second_frequency():
     g = np.array([[0.0, 0, 0], [3.0, 0, 0]])
     run(np.array([2.0 + 0.1j]), g, guess_type="none")
