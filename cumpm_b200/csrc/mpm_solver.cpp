@@ -330,7 +330,7 @@ void DipoleSolver::sweep_device(const std::vector<cdouble>& init, std::vector<cd
     dSC_.ensure(sizeof(double2) * N_ * M);
     dX_.ensure(3 * bytes);  // this frequency's solution and the two before it
     dFrame_.ensure(bytes);
-    hX_.ensure(2 * bytes);  // a frequency's dipoles travel while the next one is solved
+    hX_.ensure(bytes);
     upload_inputs();
     dInit_.ensure(bytes);
     std::copy(init.begin(), init.begin() + rows * M, hX_.as<cdouble>());
@@ -341,7 +341,7 @@ void DipoleSolver::sweep_device(const std::vector<cdouble>& init, std::vector<cd
     const SolveOptions so = solve_options();
     frame_dip.resize(W * rows * M);
     auto collect = [&](size_t w) {
-        std::copy_n(hX_.as<cdouble>() + (w % 2) * rows * M, rows * M, frame_dip.data() + w * rows * M);
+        std::copy_n(hX_.as<cdouble>(), rows * M, frame_dip.data() + w * rows * M);
     };
     const bool mean = guess_type_ == "mean_field" || guess_type_ == "mean-field";
     for (size_t w = 0; w < W; ++w) {
@@ -364,9 +364,10 @@ void DipoleSolver::sweep_device(const std::vector<cdouble>& init, std::vector<cd
         for (int v : last_stats_.iters) iters_.push_back(v);
         k_to_frame<<<nblk_s(n, 256), 256, 0, stream_>>>(slot(w), M, int(N_), M, dFrame_.as<double2>());
         MPM_LAUNCH();
-        if (w > 0) collect(w - 1);      // its copy ended before this solve did
-        MPM_CUDA(cudaMemcpyAsync(hX_.as<cdouble>() + (w % 2) * rows * M, dFrame_.p, bytes, cudaMemcpyDeviceToHost,
-                                 stream_));
+        // a frequency's dipoles are copied before the next solve starts, and
+        // taken when that solve, which the host waits for, has ended
+        if (w > 0) collect(w - 1);
+        MPM_CUDA(cudaMemcpyAsync(hX_.p, dFrame_.p, bytes, cudaMemcpyDeviceToHost, stream_));
     }
     MPM_CUDA(cudaStreamSynchronize(stream_));
     collect(W - 1);
