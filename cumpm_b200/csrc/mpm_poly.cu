@@ -267,6 +267,14 @@ template <typename R> __host__ __device__ constexpr size_t poly_spread_smem(int 
     return size_t(kPolyStages) * kPolyPer * 64 * 24 * sizeof(R) + size_t(cap) * (3 * CM * sizeof(cplx<R>) + 24 * 2 + 4);
 }
 
+// A frame is refused when more particles' bins than these reach one tile (the
+// list before those are left out whose support does not cover it); the spread
+// of as many fits in shared memory in both precisions.
+constexpr int kPolyCandMax = 331;
+static_assert(poly_spread_smem<float>(kPolyCandMax, 16) <= 227 * 1024 &&
+                  poly_spread_smem<double>(kPolyCandMax, 8) <= 227 * 1024,
+              "the longest candidate list must fit in shared memory");
+
 template <typename R, int CM>
 __global__ void __launch_bounds__(256) k_poly_spread(const double2* __restrict__ X, int M, const R* __restrict__ w,
                                                      const int4* __restrict__ base, const int* __restrict__ toff,
@@ -857,14 +865,12 @@ void Field::poly_weights(PointSet& ps, const double* radius_dev, cudaStream_t s,
                                                                    ptlist_.as<int>(), ptcnt_.as<int>(),
                                                                    ptclist_.as<int>(), ptmax_.as<int>());
     MPM_LAUNCH();
-    // the spread's shared memory holds the candidates that are left (the limit
-    // on a frame is that of the unfiltered lists)
+    // the spread's shared memory holds the candidates that are left
     int kept = 0;
     MPM_CUDA(cudaMemcpyAsync(&kept, ptmax_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     MPM_CUDA(cudaStreamSynchronize(s));
     pcand_cap_ = std::max(1, kept);
-    const size_t shm = 65536 + (3 * 128 + 9 * sizeof(int)) * size_t(std::max(1, h));
-    if (shm > 200 * 1024 || pgeom_.P > 255)
+    if (h > kPolyCandMax || pgeom_.P > 255)
         throw std::runtime_error("polydisperse spread: " + std::to_string(h) +
                                  " particles reach one 8^3 voxel tile, more than the shared candidate list holds");
 }
