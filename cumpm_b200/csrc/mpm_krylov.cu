@@ -523,10 +523,10 @@ __device__ __forceinline__ void shift_givens_body(GState* __restrict__ mst, GSta
     if (threadIdx.x == 0) flag[0] = n;
 }
 
-// The seeds' second projection (k_arn_finish pass 2, no Givens) and the
-// members' Givens updates (shift_givens_body) in one CTA: the members
-// read only the seeds' Hessenberg column and norm, which the first part
-// writes, so the seeds' normalisation of V_{k+1} can follow.
+// The members of a shifted solve: their Givens updates (shift_givens_body)
+// follow the seeds' second projection (arn_finish2_body without Givens) in the
+// same CTA (finish2_body).  They read only the seeds' Hessenberg column and
+// norm, so the seeds' normalisation of V_{k+1} can follow.
 struct MemberArgs {
     GState* st;             // null: no members (plain GMRES)
     const double2* sigma;
@@ -1222,7 +1222,7 @@ void BatchSolver::gmres(Field& F, const double2* b, double2* x, int M, const dou
     w_.ensure(sizeof(double2) * n);
     r_.ensure(sizeof(double2) * n);
     bj_.ensure(sizeof(double2) * n);
-    flagdev_.ensure(sizeof(int) * (M + 2));   // count, M column flags, second-pass count
+    flagdev_.ensure(sizeof(int) * (M + 2));   // count, M column flags
     cur_cols_.clear();  // self coefficients may differ from the previous call
     double2* V = V_.as<double2>();
     GState* gs = state_.as<GState>();

@@ -132,7 +132,6 @@ private:
     int* poll_words(int M);
     int wait_flags(cudaStream_t s);
     std::vector<int> cur_cols_;          // column list the device buffers hold
-    const double2* cur_sc_ = nullptr;    // self coefficients gathered into scc_
 };
 
 }  // namespace mpm
