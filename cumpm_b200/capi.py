@@ -201,8 +201,8 @@ def line_fft(data, n, es, ncols, os, nouter, mode=0, scale=None, sz=1, sb=1, gen
     column c at flat index o*os + e*es + c.  mode 0 forward, 1 inverse,
     2 forward * scale[(e*nouter + o)*sz + c//sb] then inverse (scale a real
     CUDA tensor of the matching precision).  Returns the split n = r1 * r2 of
-    the kernel that ran (r2 above 16: a prime), (0, 0) for the multi-pass
-    kernel."""
+    the kernel that ran (r2 above 16: a product with tables or Rader's
+    convolution), (0, 0) for the multi-pass kernel."""
     import torch
 
     if not data.is_cuda or not data.is_contiguous() or data.dtype not in (torch.complex64, torch.complex128):

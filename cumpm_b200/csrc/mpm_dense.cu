@@ -436,7 +436,7 @@ int sm_count() {
     return sms;
 }
 
-// Tables longer than this stay in global memory (L1): m above 131.
+// Tables longer than this stay in global memory (L1): m above 191, in fp64 127.
 constexpr size_t kDenseTableSmem = 72 * 1024;
 
 void DenseDFT::init(int n, int r1) {

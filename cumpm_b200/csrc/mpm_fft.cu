@@ -268,6 +268,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_axis(cplx<R>* __restrict__ 
     // dead columns copy nothing; their source address is only a placeholder
     const cplx<R>* src = live ? line : data;
     const size_t ses = live ? es : 0;
+    chain_enter();
     for (int e = lane; e < n; e += ROWS) copy_async<R>(A + e * CW + c, src + size_t(e) * ses, live);
     if (STREAM)
         for (int t = threadIdx.x; t < f.pt_total; t += kFftThreads) PT[t] = ptw[t];
@@ -426,6 +427,10 @@ std::pair<int, int> fft2_split(int n) {
     }
     return best;
 }
+
+// longest composite m of a dense pass (m FMAs per element against the general
+// kernel's extra shared round trips)
+constexpr int kDenseMaxComposite = 131;
 
 size_t fft2_smem(int n, int cw, size_t elem) { return (size_t(n) * cw + n) * elem; }
 
@@ -674,7 +679,7 @@ void launch_cw(int cls, bool stream, int nouter, size_t shm, cudaStream_t s, cpl
     const int ngroups = (ncols + CW - 1) / CW;
     auto go = [&](auto kern) {
         set_smem_limit(kern, shm);
-        kern<<<nouter * ngroups, kFftThreads, shm, s>>>(data, f, tw, es, ncols, os, ptw, ngroups, ks);
+        launch_chained(kern, nouter * ngroups, kFftThreads, shm, s, data, f, tw, es, ncols, os, ptw, ngroups, ks);
     };
     if (stream) {
         if (cls == 8) go(k_fft_axis<R, INV, CW, 8, true, KSCALE>);
@@ -751,10 +756,22 @@ void AxisFFT::init(int n) {
     }
     f_.pt_total = int(p64.size());
     upload_table(p64, pt64_, pt32_);
-    // (no product for a composite rest: the general kernel's short radices are
-    // as fast or faster, 8.9 us against 19.4 for 300 points, 9 columns and 80
-    // lines, and its largest errors smaller)
-    dense_.init(n, r1_);
+    // A length of neither kind whose largest prime is 11 or 13, which the
+    // general kernel transforms by sums of as many terms, takes the product
+    // with the largest radix up to 16 in front (us, product and general, grids
+    // in L2: 260 points, 9 columns, 60 lines 7.5 and 10.0, fp64 6.3 and 14.8;
+    // 364 points, 90 columns 19.5 and 39.7).  With primes up to 7 the general
+    // kernel's largest errors are smaller (384 points: 0.7 of the product's)
+    // and its fused scale is faster; so are its errors at 17 and 19 times 18
+    // or 20.
+    int dr = r1_;
+    if (!kind_ && !pf.empty() && (pf.back() == 11 || pf.back() == 13)) {
+        dr = 1;
+        for (int r = 2; r <= 16; ++r)
+            if (n % r == 0) dr = r;
+        if (n / dr > kDenseMaxComposite) dr = 0;
+    }
+    dense_.init(n, dr);
     const std::pair<int, int> ab =
         kind_ == 2 && (rader_faster(true) || rader_faster(false)) ? fft2_split(r2_ - 1) : std::pair<int, int>{0, 0};
     rader_.init(n, r1_, r2_, ab.first, ab.second);
@@ -842,7 +859,6 @@ void AxisFFT::launch_line(cplx<R>* data, size_t es, int ncols, size_t os, int no
     if (mode == 2) launch<R, false, true>(cw, cls, stream, grd, shm, s, data, f, tw, es, ncols, os, ptw, ks);
     else if (mode == 1) launch<R, true, false>(cw, cls, stream, grd, shm, s, data, f, tw, es, ncols, os, ptw, ks);
     else launch<R, false, false>(cw, cls, stream, grd, shm, s, data, f, tw, es, ncols, os, ptw, ks);
-    MPM_LAUNCH();
 }
 
 template <typename R>

@@ -40,6 +40,8 @@ public:
     void init(int n, int r1);     // (the caller waits for the uploads, uploads_done)
     // whether a tile of four columns fits in shared memory
     bool fits(bool fp64) const;
+    int radix() const { return r1_; }
+    int rest() const { return m_; }
     // as AxisFFT::run / run_scaled (mode 2: two launches); tw: W_n^t, t < n
     template <typename R>
     void run(cplx<R>* data, const cplx<R>* tw, size_t es, int ncols, size_t os, int nouter, int mode, const R* scale,
@@ -92,7 +94,8 @@ public:
     // kernel a transform of ncols columns takes: 1 two-pass in registers (both
     // factors in-register radices, at least half a tile of columns per line),
     // 2 in-register radix times table product or a second one (mpm_dense.cu:
-    // lengths with one prime above 16, two radices with few columns per line),
+    // lengths with one prime above 16, two radices with few columns per line,
+    // other lengths with a factor of 11 or 13 and none above),
     // 3 in-register radix and Rader's convolution (mpm_rader.cu: one prime too
     // long for the product, at least half a tile of columns per line, no
     // fused scale), 0 general multi-pass
@@ -105,7 +108,9 @@ public:
     // the split of the kernel that such a transform takes, (0, 0) for the
     // general one
     std::pair<int, int> split(int ncols, bool fp64, int mode) const {
-        return path(ncols, fp64, mode) ? std::pair<int, int>{r1_, r2_} : std::pair<int, int>{0, 0};
+        const int p = path(ncols, fp64, mode);
+        if (p == 2) return {dense_.radix(), dense_.rest()};
+        return p ? std::pair<int, int>{r1_, r2_} : std::pair<int, int>{0, 0};
     }
 
     // The k-space step of the pruned (z-slab) monodisperse grid fused with

@@ -261,8 +261,8 @@ MPM_API int mpm_field_grad(mpm_field* f, const void* lam, const void* p, int M, 
  * element e of line o, column c by scale[(e*nouter + o)*sz + c/sb], inverse.
  * general != 0 forces the multi-pass kernel; split (optional, 2 ints)
  * receives the factorisation n = r1 * r2 of the kernel that ran (r1 a radix
- * up to 16; r2 another, or a prime above 16 whose transforms are products
- * with tables or Rader's convolutions) or (0, 0) for the multi-pass kernel.
+ * up to 16; r2 another, or a rest whose transforms are products with tables
+ * or, of a prime, Rader's convolutions) or (0, 0) for the multi-pass kernel.
  * Synchronises the stream before returning. */
 MPM_API int mpm_line_fft(void* data, int fp64, int n, size_t es, int ncols, size_t os, int nouter, int mode,
                          const void* scale, int sz, int sb, int general, int* split, void* stream);

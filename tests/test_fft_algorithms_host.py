@@ -1,5 +1,5 @@
 """numpy restatements of the index algebra the in-house line transforms use
-(mpm_fft.cu), checked against numpy's FFT on the CPU: the two-pass Stockham
+(mpm_fft.cu, mpm_rader.cu), checked against numpy's FFT on the CPU: the two-pass Stockham
 split n = r1 * r2, the fused forward-scale-inverse pass (the forward pass-2
 outputs of butterfly j are the inputs of the first inverse butterfly j), and
 the Rader prime pass with its tables (primitive root g, a_q = x[g^-q],

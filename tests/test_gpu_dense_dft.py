@@ -1,7 +1,8 @@
 """Line transforms by table products (mpm_dense.cu) against numpy in 64 bits,
 at the sizes where they can go wrong: one and two points per product, even
-middles, tables that stay in global memory (m above 131), radices up to 16 in
-front, columns that do not fill a tile, and few columns per line (lines and
+middles, the longest product in one sum and the first in blocks (47, 53 points),
+tables that stay in global memory (m above 191, in fp64 127), radices up to 16 in
+front, composite rests (260, 286, 352; 1144 = 13 * 88), columns that do not fill a tile, and few columns per line (lines and
 columns enumerated together).  Tolerance: a product sums m / 2 rounded terms, so
 its error is at most about sqrt(m) roundings of the result's root mean square."""
 import numpy as np
@@ -13,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("fp64", [False, True])
-@pytest.mark.parametrize("n", [3, 17, 22, 53, 84, 109, 131, 137, 251, 260, 272, 366])
+@pytest.mark.parametrize("n", [3, 17, 22, 47, 53, 84, 109, 131, 137, 251, 260, 272, 286, 352, 366, 1144])
 def test_product_transform(n, fp64):
     from cumpm_b200 import capi
 

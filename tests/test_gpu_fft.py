@@ -13,11 +13,11 @@ pytestmark = pytest.mark.gpu
 
 # two radices in registers: 2 = 2x1, 16 = 4x4, 49 = 7x7, 80 = 10x8,
 # 108 = 12x9, 112 = 14x8, 143 = 13x11, 256 = 16x16; a radix and a prime:
-# 34 = 2x17, 97 = 1x97, 206 = 2x103, 238 = 14x17, 366 = 6x61; general only:
-# 289 = 17*17
-LENGTHS = [2, 16, 34, 49, 80, 97, 108, 112, 143, 206, 238, 256, 289, 366]
+# 34 = 2x17, 97 = 1x97, 206 = 2x103, 238 = 14x17, 366 = 6x61; a radix and a
+# composite rest: 260 = 13x20, 352 = 16x22; general only: 289 = 17*17, 360, 380
+LENGTHS = [2, 16, 34, 49, 80, 97, 108, 112, 143, 206, 238, 256, 260, 289, 352, 360, 366, 380]
 SPLITS = {2: (2, 1), 16: (4, 4), 34: (2, 17), 49: (7, 7), 80: (10, 8), 108: (12, 9), 112: (14, 8),
-          143: (13, 11), 256: (16, 16), 97: (1, 97), 206: (2, 103), 238: (14, 17), 366: (6, 61)}
+          143: (13, 11), 256: (16, 16), 97: (1, 97), 206: (2, 103), 238: (14, 17), 366: (6, 61), 260: (13, 20), 352: (16, 22)}
 
 
 def run_case(n, layout, ncols, nouter, fp64, mode, general, seed=0, sb=4):
