@@ -267,9 +267,9 @@ def kernel_launches():
 
 
 def empty_cache():
-    """Gives the buffers that dropped solvers and near fields left for the next
-    ones (at most 256 MB of device and 64 MB of page-locked memory) back to the
-    driver."""
+    """Gives the buffers that dropped solvers, near fields and fields left for the
+    next ones (at most 256 MB of device and 64 MB of page-locked memory) back to
+    the driver."""
     lib().mpm_empty_cache()
 
 

@@ -279,7 +279,7 @@ MPM_API int mpm_profile_read(double* ms, long long* count, int n);
 MPM_API long long mpm_kernel_launches(void);
 
 /* ---- memory (no counterpart in the reference) ----------------------------
- * Dipole solvers and near fields keep the buffers that they release for the
+ * Solvers, near fields and fields keep the buffers that they release for the
  * next one (at most 256 MB of device and 64 MB of page-locked memory in the
  * whole process); this gives them back to the driver. */
 MPM_API void mpm_empty_cache(void);
